@@ -350,10 +350,23 @@ extern "C" vvlic_status vvlic_create(vvlic_ctx** out, int32_t device) {
   return VVLIC_OK;
 }
 
+namespace vvlic {
+void free_textures(Volume& v) {
+  for (int i = 0; i < 3; ++i) {
+    if (v.tex[i]) cudaDestroyTextureObject(v.tex[i]);
+    if (v.surf[i]) cudaDestroySurfaceObject(v.surf[i]);
+    if (v.array[i]) cudaFreeArray(v.array[i]);
+    v.tex[i] = 0;
+    v.surf[i] = 0;
+    v.array[i] = nullptr;
+  }
+  v.array_bytes = 0;
+}
+}  // namespace vvlic
+
 static void free_volume(Volume& v) {
   if (v.d_licvol) cudaFree(v.d_licvol);
-  if (v.tex) cudaDestroyTextureObject(v.tex);
-  if (v.array) cudaFreeArray(v.array);
+  free_textures(v);
   if (v.d_texels) cudaFree(v.d_texels);
   if (v.d_cells) cudaFree(v.d_cells);
   v = Volume();

@@ -49,6 +49,12 @@ __global__ void field_maxlen_kernel(const void* xyz, int dtype, size_t count, un
   if ((threadIdx.x & 31) == 0) atomicMax(maxbits, __float_as_uint(m));
 }
 
+// The machine word(s) of one texel.
+template <int ST> struct TexelWord {
+  using type = typename std::conditional<ST == VVLIC_STORAGE_F32, float4,
+                                         typename std::conditional<ST == VVLIC_STORAGE_UNORM8, uint32_t, uint2>::type>::type;
+};
+
 template <int ST>
 __device__ __forceinline__ void store_texel(void* out, size_t a, float r, float g, float b, float al) {
   if (ST == VVLIC_STORAGE_F32) {
@@ -267,8 +273,7 @@ __global__ void noise_grad_filter_kernel(const uint8_t* v, const float4* g, int 
 // cell c per axis covers texels clamp(c-1), clamp(c): (n+1)^3 cells of 8 texels
 template <int ST>
 __global__ void field_cells_kernel(const void* texels, int nx, int ny, int nz, void* cells) {
-  using T = typename std::conditional<ST == VVLIC_STORAGE_F32, float4,
-                                      typename std::conditional<ST == VVLIC_STORAGE_UNORM8, uint32_t, uint2>::type>::type;
+  using T = typename TexelWord<ST>::type;
   const T* t = reinterpret_cast<const T*>(texels);
   T* c = reinterpret_cast<T*>(cells);
   const int cx = nx + 1, cy = ny + 1, cz = nz + 1;
@@ -321,14 +326,63 @@ inline int grid_for(size_t count) {
   return (int)(b < 152 * 64 ? (b == 0 ? 1 : b) : 152 * 64);
 }
 
-// One RGBA texel per iteration: four bf16 values (8 bytes) -> four halves (8 bytes), the
-// component order kept (x in the low half of the first word).
-__global__ void bf16_to_half_kernel(const uint2* in, size_t count, uint2* out) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
-    const uint2 r = in[i];
-    __half2 lo = __floats2half2_rn(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u));
-    __half2 hi = __floats2half2_rn(__uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
-    out[i] = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+// Division of a 31-bit index by a fixed extent as a multiply-high and a shift.
+struct FastDiv {
+  unsigned mul, shift, d;
+};
+inline FastDiv fast_div(unsigned d) {
+  FastDiv f;
+  f.d = d;
+  f.shift = 0;
+  while ((1ull << f.shift) < d) ++f.shift;
+  f.mul = (unsigned)((((1ull << f.shift) - d) << 32) / d + 1);
+  return f;
+}
+__device__ __forceinline__ unsigned quotient(unsigned a, const FastDiv& f) { return (__umulhi(a, f.mul) + a) >> f.shift; }
+
+// Voxel index -> coordinates.
+struct VoxelMap {
+  FastDiv nx, ny;
+};
+__device__ __forceinline__ void voxel_xyz(unsigned a, const VoxelMap& m, int& x, int& y, int& z) {
+  const unsigned row = quotient(a, m.nx), slice = quotient(row, m.ny);
+  x = (int)(a - row * m.nx.d);
+  y = (int)(row - slice * m.ny.d);
+  z = (int)slice;
+}
+inline VoxelMap voxel_map(const int n[3]) { return VoxelMap{fast_div((unsigned)n[0]), fast_div((unsigned)n[1])}; }
+
+// The texel of voxel (x, y, z) into the volume's texture arrays.
+template <int ST>
+__device__ __forceinline__ void store_array(const FieldSurfaces& s, int x, int y, int z,
+                                            typename TexelWord<ST>::type t) {
+  if constexpr (ST == VVLIC_STORAGE_F32) {
+    surf3Dwrite(make_float2(t.x, t.y), s.rgba, x * 8, y, z);
+    surf3Dwrite(t.z, s.z, x * 4, y, z);
+    surf3Dwrite(t.w, s.w, x * 4, y, z);
+  } else if constexpr (ST == VVLIC_STORAGE_BF16) {
+    const __half2 lo = __floats2half2_rn(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xffff0000u));
+    const __half2 hi = __floats2half2_rn(__uint_as_float(t.y << 16), __uint_as_float(t.y & 0xffff0000u));
+    surf3Dwrite(make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi)), s.rgba,
+                x * 8, y, z);
+  } else if constexpr (ST == VVLIC_STORAGE_F16) {
+    surf3Dwrite(t, s.rgba, x * 8, y, z);
+  } else {
+    surf3Dwrite(t, s.rgba, x * 4, y, z);
+  }
+}
+
+// Texels -> texture arrays through surface writes, one voxel per thread and iteration.  Bound by
+// memory; it replaces a cudaMemcpy3D per array: a 512^3 half4 field update, whose last pass this is,
+// went from 1762 to 1556 us.
+template <int ST>
+__global__ void fill_arrays_kernel(const void* texels, unsigned count, const __grid_constant__ VoxelMap m,
+                                   const __grid_constant__ FieldSurfaces arr) {
+  const auto* t = reinterpret_cast<const typename TexelWord<ST>::type*>(texels);
+  for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < count; a += gridDim.x * blockDim.x) {
+    int x, y, z;
+    voxel_xyz(a, m, x, y, z);
+    store_array<ST>(arr, x, y, z, t[a]);
   }
 }
 
@@ -402,9 +456,17 @@ cudaError_t launch_build_field_cells(const void* d_texels, const int n[3], int s
   return cudaGetLastError();
 }
 
-cudaError_t launch_bf16_to_half(const void* d_bf16, size_t count, void* d_half, cudaStream_t s) {
-  bf16_to_half_kernel<<<grid_for(count), kThreads, 0, s>>>(reinterpret_cast<const uint2*>(d_bf16), count,
-                                                          reinterpret_cast<uint2*>(d_half));
+cudaError_t launch_fill_arrays(const void* d_texels, const int n[3], int storage, const FieldSurfaces& arr,
+                               cudaStream_t s) {
+  const unsigned count = (unsigned)n[0] * (unsigned)n[1] * (unsigned)n[2];  // < 2^31 (valid_dims)
+  const VoxelMap m = voxel_map(n);
+  const int g = grid_for(count);
+  if (storage == VVLIC_STORAGE_F32) fill_arrays_kernel<VVLIC_STORAGE_F32><<<g, kThreads, 0, s>>>(d_texels, count, m, arr);
+  else if (storage == VVLIC_STORAGE_F16)
+    fill_arrays_kernel<VVLIC_STORAGE_F16><<<g, kThreads, 0, s>>>(d_texels, count, m, arr);
+  else if (storage == VVLIC_STORAGE_UNORM8)
+    fill_arrays_kernel<VVLIC_STORAGE_UNORM8><<<g, kThreads, 0, s>>>(d_texels, count, m, arr);
+  else fill_arrays_kernel<VVLIC_STORAGE_BF16><<<g, kThreads, 0, s>>>(d_texels, count, m, arr);
   return cudaGetLastError();
 }
 

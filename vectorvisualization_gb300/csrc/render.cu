@@ -40,64 +40,48 @@ vvlic_status ensure_noise_cells(vvlic_ctx* c, NoiseTex& n, cudaStream_t s) {
   return VVLIC_OK;
 }
 
-// Copies the volume's texels into its texture array (allocated by ensure_texture).  The texture
-// unit has no bf16 format: a BF16 volume's texture is a half4 array holding its BF16 texels
-// converted to half (exact for the encoded texels, all in [0, 1], down to 2^-14).
-vvlic_status copy_field_texture(vvlic_ctx* c, Volume& v, cudaStream_t s) {
-  const bool bf16 = v.storage == VVLIC_STORAGE_BF16;
-  const size_t tb = texel_bytes(v.storage);  // 8 bytes for F16, BF16 and their half4 copy alike
-  const size_t count = (size_t)v.n[0] * v.n[1] * v.n[2];
-  void* src = v.d_texels;
-  cudaError_t e;
-  if (bf16) {
-    // stream-ordered scratch: freed behind the array copy that reads it
-    e = cudaMallocAsync(&src, count * tb, s);
-    if (e != cudaSuccess) return cuda_fail(c, e, "BF16 texture staging allocation");
-    e = launch_bf16_to_half(v.d_texels, count, src, s);
-    if (e != cudaSuccess) {
-      cudaFreeAsync(src, s);
-      return cuda_fail(c, e, "BF16 texture conversion");
-    }
-  }
-  cudaMemcpy3DParms cp;
-  std::memset(&cp, 0, sizeof cp);
-  cp.srcPtr = make_cudaPitchedPtr(src, v.n[0] * tb, v.n[0], v.n[1]);
-  cp.dstArray = v.array;
-  cp.extent = make_cudaExtent(v.n[0], v.n[1], v.n[2]);
-  cp.kind = cudaMemcpyDeviceToDevice;
-  e = cudaMemcpy3DAsync(&cp, s);
-  if (bf16) {
-    cudaError_t ef = cudaFreeAsync(src, s);
-    if (e == cudaSuccess) e = ef;
-  }
-  if (e != cudaSuccess) return cuda_fail(c, e, "texture array copy");
+// Copies the volume's texels into its texture arrays (allocated by ensure_texture).
+vvlic_status fill_textures(vvlic_ctx* c, Volume& v, cudaStream_t s) {
+  FieldSurfaces arr;
+  arr.rgba = v.surf[0];
+  arr.z = v.surf[1];
+  arr.w = v.surf[2];
+  const cudaError_t e = launch_fill_arrays(v.d_texels, v.n, v.storage, arr, s);
+  if (e != cudaSuccess) return cuda_fail(c, e, "texture array fill");
   return VVLIC_OK;
 }
 
+// Texture copy of a volume.  128-bit texels filter at an eighth of the texture unit's rate, so F32
+// fields are held as a float2 array of (x, y) and two float arrays (Field<F32, kTexture>).
 vvlic_status ensure_texture(vvlic_ctx* c, Volume& v, cudaStream_t s) {
-  if (v.tex) return VVLIC_OK;
-  const bool bf16 = v.storage == VVLIC_STORAGE_BF16;
-  cudaChannelFormatDesc desc = v.storage == VVLIC_STORAGE_F32 ? cudaCreateChannelDesc<float4>()
-                               : (v.storage == VVLIC_STORAGE_F16 || bf16) ? cudaCreateChannelDescHalf4()
-                                                                          : cudaCreateChannelDesc<uchar4>();
-  cudaExtent ext = make_cudaExtent(v.n[0], v.n[1], v.n[2]);
-  cudaError_t e = cudaMalloc3DArray(&v.array, &desc, ext);
-  if (e != cudaSuccess) return cuda_fail(c, e, "texture array allocation");
-  v.array_bytes = (size_t)v.n[0] * v.n[1] * v.n[2] * texel_bytes(v.storage);
-  vvlic_status st = copy_field_texture(c, v, s);
+  if (v.array_bytes) return VVLIC_OK;
+  const bool f32 = v.storage == VVLIC_STORAGE_F32, u8 = v.storage == VVLIC_STORAGE_UNORM8;
+  const cudaChannelFormatDesc desc[3] = {f32 ? cudaCreateChannelDesc<float2>()
+                                             : (u8 ? cudaCreateChannelDesc<uchar4>() : cudaCreateChannelDescHalf4()),
+                                         cudaCreateChannelDesc<float>(), cudaCreateChannelDesc<float>()};
+  const cudaExtent ext = make_cudaExtent(v.n[0], v.n[1], v.n[2]);
+  free_textures(v);  // what an earlier call that failed half way left
+  for (int i = 0; i < (f32 ? 3 : 1); ++i) {
+    cudaError_t e = cudaMalloc3DArray(&v.array[i], &desc[i], ext, cudaArraySurfaceLoadStore);
+    if (e != cudaSuccess) return cuda_fail(c, e, "texture array allocation");
+    cudaResourceDesc rd;
+    std::memset(&rd, 0, sizeof rd);
+    rd.resType = cudaResourceTypeArray;
+    rd.res.array.array = v.array[i];
+    e = cudaCreateSurfaceObject(&v.surf[i], &rd);
+    if (e != cudaSuccess) return cuda_fail(c, e, "texture surface");
+    cudaTextureDesc td;
+    std::memset(&td, 0, sizeof td);
+    td.addressMode[0] = td.addressMode[1] = td.addressMode[2] = cudaAddressModeClamp;  // CLAMP_TO_EDGE
+    td.filterMode = cudaFilterModeLinear;
+    td.readMode = u8 ? cudaReadModeNormalizedFloat : cudaReadModeElementType;
+    td.normalizedCoords = 1;  // GL texture coordinates
+    e = cudaCreateTextureObject(&v.tex[i], &rd, &td, nullptr);
+    if (e != cudaSuccess) return cuda_fail(c, e, "texture object");
+  }
+  const vvlic_status st = fill_textures(c, v, s);
   if (st) return st;
-  cudaResourceDesc rd;
-  std::memset(&rd, 0, sizeof rd);
-  rd.resType = cudaResourceTypeArray;
-  rd.res.array.array = v.array;
-  cudaTextureDesc td;
-  std::memset(&td, 0, sizeof td);
-  td.addressMode[0] = td.addressMode[1] = td.addressMode[2] = cudaAddressModeClamp;  // CLAMP_TO_EDGE
-  td.filterMode = cudaFilterModeLinear;
-  td.readMode = v.storage == VVLIC_STORAGE_UNORM8 ? cudaReadModeNormalizedFloat : cudaReadModeElementType;
-  td.normalizedCoords = 1;  // GL texture coordinates
-  e = cudaCreateTextureObject(&v.tex, &rd, &td, nullptr);
-  if (e != cudaSuccess) return cuda_fail(c, e, "texture object");
+  v.array_bytes = (size_t)v.n[0] * v.n[1] * v.n[2] * texel_bytes(v.storage);
   return VVLIC_OK;
 }
 
@@ -147,7 +131,7 @@ vvlic_status refresh_volume_layouts(vvlic_ctx* c, Volume& v, cudaStream_t s) {
     cudaError_t e = launch_build_field_cells(v.d_texels, v.n, v.storage, v.d_cells, s);
     if (e != cudaSuccess) return cuda_fail(c, e, "cell layout rebuild");
   }
-  if (v.array) return copy_field_texture(c, v, s);
+  if (v.array_bytes) return fill_textures(c, v, s);
   return VVLIC_OK;
 }
 
@@ -199,13 +183,17 @@ vvlic_status build_render_args_ex(vvlic_ctx* c, Volume& v, int W, int H, cudaStr
     case VVLIC_SAMPLER_TEXTURE:
       if ((st = ensure_texture(c, v, s))) return st;
       if ((st = ensure_noise_texture(c, c->noise, s))) return st;
-      a.tex = v.tex;
+      a.tex = v.tex[0];
+      a.tex_z = v.tex[1];
+      a.tex_w = v.tex[2];
       a.noise_tex = c->noise.tex;
       break;
     default:  // HYBRID
       if ((st = ensure_texture(c, v, s))) return st;
       if ((st = ensure_noise_cells(c, c->noise, s))) return st;
-      a.tex = v.tex;
+      a.tex = v.tex[0];
+      a.tex_z = v.tex[1];
+      a.tex_w = v.tex[2];
       a.noise = c->noise.d_cells;
       break;
   }

@@ -23,7 +23,8 @@ enum Layout : int { kGather = 0, kCell = 1, kTexture = 2, kCellFast = 3 };
 // the constant bank; the taps are read warp-uniformly so they broadcast).
 struct RenderArgs {
   const void* field;          // GATHER: n0*n1*n2 RGBA texels; CELL: (n+1)^3 cells of 8 texels
-  cudaTextureObject_t tex;    // TEXTURE layout
+  // TEXTURE layout: RGBA texels in tex; F32 fields: (x, y) in tex, z in tex_z, w in tex_w
+  cudaTextureObject_t tex, tex_z, tex_w;
   int n[3];
   const uint8_t* noise;       // GATHER: m0*m1*m2 texels of noise_ch bytes; CELL: m^3 cells
   cudaTextureObject_t noise_tex;  // TEXTURE layout
@@ -280,6 +281,28 @@ template <int ST> struct Field<ST, kTexture> {  // hardware trilinear, normalise
     return tex3D<float4>(a.tex, s.x, s.y, s.z);
   }
 };
+// FP32 texels as three textures: the texture unit filters 32- and 64-bit texels at its full rate
+// (588 G trilinear fetches/s measured) and 128-bit ones at an eighth of it (75 G/s), with the
+// same filter arithmetic (2^20 random fetches of both forms agree bit for bit).  A 512^2 lit Heun
+// frame of a 256^3 field went from 87.9 to 36.7 ms, the 64^3 Euler frame at 256^2 from 9.2 to 3.1 ms.
+template <> struct Field<VVLIC_STORAGE_F32, kTexture> {
+  static __device__ __forceinline__ float4 sample(const RenderArgs& a, float3 s) {
+    const float2 xy = tex3D<float2>(a.tex, s.x, s.y, s.z);
+    return make_float4(xy.x, xy.y, tex3D<float>(a.tex_z, s.x, s.y, s.z), tex3D<float>(a.tex_w, s.x, s.y, s.z));
+  }
+};
+
+// The field at a streamline position: .w is read only under SPEED_OF_FLOW (a separate texture
+// for F32 fields; the other layouts deliver it with x, y and z).
+template <int ST, int LAYOUT> __device__ __forceinline__ float4 sample_step(const RenderArgs& a, float3 s) {
+  if constexpr (ST == VVLIC_STORAGE_F32 && LAYOUT == kTexture) {
+    const float2 xy = tex3D<float2>(a.tex, s.x, s.y, s.z);
+    const float z = tex3D<float>(a.tex_z, s.x, s.y, s.z);
+    return make_float4(xy.x, xy.y, z, a.sof ? tex3D<float>(a.tex_w, s.x, s.y, s.z) : 0.0f);
+  } else {
+    return Field<ST, LAYOUT>::sample(a, s);
+  }
+}
 
 // ------------------------------------------------------------------------------------------
 // noise sampling: texture3D(noiseSampler, s), LINEAR + REPEAT (dataset.cpp:1333-1335), uint8/255.
@@ -507,21 +530,20 @@ __device__ __forceinline__ float3 slope_h(float4 f, float h) {
 // first-same-as-last reuse of the reference's `step` in/out argument).
 template <int ST, int FL, int INTEG>
 __device__ __forceinline__ float3 lic_step(const RenderArgs& a, float3 p, float4& step, float dirs) {
-  using F = Field<ST, FL>;
   const float hs = a.sof ? a.h_eff * dirs * step.w : a.h_eff * dirs;
   float3 k1 = INTEG == VVLIC_RK4 ? scl3(slope(step), hs) : slope_h(step, hs);
   if (INTEG == VVLIC_EULER) {
     p = add3(p, k1);
   } else if (INTEG == VVLIC_HEUN) {
-    float3 k2 = slope_h(F::sample(a, add3(p, k1)), hs);
+    float3 k2 = slope_h(sample_step<ST, FL>(a, add3(p, k1)), hs);
     p = add3(p, scl3(add3(k1, k2), 0.5f));
   } else {
-    float3 k2 = scl3(slope(F::sample(a, add3(p, scl3(k1, 0.5f)))), hs);
-    float3 k3 = scl3(slope(F::sample(a, add3(p, scl3(k2, 0.5f)))), hs);
-    float3 k4 = scl3(slope(F::sample(a, add3(p, k3))), hs);
+    float3 k2 = scl3(slope(sample_step<ST, FL>(a, add3(p, scl3(k1, 0.5f)))), hs);
+    float3 k3 = scl3(slope(sample_step<ST, FL>(a, add3(p, scl3(k2, 0.5f)))), hs);
+    float3 k4 = scl3(slope(sample_step<ST, FL>(a, add3(p, k3))), hs);
     p = add3(p, scl3(add3(add3(k1, scl3(k2, 2.0f)), add3(scl3(k3, 2.0f), k4)), 1.0f / 6.0f));
   }
-  step = F::sample(a, p);
+  step = sample_step<ST, FL>(a, p);
   return p;
 }
 

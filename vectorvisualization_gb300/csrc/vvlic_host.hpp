@@ -28,9 +28,12 @@ struct Volume {
   size_t texel_bytes = 0;
   void* d_cells = nullptr;        // corner-packed cells, built on first CELL render
   size_t cell_bytes = 0;
-  cudaArray_t array = nullptr;    // texture copy, built on first TEXTURE render
-  cudaTextureObject_t tex = 0;
-  size_t array_bytes = 0;
+  // texture copy, built on first TEXTURE render: RGBA texels in [0], or F32 texels as (x, y) in [0],
+  // z in [1] and w in [2]
+  cudaArray_t array[3] = {nullptr, nullptr, nullptr};
+  cudaSurfaceObject_t surf[3] = {0, 0, 0};
+  cudaTextureObject_t tex[3] = {0, 0, 0};
+  size_t array_bytes = 0;         // 0 until all of them exist
   float* d_licvol = nullptr;      // precomputed LIC volume (vvlic_compute_lic_volume)
   int ln[3] = {0, 0, 0};
   bool licvol_valid = false;      // false after a field update until the next precompute
@@ -164,6 +167,7 @@ vvlic_status ensure_illum_luts(vvlic_ctx* c);
 cudaError_t after_launches(vvlic_ctx* c);
 vvlic_status cuda_fail(vvlic_ctx* c, cudaError_t e, const char* what);
 // Rewrite the cell and texture copies that exist from the texels, in place (render.cu).
+void free_textures(Volume& v);  // texture objects, surfaces and arrays of the texture copy
 vvlic_status refresh_volume_layouts(vvlic_ctx* c, Volume& v, cudaStream_t s);
 vvlic_status refresh_noise_layouts(vvlic_ctx* c, NoiseTex& n, cudaStream_t s);
 Geometry make_geometry(const int n[3], const float* slice_dist);
