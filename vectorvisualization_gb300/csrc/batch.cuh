@@ -12,11 +12,10 @@ namespace vvlic {
 constexpr int kWarpsPerCta = kThreads / 32;
 
 // Register cap of the unlit Euler / Heun batch kernels, whose arguments come from shared memory
-// rather than the constant bank.  On the 64-volume unlit batch: 8 CTAs/SM (64 registers) 1253 ms,
-// 7 1283 ms, 6 1326 ms.  (The single-render unlit kernels measured best at 7: 27.5 ms against
-// 29.7 at 8 and 33.5 at 9 on the 128^3 4-view forward.)
+// rather than the constant bank.  With packed noise taps, 24 views of 8 uneven volumes at 512^2:
+// 7 CTAs/SM (73 registers) 100.6 ms, 8 (64 registers) 112.5 ms, 6 105.4 ms, 5 104.7 ms.
 #ifndef VVLIC_BATCH_UNLIT_MIN_BLOCKS
-#define VVLIC_BATCH_UNLIT_MIN_BLOCKS 8
+#define VVLIC_BATCH_UNLIT_MIN_BLOCKS 7
 #endif
 template <int INTEG, bool GRAD> constexpr int batch_min_blocks() {
   return (!GRAD && INTEG != VVLIC_RK4) ? VVLIC_BATCH_UNLIT_MIN_BLOCKS : min_blocks<INTEG, GRAD>();

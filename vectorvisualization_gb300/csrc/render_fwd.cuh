@@ -16,12 +16,11 @@ constexpr int kTileW = 16, kTileH = 8;  // static schedule: 128 threads, a warp 
 constexpr int kWarpTileW = 8, kWarpTileH = 4;  // queue schedule: one warp per 8x4 pixel tile
 constexpr int kThreads = 128;
 // Minimum resident CTAs per SM requested from the compiler for the render kernels, i.e. a cap
-// of 65536 / (kThreads * VVLIC_MIN_BLOCKS) registers per thread.  6 (80 registers, no spills)
-// measured 155 Gsample-steps/s on the lit 1024^2 frame against 142 with the compiler's own
-// choice; 7 (73 registers, ~60 B spilled) beat 6 on the same GPU by 2 % (lit 1024^2 frame),
-// 5 % (the 64-volume batch) and 1 % (the 512^3 RK4 frame); 8 (64 registers) measured as 6.
+// of 65536 / (kThreads * VVLIC_MIN_BLOCKS) registers per thread.  With packed noise taps, at 8 / 7 /
+// 6 / 5: lit 1024^2 Heun frame of 256^3 68.2 / 61.2 / 60.7 / 60.0 ms, four-view fit step of 128^3
+// 70.8 / 68.7 / 66.1 / 63.0 ms, unlit 853x481 frame 7.15 / 7.15 / 7.11 / 7.11 ms.
 #ifndef VVLIC_MIN_BLOCKS
-#define VVLIC_MIN_BLOCKS 7
+#define VVLIC_MIN_BLOCKS 6
 #endif
 // The same for the RK4 kernels, which hold four slopes per step and trace two samples per pass
 // (trace_ray): 4 CTAs, 128 registers.  With one sample per pass, 6 CTAs (80 registers) was
