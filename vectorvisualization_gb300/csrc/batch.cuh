@@ -1,6 +1,7 @@
 // Batched LIC ray-cast: many render jobs (volume x view x image, each with its own LIC
 // parameters and filter) in one persistent launch.  Warps pull (job, tile) items from one
-// device work queue in job-major order (batch.cu); on a job switch a warp copies that
+// device work queue in job-major order (batch.cu) and trace a tile's rays in groups of four samples
+// (trace_group); on a job switch a warp copies that
 // job's argument block into its own shared-memory slot and traces the tile from there.  The
 // transfer function is the context's and is shared by every job.
 #pragma once
@@ -9,8 +10,6 @@
 
 namespace vvlic {
 
-constexpr int kWarpsPerCta = kThreads / 32;
-
 // Register cap of the unlit Euler / Heun batch kernels, whose arguments come from shared memory
 // rather than the constant bank.  With packed noise taps, 24 views of 8 uneven volumes at 512^2:
 // 7 CTAs/SM (73 registers) 100.6 ms, 8 (64 registers) 112.5 ms, 6 105.4 ms, 5 104.7 ms.
@@ -18,7 +17,7 @@ constexpr int kWarpsPerCta = kThreads / 32;
 #define VVLIC_BATCH_UNLIT_MIN_BLOCKS 7
 #endif
 template <int INTEG, bool GRAD> constexpr int batch_min_blocks() {
-  return (!GRAD && INTEG != VVLIC_RK4) ? VVLIC_BATCH_UNLIT_MIN_BLOCKS : min_blocks<INTEG, GRAD>();
+  return (!GRAD && INTEG != VVLIC_RK4) ? VVLIC_BATCH_UNLIT_MIN_BLOCKS : min_blocks<INTEG>();
 }
 
 template <int ST, int FL, int NL, int INTEG, bool GRAD>
@@ -27,7 +26,7 @@ __global__ void __launch_bounds__(kThreads, batch_min_blocks<INTEG, GRAD>())
                          unsigned* __restrict__ next, const float* __restrict__ tf, unsigned long long* counters,
                          int tw) {
   __shared__ __align__(16) float s_tf[5 * VVLIC_TF_ENTRIES];
-  __shared__ __align__(16) RenderArgs s_args[kWarpsPerCta];
+  __shared__ __align__(16) RenderArgs s_args[kWarps];
   for (int i = threadIdx.x; i < 5 * VVLIC_TF_ENTRIES; i += blockDim.x) s_tf[i] = __ldg(tf + i);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -50,15 +49,22 @@ __global__ void __launch_bounds__(kThreads, batch_min_blocks<INTEG, GRAD>())
       cur = item.x;
     }
     const int tiles_x = (a.W + tw - 1) / tw;
-    const int px = (int)(item.y % tiles_x) * tw + lane % tw;
-    const int py = (int)(item.y / tiles_x) * th + lane / tw;
-    if (px < a.W && py < a.H) {
+    // the tile's 32 pixels in four groups of 8 rays (4x2; 8x1 in one-row tiles), four samples at a time
+    constexpr int S = 4, R = 32 / S;
+    const int gw = th == 1 ? R : 4, gx = tw / gw, r = lane % R;
+    for (int sub = 0; sub < S; ++sub) {
+      const int px = (int)(item.y % tiles_x) * tw + (sub % gx) * gw + r % gw;
+      const int py = (int)(item.y / tiles_x) * th + (sub / gx) * (R / gw) + r / gw;
+      const bool ray = px < a.W && py < a.H;
+      if (!__any_sync(0xffffffffu, ray)) continue;
       uint32_t samples, hit;
-      float4 dest = trace_ray<ST, FL, NL, INTEG, GRAD>(a, s_tf, px, py, samples, hit);
-      store_pixel(a, px, py, dest, samples);
-      samples_acc += samples;
-      hits_acc += hit;
-      steps_acc += (unsigned long long)samples * (a.lb + a.lf);
+      const float4 dest = trace_group<ST, FL, NL, INTEG, GRAD, S>(a, s_tf, ray, px, py, samples, hit);
+      if (ray && lane < R) {
+        store_pixel(a, px, py, dest, samples);
+        samples_acc += samples;
+        hits_acc += hit;
+        steps_acc += (unsigned long long)samples * (a.lb + a.lf);
+      }
     }
   }
   unsigned s = __reduce_add_sync(0xffffffffu, samples_acc);

@@ -297,18 +297,18 @@ cudaError_t launch_technique(int storage, const RenderArgs& a, const TechArgs& t
   }
 }
 
-cudaError_t launch_raycast(const RenderArgs& a, int storage, int sampler, int integ, bool grad, const Schedule& sch,
+cudaError_t launch_raycast(const RenderArgs& a, int storage, int sampler, int integ, bool grad, int num_sms,
                            cudaStream_t s) {
   switch (kernel_storage(storage, sampler)) {
-    case VVLIC_STORAGE_F32: return launch_raycast_f32(a, sampler, integ, grad, sch, s);
-    case VVLIC_STORAGE_F16: return launch_raycast_f16(a, sampler, integ, grad, sch, s);
-    case VVLIC_STORAGE_UNORM8: return launch_raycast_u8(a, sampler, integ, grad, sch, s);
-    default: return launch_raycast_bf16(a, sampler, integ, grad, sch, s);
+    case VVLIC_STORAGE_F32: return launch_raycast_f32(a, sampler, integ, grad, num_sms, s);
+    case VVLIC_STORAGE_F16: return launch_raycast_f16(a, sampler, integ, grad, num_sms, s);
+    case VVLIC_STORAGE_UNORM8: return launch_raycast_u8(a, sampler, integ, grad, num_sms, s);
+    default: return launch_raycast_bf16(a, sampler, integ, grad, num_sms, s);
   }
 }
 
 // ------------------------------------------------------------------------------------------
-// longest-first tile order for the queue schedule
+// longest-first tile order for the adjoint's queue
 // ------------------------------------------------------------------------------------------
 namespace {
 
@@ -379,7 +379,7 @@ cudaError_t launch_tile_order(const RenderArgs& a, int ntiles, int tiles_x, int 
 
 namespace {
 
-// Queue schedule for one image: longest-first tile order in the context's scratch.
+// Adjoint queue for one image: longest-first tile order in the context's scratch.
 vvlic_status make_schedule(vvlic_ctx* c, const RenderArgs& a, const Geometry& gm, int w, int h, cudaStream_t s,
                            Schedule& sch) {
   const int tiles_x = (w + 7) / 8, ntiles = tiles_x * ((h + 3) / 4);
@@ -508,20 +508,16 @@ extern "C" vvlic_status vvlic_render_device(vvlic_ctx* c, int32_t vol_id, float*
     c->tape_valid = false;
     if ((st = prepare_tape(c, w, h, a, s))) return st;
   }
-  Schedule sch;
-  sch.num_sms = c->num_sms;
   const bool grad = c->params.illum == VVLIC_ILLUM_GRADIENT;
   const bool brick = c->params.sampler == VVLIC_SAMPLER_BRICK;
   BrickArgs bargs;
   if (brick && (st = prepare_brick(c, it->second, a, grad, bargs))) return st;
   cudaError_t e = cudaMemsetAsync(c->d_counters, 0, 4 * sizeof(unsigned long long), s);
   if (e != cudaSuccess) return cuda_fail(c, e, "render");
-  if (!brick && c->params.schedule == VVLIC_SCHEDULE_QUEUE && (st = make_schedule(c, a, it->second.geom, w, h, s, sch)))
-    return st;
   e = cudaEventRecord(c->ev0, s);
   if (e == cudaSuccess)
     e = brick ? launch_brick(it->second.storage, a, bargs, c->params.integrator, grad, s)
-              : launch_raycast(a, it->second.storage, c->params.sampler, c->params.integrator, grad, sch, s);
+              : launch_raycast(a, it->second.storage, c->params.sampler, c->params.integrator, grad, c->num_sms, s);
   if (e == cudaSuccess) e = cudaEventRecord(c->ev1, s);
   if (e != cudaSuccess) return cuda_fail(c, e, "render launch");
   c->stats_pending = true;

@@ -1,10 +1,13 @@
-// Forward LIC ray-cast kernels: one thread per pixel runs the whole lic3d_fragment.glsl main()
-// (lic3d_fragment.glsl:5-99).  Two work distributions:
-//   * static: one CTA per 16x8 pixel tile in raster order;
-//   * queue:  persistent CTAs whose warps pull 8x4 pixel tiles from a device work queue, the
-//             tiles pre-ordered longest ray chord first (one atomicAdd per tile, no waiting).
-// Instantiated per field storage in render_f32.cu / render_f16.cu / render_bf16.cu /
-// render_u8.cu so the translation units compile in parallel.
+// Forward LIC ray-cast kernels: the lic3d_fragment.glsl main() (lic3d_fragment.glsl:5-99) on a raster
+// grid of small CTAs, each warp on a tile of rays with S consecutive samples of each side by side
+// (trace_group).  Instantiated per field storage in render_f32.cu / render_f16.cu /
+// render_bf16.cu / render_u8.cu so the translation units compile in parallel.
+//
+// The raster grid took the place of persistent warps that pulled 8x4-pixel tiles longest ray first
+// and of a static grid of 16x8-pixel CTAs.  With S = 8 the items are so short that the order no
+// longer matters for the tail, and neighbouring rays that run on one SM at a time share texels and
+// cells in its L1.  Queue -> raster, both with groups: lit 1024^2 Heun frame of 256^3 60.8 -> 57.7 ms
+// (FP32 at 512^2 30.9 -> 27.3), unlit 853x481 frame 2.82 -> 2.68 ms, 128^2 preview 348 -> 190 us.
 #pragma once
 
 #include "vvlic_device.cuh"
@@ -12,29 +15,23 @@
 
 namespace vvlic {
 
-constexpr int kTileW = 16, kTileH = 8;  // static schedule: 128 threads, a warp covers 16x2 pixels
-constexpr int kWarpTileW = 8, kWarpTileH = 4;  // queue schedule: one warp per 8x4 pixel tile
-constexpr int kThreads = 128;
-// Minimum resident CTAs per SM requested from the compiler for the render kernels, i.e. a cap
-// of 65536 / (kThreads * VVLIC_MIN_BLOCKS) registers per thread.  With packed noise taps, at 8 / 7 /
-// 6 / 5: lit 1024^2 Heun frame of 256^3 68.2 / 61.2 / 60.7 / 60.0 ms, four-view fit step of 128^3
-// 70.8 / 68.7 / 66.1 / 63.0 ms, unlit 853x481 frame 7.15 / 7.15 / 7.11 / 7.11 ms.
+constexpr int kTileW = 16, kTileH = 8;         // techniques.cuh: one CTA of 128 threads per tile
+constexpr int kWarpTileW = 8, kWarpTileH = 4;  // adjoint.cuh, batch.cuh: 32 pixels per warp
+constexpr int kThreads = 128, kWarps = kThreads / 32;
+
+// Registers: the ray-cast kernels are compiled for at most 65536 / (128 * VVLIC_MIN_BLOCKS) registers
+// per thread and launched in CTAs of up to kCastThreads threads.  Euler and Heun at 7 / 6 / 5, groups of
+// four: 512^2 lit frame of 256^3 17.9 / 17.7 / 17.3 ms, 1024^2 61.1 / 60.9 / 62.7 ms, FP32 31.9 / 30.9 /
+// 30.0 ms, unlit 853x481 UNORM8 frame 2.90 / 2.79 / 2.78 ms.  RK4 (four slopes per step), 1024^2 frame
+// of the lit 512^3 orbit, at 6 / 5 / 4: 488 / 474 / 482 ms.
 #ifndef VVLIC_MIN_BLOCKS
 #define VVLIC_MIN_BLOCKS 6
 #endif
-// The same for the RK4 kernels, which hold four slopes per step and trace two samples per pass
-// (trace_ray): 4 CTAs, 128 registers.  With one sample per pass, 6 CTAs (80 registers) was
-// best: 7 and 8 CTAs spilled and ran 1.5-3 % slower on the 512^3 RK4 orbit frames.
 #ifndef VVLIC_RK4_MIN_BLOCKS
-#define VVLIC_RK4_MIN_BLOCKS 4
+#define VVLIC_RK4_MIN_BLOCKS 5
 #endif
-// Unlit (and line-lit) Euler / Heun kernels: no noise gradients to carry.
-#ifndef VVLIC_UNLIT_MIN_BLOCKS
-#define VVLIC_UNLIT_MIN_BLOCKS VVLIC_MIN_BLOCKS
-#endif
-template <int INTEG, bool GRAD> constexpr int min_blocks() {
-  return INTEG == VVLIC_RK4 ? VVLIC_RK4_MIN_BLOCKS : (GRAD ? VVLIC_MIN_BLOCKS : VVLIC_UNLIT_MIN_BLOCKS);
-}
+template <int INTEG> constexpr int min_blocks() { return INTEG == VVLIC_RK4 ? VVLIC_RK4_MIN_BLOCKS : VVLIC_MIN_BLOCKS; }
+template <int INTEG> constexpr int cast_threads() { return INTEG == VVLIC_RK4 ? 128 : 256; }
 
 __device__ __forceinline__ void load_tf(const RenderArgs& a, float* s_tf) {
   for (int i = threadIdx.x; i < 5 * VVLIC_TF_ENTRIES; i += blockDim.x) s_tf[i] = __ldg(a.tf + i);
@@ -61,89 +58,94 @@ __device__ __forceinline__ void flush_counters(const RenderArgs& a, uint32_t sam
   }
 }
 
-template <int ST, int FL, int NL, int INTEG, bool GRAD>
-__global__ void __launch_bounds__(kThreads, min_blocks<INTEG, GRAD>()) raycast_kernel(const __grid_constant__ RenderArgs a) {
-  __shared__ __align__(16) float s_tf[5 * VVLIC_TF_ENTRIES];
-  load_tf(a, s_tf);
-  const int px = blockIdx.x * kTileW + (threadIdx.x % kTileW);
-  const int py = blockIdx.y * kTileH + (threadIdx.x / kTileW);
-  uint32_t samples = 0, hit = 0;
-  if (px < a.W && py < a.H) {
-    float4 dest = trace_ray<ST, FL, NL, INTEG, GRAD>(a, s_tf, px, py, samples, hit);
-    store_pixel(a, px, py, dest, samples);
-  }
-  flush_counters(a, samples, hit);
+// Pixels of a CTA: warps of (32 / S) rays, two wide and the rest on top of one another.
+template <int S> struct GroupTile {
+  static constexpr int w = 2, h = 16 / S;
+};
+struct CtaShape {
+  int wx, wy;  // warps across and up
+};
+__host__ __device__ inline CtaShape cta_shape(int threads) {
+  return threads >= 128 ? CtaShape{2, threads / 64} : CtaShape{1, threads / 32};
 }
 
-template <int ST, int FL, int NL, int INTEG, bool GRAD>
-__global__ void __launch_bounds__(kThreads, min_blocks<INTEG, GRAD>()) raycast_queue_kernel(const __grid_constant__ RenderArgs a,
-                                                                 const uint32_t* __restrict__ order, int ntiles,
-                                                                 unsigned* __restrict__ next) {
+template <int ST, int FL, int NL, int INTEG, bool GRAD, int S>
+__global__ void __launch_bounds__(cast_threads<INTEG>(), min_blocks<INTEG>() * 128 / cast_threads<INTEG>())
+    raycast_kernel(const __grid_constant__ RenderArgs a, int strip) {
   __shared__ __align__(16) float s_tf[5 * VVLIC_TF_ENTRIES];
   load_tf(a, s_tf);
-  const int lane = threadIdx.x & 31;
-  const int tiles_x = (a.W + kWarpTileW - 1) / kWarpTileW;
-  uint32_t samples_acc = 0, hits_acc = 0;
-  for (;;) {
-    unsigned t = 0;
-    if (lane == 0) t = atomicAdd(next, 1u);
-    t = __shfl_sync(0xffffffffu, t, 0);
-    if (t >= (unsigned)ntiles) break;
-    const unsigned tile = __ldg(order + t);
-    const int px = (int)(tile % tiles_x) * kWarpTileW + (lane & (kWarpTileW - 1));
-    const int py = (int)(tile / tiles_x) * kWarpTileH + (lane / kWarpTileW);
-    if (px < a.W && py < a.H) {
-      uint32_t samples, hit;
-      float4 dest = trace_ray<ST, FL, NL, INTEG, GRAD>(a, s_tf, px, py, samples, hit);
-      store_pixel(a, px, py, dest, samples);
-      samples_acc += samples;
-      hits_acc += hit;
-    }
+  using T = GroupTile<S>;
+  const CtaShape cta = cta_shape(blockDim.x);
+  unsigned bx = blockIdx.x, by = blockIdx.y;
+  if (strip) {  // CTAs run up one strip of `strip` columns after the other
+    const unsigned i = by * gridDim.x + bx, col = i / (strip * gridDim.y) * strip, rest = i - col * gridDim.y;
+    const unsigned width = min((unsigned)strip, gridDim.x - col);
+    bx = col + rest % width;
+    by = rest / width;
   }
-  flush_counters(a, samples_acc, hits_acc);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane % (32 / S);
+  const int px = ((int)bx * cta.wx + warp % cta.wx) * T::w + r % T::w;
+  const int py = ((int)by * cta.wy + warp / cta.wx) * T::h + r / T::w;
+  const bool ray = px < a.W && py < a.H;
+  uint32_t samples, hit;
+  const float4 dest = trace_group<ST, FL, NL, INTEG, GRAD, S>(a, s_tf, ray, px, py, samples, hit);
+  const bool store = ray && lane < 32 / S;
+  if (store) store_pixel(a, px, py, dest, samples);
+  flush_counters(a, store ? samples : 0u, store ? hit : 0u);
 }
 
+// CTA and group size by the number of 2x2-ray warp tiles against the warps the chip holds:
+//   fewer tiles than half of them: 16 samples at a time (2x1 rays), the 64^2 preview of a 64^3 field
+//     85 us against 125;
+//   up to twice as many: 64-thread CTAs, which spread over the SMs more evenly (128^2 preview 189 us
+//     against 203 in 128 threads and 234 in 256);
+//   from 16 times as many, lit Euler and Heun kernels: 256-thread CTAs, whose 4x8 rays share more noise
+//     cells in L1 (FP32 512^2 lit frame 27.3 ms against 29.1; FP16 1024^2 57.7 against 58.9); the unlit ones
+//     read a quarter of the cell bytes and lose 1 % by it;
+//   128 threads otherwise.
+// RK4 grids run up strips of 16 CTAs, so that the rays in flight are a block of the image and not a
+// few rows: 2048^2 orbit frame 1379 against 1404 ms, 1024^2 447 against 453 (Heun: 59.6 against 58.9).
 template <int ST, int FL, int NL, int INTEG, bool GRAD>
-static cudaError_t launch_one(const RenderArgs& a, const Schedule& sch, cudaStream_t stream) {
-  if (!sch.order) {
-    dim3 grid((a.W + kTileW - 1) / kTileW, (a.H + kTileH - 1) / kTileH);
-    raycast_kernel<ST, FL, NL, INTEG, GRAD><<<grid, kThreads, 0, stream>>>(a);
-    return cudaGetLastError();
-  }
-  auto kern = raycast_queue_kernel<ST, FL, NL, INTEG, GRAD>;
-  int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, 0);
-  if (e != cudaSuccess) return e;
-  const int grid = std::max(1, per_sm) * sch.num_sms;
-  kern<<<grid, kThreads, 0, stream>>>(a, sch.order, sch.ntiles, sch.next);
+static cudaError_t launch_one(const RenderArgs& a, int num_sms, cudaStream_t stream) {
+  const long long resident = 24ll * num_sms;
+  const long long tiles = (long long)((a.W + 1) / 2) * ((a.H + 1) / 2);
+  const int threads = tiles <= 2 * resident ? 64 : (GRAD && INTEG != VVLIC_RK4 && tiles >= 16 * resident ? 256 : 128);
+  const int strip = INTEG == VVLIC_RK4 ? 16 : 0;
+  const CtaShape cta = cta_shape(threads);
+  const auto grid = [&](int th) {
+    return dim3((unsigned)((a.W + 2 * cta.wx - 1) / (2 * cta.wx)), (unsigned)((a.H + th * cta.wy - 1) / (th * cta.wy)));
+  };
+  if (2 * tiles <= resident)
+    raycast_kernel<ST, FL, NL, INTEG, GRAD, 16><<<grid(GroupTile<16>::h), threads, 0, stream>>>(a, strip);
+  else
+    raycast_kernel<ST, FL, NL, INTEG, GRAD, 8><<<grid(GroupTile<8>::h), threads, 0, stream>>>(a, strip);
   return cudaGetLastError();
 }
 
 template <int ST, int FL, int NL>
-static cudaError_t launch_layout(const RenderArgs& a, int integ, bool grad, const Schedule& sch, cudaStream_t s) {
+static cudaError_t launch_layout(const RenderArgs& a, int integ, bool grad, int num_sms, cudaStream_t s) {
   if (grad) {
-    if (integ == VVLIC_EULER) return launch_one<ST, FL, NL, VVLIC_EULER, true>(a, sch, s);
-    if (integ == VVLIC_HEUN) return launch_one<ST, FL, NL, VVLIC_HEUN, true>(a, sch, s);
-    return launch_one<ST, FL, NL, VVLIC_RK4, true>(a, sch, s);
+    if (integ == VVLIC_EULER) return launch_one<ST, FL, NL, VVLIC_EULER, true>(a, num_sms, s);
+    if (integ == VVLIC_HEUN) return launch_one<ST, FL, NL, VVLIC_HEUN, true>(a, num_sms, s);
+    return launch_one<ST, FL, NL, VVLIC_RK4, true>(a, num_sms, s);
   }
-  if (integ == VVLIC_EULER) return launch_one<ST, FL, NL, VVLIC_EULER, false>(a, sch, s);
-  if (integ == VVLIC_HEUN) return launch_one<ST, FL, NL, VVLIC_HEUN, false>(a, sch, s);
-  return launch_one<ST, FL, NL, VVLIC_RK4, false>(a, sch, s);
+  if (integ == VVLIC_EULER) return launch_one<ST, FL, NL, VVLIC_EULER, false>(a, num_sms, s);
+  if (integ == VVLIC_HEUN) return launch_one<ST, FL, NL, VVLIC_HEUN, false>(a, num_sms, s);
+  return launch_one<ST, FL, NL, VVLIC_RK4, false>(a, num_sms, s);
 }
 
 // Sampler (VVLIC_SAMPLER_*) -> (field layout, noise layout).
 template <int ST>
-static cudaError_t launch_storage(const RenderArgs& a, int sampler, int integ, bool grad, const Schedule& sch,
-                                  cudaStream_t s) {
+static cudaError_t launch_storage(const RenderArgs& a, int sampler, int integ, bool grad, int num_sms, cudaStream_t s) {
   switch (sampler) {
-    case VVLIC_SAMPLER_GATHER: return launch_layout<ST, kGather, kGather>(a, integ, grad, sch, s);
-    case VVLIC_SAMPLER_CELL: return launch_layout<ST, kCell, kCell>(a, integ, grad, sch, s);
+    case VVLIC_SAMPLER_GATHER: return launch_layout<ST, kGather, kGather>(a, integ, grad, num_sms, s);
+    case VVLIC_SAMPLER_CELL: return launch_layout<ST, kCell, kCell>(a, integ, grad, num_sms, s);
     case VVLIC_SAMPLER_TEXTURE:
       if constexpr (ST == VVLIC_STORAGE_BF16) return cudaErrorNotSupported;  // runs as F16 (kernel_storage)
-      else return launch_layout<ST, kTexture, kTexture>(a, integ, grad, sch, s);
+      else return launch_layout<ST, kTexture, kTexture>(a, integ, grad, num_sms, s);
     case VVLIC_SAMPLER_HYBRID:
       if constexpr (ST == VVLIC_STORAGE_BF16) return cudaErrorNotSupported;
-      else return launch_layout<ST, kTexture, kCellFast>(a, integ, grad, sch, s);
+      else return launch_layout<ST, kTexture, kCellFast>(a, integ, grad, num_sms, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -1018,134 +1018,96 @@ __device__ __forceinline__ size_t tape_entry_checked(const RenderArgs& a, int px
   return in_range(a, (long long)e, tape_entries(a), VVLIC_CHECK_TAPE) ? e : 0;
 }
 
-// The whole lic3d_fragment.glsl main() for one pixel: returns dest, counts samples.
-template <int ST, int FL, int NL, int INTEG, bool GRAD>
-__device__ __forceinline__ float4 trace_pixel(const RenderArgs& a, const float* s_tf, int px, int py,
+// Records sample k of the ray at (px, py) on the adjoint tape: intensity, TF coordinate, with
+// gradient lighting the gradient sums, and every kSegment samples the position and the
+// compositing state before the sample.
+template <bool GRAD>
+__device__ __forceinline__ void record_sample(const RenderArgs& a, int px, int py, uint32_t k, float3 pos, float4 dest,
+                                              float4 il, float tfc) {
+  if (k % kSegment == 0 && k / kSegment < (uint32_t)a.tape_nck) {
+    const size_t ce = tape_ck_entry(a, px, py, k / kSegment);
+    if (in_range(a, (long long)ce + 32, tape_ck_entries(a), VVLIC_CHECK_TAPE)) {
+      float4* ck = a.tape_ck + ce;
+      ck[0] = make_float4(pos.x, pos.y, pos.z, 0.f);
+      ck[32] = dest;
+    }
+  }
+  if (k < (uint32_t)a.tape_stride &&
+      in_range(a, (long long)tape_entry(a, px, py, k), tape_entries(a), VVLIC_CHECK_TAPE)) {
+    const size_t e = tape_entry(a, px, py, k);
+    a.tape_is[e] = make_float2(il.w, tfc);
+    if (GRAD) {
+      const __half2 xy = __floats2half2_rn(il.x, il.y), z0 = __floats2half2_rn(il.z, 0.0f);
+      a.tape_g[e] = make_uint2(*reinterpret_cast<const unsigned*>(&xy), *reinterpret_cast<const unsigned*>(&z0));
+    }
+  }
+}
+
+__device__ __forceinline__ float3 march(float3 p, float3 dir, float step) {
+  return f3(fmaf(dir.x, step, p.x), fmaf(dir.y, step, p.y), fmaf(dir.z, step, p.z));
+}
+
+// The whole lic3d_fragment.glsl main() by a warp on a tile of 32 / S rays: lanes r, r + 32/S, ...
+// compute S consecutive samples of ray r side by side, then every lane of the ray composites
+// them in order (4 S shuffles a pass against thousands of instructions of streamline work).  Each
+// sample's LIC runs in one lane and the blends in sample order, so images, sample counts and tapes
+// are those of one lane marching the ray, bit for bit; samples after the one that ends the ray are
+// dropped, and those past the box are not computed.  The nested numIterations loops are one bound
+// of numIterations^2 samples (the outer loop only re-enters the inner one).
+//
+// S > 1 makes work items of 1/S the length (a 512^2 frame has only two 8x4-pixel tiles per resident
+// warp, each as long as its longest ray), keeps lanes together when rays end at different samples,
+// and lets the lanes of a warp read overlapping streamlines: a sample's noise cells are mostly its
+// neighbour's.  `ray` is false for lanes without a pixel.  Every lane of the warp calls.
+template <int ST, int FL, int NL, int INTEG, bool GRAD, int S>
+__device__ __forceinline__ float4 trace_group(const RenderArgs& a, const float* s_tf, bool ray, int px, int py,
                                               uint32_t& samples, uint32_t& hit) {
+  constexpr int R = 32 / S;
+  const int lane = threadIdx.x & 31, k = lane / R, r = lane % R;
+  static_assert(S == 4 || S == 8 || S == 16, "samples per group");
+  const unsigned mine = (S == 4 ? 0x01010101u : (S == 8 ? 0x11111111u : 0x55555555u)) << r;  // this ray's lanes
   float4 dest = make_float4(0.f, 0.f, 0.f, 0.f);
-  float3 pos, dir;
+  float3 pos = f3(0.f, 0.f, 0.f), dir = pos;
   samples = 0;
-  hit = 0;
-  if (!ray_setup(a, px, py, pos, dir)) return dest;
-  hit = 1;
-  float4 src = make_float4(0.f, 0.f, 0.f, 0.f);
-  bool outside = false;
-  for (int j = 0; !outside && j < a.num_iter; ++j) {
-    for (int i = 0; i < a.num_iter; ++i) {
-      const float4 f = Field<ST, FL>::sample(a, pos);
-      const float tfc = a.tf_index == VVLIC_TF_INDEX_MAGNITUDE ? f.w : f.z;
-      const float4 tf = tf_rgba(s_tf, tfc);
-      float4 il = compute_lic<ST, FL, NL, INTEG, GRAD>(a, pos, f);
-      il.w *= a.intensity_scale;
-      if (a.tape_is) {  // record for the adjoint
-        if (samples % kSegment == 0 && samples / kSegment < (uint32_t)a.tape_nck) {
-          const size_t ce = tape_ck_entry(a, px, py, samples / kSegment);
-          if (in_range(a, (long long)ce + 32, tape_ck_entries(a), VVLIC_CHECK_TAPE)) {
-            float4* ck = a.tape_ck + ce;
-            ck[0] = make_float4(pos.x, pos.y, pos.z, 0.f);
-            ck[32] = dest;
-          }
-        }
-        if (samples < (uint32_t)a.tape_stride &&
-            in_range(a, (long long)tape_entry(a, px, py, samples), tape_entries(a), VVLIC_CHECK_TAPE)) {
-          const size_t e = tape_entry(a, px, py, samples);
-          a.tape_is[e] = make_float2(il.w, tfc);
-          if (GRAD) {
-            const __half2 xy = __floats2half2_rn(il.x, il.y), z0 = __floats2half2_rn(il.z, 0.0f);
-            a.tape_g[e] = make_uint2(*reinterpret_cast<const unsigned*>(&xy), *reinterpret_cast<const unsigned*>(&z0));
-          }
-        }
-      }
-      ++samples;
-      src = shade<GRAD>(a, s_tf, il, tf, pos, dir, f);
-      dest = blend(dest, src);
-      pos = add3(pos, scl3(dir, a.step_size));
-      outside = outside_box(a, pos) || src.w > a.alpha_thr;
-      if (outside) break;
-    }
-  }
-  return dest;
-}
-
-// trace_pixel computing the LIC of two consecutive samples together (compute_lic2).  The second
-// sample's LIC is speculative: it is discarded when the first sample ends the ray.  Samples,
-// images and tapes are identical to trace_pixel's; the nested numIterations loops become one
-// bound of numIterations^2 samples (the outer loop only re-enters the inner one).
-template <int ST, int FL, int NL, int INTEG, bool GRAD>
-__device__ __forceinline__ float4 trace_pixel2(const RenderArgs& a, const float* s_tf, int px, int py,
-                                               uint32_t& samples, uint32_t& hit) {
-  float4 dest = make_float4(0.f, 0.f, 0.f, 0.f);
-  float3 pos, dir;
-  samples = 0;
-  hit = 0;
-  if (!ray_setup(a, px, py, pos, dir)) return dest;
-  hit = 1;
+  bool alive = ray && ray_setup(a, px, py, pos, dir);
+  hit = alive;
   const uint32_t max_samples = (uint32_t)a.num_iter * (uint32_t)a.num_iter;
-  const float3 dstep = scl3(dir, a.step_size);
-  while (samples < max_samples) {
-    const float3 pos1 = add3(pos, dstep);
-    const float4 f0 = Field<ST, FL>::sample(a, pos), f1 = Field<ST, FL>::sample(a, pos1);
-    float4 il[2];
-    compute_lic2<ST, FL, NL, INTEG, GRAD>(a, pos, f0, pos1, f1, il[0], il[1]);
-    bool outside = false;
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const float4 f = k == 0 ? f0 : f1;
-      const float3 p = k == 0 ? pos : pos1;
-      const float tfc = a.tf_index == VVLIC_TF_INDEX_MAGNITUDE ? f.w : f.z;
+  for (int j = 0; j < k; ++j) pos = march(pos, dir, a.step_size);
+  while (__any_sync(0xffffffffu, alive)) {
+    const float3 next = march(pos, dir, a.step_size);
+    // the ray leaves the box after this sample, or has no samples left
+    const bool leaves = outside_box(a, next) || samples + k + 1 >= max_samples;
+    const unsigned left = __ballot_sync(0xffffffffu, leaves) & mine;
+    const bool take = alive && (left & ((1u << lane) - 1u)) == 0;
+    float4 src = dest;
+    float4 il = make_float4(0.f, 0.f, 0.f, 0.f);
+    float tfc = 0.0f;
+    if (take) {
+      const float4 f = Field<ST, FL>::sample(a, pos);
+      tfc = a.tf_index == VVLIC_TF_INDEX_MAGNITUDE ? f.w : f.z;
       const float4 tf = tf_rgba(s_tf, tfc);
-      float4 l = il[k];
-      l.w *= a.intensity_scale;
-      if (a.tape_is) {  // record for the adjoint
-        if (samples % kSegment == 0 && samples / kSegment < (uint32_t)a.tape_nck) {
-          const size_t ce = tape_ck_entry(a, px, py, samples / kSegment);
-          if (in_range(a, (long long)ce + 32, tape_ck_entries(a), VVLIC_CHECK_TAPE)) {
-            float4* ck = a.tape_ck + ce;
-            ck[0] = make_float4(p.x, p.y, p.z, 0.f);
-            ck[32] = dest;
-          }
-        }
-        if (samples < (uint32_t)a.tape_stride &&
-            in_range(a, (long long)tape_entry(a, px, py, samples), tape_entries(a), VVLIC_CHECK_TAPE)) {
-          const size_t e = tape_entry(a, px, py, samples);
-          a.tape_is[e] = make_float2(l.w, tfc);
-          if (GRAD) {
-            const __half2 xy = __floats2half2_rn(l.x, l.y), z0 = __floats2half2_rn(l.z, 0.0f);
-            a.tape_g[e] = make_uint2(*reinterpret_cast<const unsigned*>(&xy), *reinterpret_cast<const unsigned*>(&z0));
-          }
-        }
-      }
-      ++samples;
-      const float4 src = shade<GRAD>(a, s_tf, l, tf, p, dir, f);
-      dest = blend(dest, src);
-      // the reference's position update pos += dir * stepSize, then its exit test
-      pos = add3(p, dstep);
-      outside = outside_box(a, pos) || src.w > a.alpha_thr || samples >= max_samples;
-      if (outside) break;
+      il = compute_lic<ST, FL, NL, INTEG, GRAD>(a, pos, f);
+      il.w *= a.intensity_scale;
+      src = shade<GRAD>(a, s_tf, il, tf, pos, dir, f);
     }
-    if (outside) break;
+    const unsigned ends = __ballot_sync(0xffffffffu, leaves || (take && src.w > a.alpha_thr)) & mine;
+    const int last = ends ? __ffs(ends) - 1 : 31;  // lane of the ray's last sample of this pass
+    const bool valid = alive && lane <= last;
+    if (a.tape_is && valid) record_sample<GRAD>(a, px, py, samples + k, pos, dest, il, tfc);
+#pragma unroll (S < 8 ? S : 8)
+    for (int j = 0; j < S; ++j) {
+      const int from = j * R + r;
+      const float4 s = make_float4(__shfl_sync(0xffffffffu, src.x, from), __shfl_sync(0xffffffffu, src.y, from),
+                                   __shfl_sync(0xffffffffu, src.z, from), __shfl_sync(0xffffffffu, src.w, from));
+      if (alive && from <= last) {
+        dest = blend(dest, s);
+        ++samples;
+      }
+    }
+    alive = alive && ends == 0;
+    for (int j = 0; j < S; ++j) pos = march(pos, dir, a.step_size);
   }
   return dest;
-}
-
-// Samples whose LIC one thread computes together: 1 (trace_pixel) or 2 (trace_pixel2, twice the
-// independent gather chains per thread at more registers per thread).  RK4 kernels, whose four
-// serial fetches per step leave a thread mostly waiting, take two: on the 512^3 / 2048^2 RK4
-// orbit frames 106.0 against 103.3 Gsample-steps/s at 128 registers (4 CTAs/SM; 102 registers
-// measured 105.7).  Euler and Heun kernels take one (two measured +1 % on the lit 1024^2 Heun
-// frame with the texture field, -9 % with the cell field).
-#ifndef VVLIC_SAMPLES_PER_PASS
-#define VVLIC_SAMPLES_PER_PASS 1
-#endif
-#ifndef VVLIC_RK4_SAMPLES_PER_PASS
-#define VVLIC_RK4_SAMPLES_PER_PASS 2
-#endif
-template <int ST, int FL, int NL, int INTEG, bool GRAD>
-__device__ __forceinline__ float4 trace_ray(const RenderArgs& a, const float* s_tf, int px, int py,
-                                            uint32_t& samples, uint32_t& hit) {
-  constexpr int spp = INTEG == VVLIC_RK4 ? VVLIC_RK4_SAMPLES_PER_PASS : VVLIC_SAMPLES_PER_PASS;
-  if constexpr (spp == 2) return trace_pixel2<ST, FL, NL, INTEG, GRAD>(a, s_tf, px, py, samples, hit);
-  else return trace_pixel<ST, FL, NL, INTEG, GRAD>(a, s_tf, px, py, samples, hit);
 }
 
 }  // namespace vvlic

@@ -23,8 +23,8 @@ cudaError_t launch_technique_bf16(const RenderArgs& a, const TechArgs& t, int sa
 cudaError_t launch_technique_u8(const RenderArgs& a, const TechArgs& t, int sampler, int integ, bool grad,
                                 cudaStream_t s);
 
-// Work distribution of one render launch: `order` == nullptr selects the static raster grid;
-// otherwise persistent CTAs pull `ntiles` 8x4 tiles in `order` through the counter `next`.
+// Work queue of an adjoint launch: persistent CTAs pull `ntiles` 8x4-pixel tiles in `order` through
+// the counter `next`.
 struct Schedule {
   const uint32_t* order = nullptr;
   int ntiles = 0;
@@ -33,14 +33,10 @@ struct Schedule {
 };
 
 // Forward ray-cast, one launcher per field storage (render_<storage>.cu).
-cudaError_t launch_raycast_f32(const RenderArgs& a, int sampler, int integ, bool grad, const Schedule& sch,
-                               cudaStream_t s);
-cudaError_t launch_raycast_f16(const RenderArgs& a, int sampler, int integ, bool grad, const Schedule& sch,
-                               cudaStream_t s);
-cudaError_t launch_raycast_bf16(const RenderArgs& a, int sampler, int integ, bool grad, const Schedule& sch,
-                                cudaStream_t s);
-cudaError_t launch_raycast_u8(const RenderArgs& a, int sampler, int integ, bool grad, const Schedule& sch,
-                              cudaStream_t s);
+cudaError_t launch_raycast_f32(const RenderArgs& a, int sampler, int integ, bool grad, int num_sms, cudaStream_t s);
+cudaError_t launch_raycast_f16(const RenderArgs& a, int sampler, int integ, bool grad, int num_sms, cudaStream_t s);
+cudaError_t launch_raycast_bf16(const RenderArgs& a, int sampler, int integ, bool grad, int num_sms, cudaStream_t s);
+cudaError_t launch_raycast_u8(const RenderArgs& a, int sampler, int integ, bool grad, int num_sms, cudaStream_t s);
 
 // Adjoint of the unlit (lit == false) or gradient-lit render (adjoint_<storage>.cu):
 // accumulates 64-bit fixed-point gradients into acc (TF 1024, opacity 256, taps).
@@ -89,7 +85,7 @@ inline BatchScratch batch_scratch(unsigned* base, int njobs, int ntiles) {
 // (exclusive prefix of tiles per job).
 cudaError_t launch_batch_order(const BatchScratch& b, int njobs, int ntiles, cudaStream_t s);
 
-// Longest-first tile order for the queue schedule (render.cu): per-tile chord cost, a
+// Longest-first tile order for the adjoint's queue (render.cu): per-tile chord cost, a
 // counting sort over 1024 cost buckets, scatter.  `scratch` holds 2*ntiles + 2048 + 1 words.
 cudaError_t launch_tile_order(const RenderArgs& a, int ntiles, int tiles_x, int shift, unsigned* scratch,
                               cudaStream_t s);
