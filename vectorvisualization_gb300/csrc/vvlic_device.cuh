@@ -1071,12 +1071,14 @@ __device__ __forceinline__ float4 trace_group(const RenderArgs& a, const float* 
   samples = 0;
   bool alive = ray && ray_setup(a, px, py, pos, dir);
   hit = alive;
-  const uint32_t max_samples = (uint32_t)a.num_iter * (uint32_t)a.num_iter;
+  const uint32_t max_samples =
+      a.num_iter > 65535 ? 0xffffffffu : (uint32_t)max(a.num_iter, 0) * (uint32_t)max(a.num_iter, 0);
+  alive = alive && max_samples > 0;
   for (int j = 0; j < k; ++j) pos = march(pos, dir, a.step_size);
   while (__any_sync(0xffffffffu, alive)) {
     const float3 next = march(pos, dir, a.step_size);
     // the ray leaves the box after this sample, or has no samples left
-    const bool leaves = outside_box(a, next) || samples + k + 1 >= max_samples;
+    const bool leaves = outside_box(a, next) || max_samples - samples <= (uint32_t)k + 1;
     const unsigned left = __ballot_sync(0xffffffffu, leaves) & mine;
     const bool take = alive && (left & ((1u << lane) - 1u)) == 0;
     float4 src = dest;
