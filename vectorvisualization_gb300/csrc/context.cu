@@ -702,32 +702,18 @@ extern "C" vvlic_status vvlic_noise_gradients_device(const uint8_t* d_noise, int
   float w27[27];
   noise_filter_weights(w27);
   cudaStream_t s = (cudaStream_t)stream;
-  float* d_grad = nullptr;
-  const size_t bytes = (size_t)mx * my * mz * kNoiseGradBytes;
-  cudaError_t e = cudaMallocAsync((void**)&d_grad, bytes, s);
+  const cudaError_t e = launch_noise_gradients(d_noise, m, mode, sd, d_rgba, w27, s);
   if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? VVLIC_ERR_OUT_OF_MEMORY : VVLIC_ERR_CUDA;
-  e = launch_noise_gradients(d_noise, m, mode, sd, d_grad, d_rgba, w27, s);
-  cudaError_t e2 = cudaFreeAsync(d_grad, s);
-  if (e != cudaSuccess || e2 != cudaSuccess) return VVLIC_ERR_CUDA;
   return VVLIC_OK;
 }
 
-// Upload-buffer layout for noise gradients: the noise bytes, then (256-byte aligned) the raw
-// float gradients (kNoiseGradBytes per voxel).
-static size_t noise_grad_offset(size_t count) { return (count + 255) & ~(size_t)255; }
-static size_t noise_staging_bytes(size_t count) { return noise_grad_offset(count) + count * kNoiseGradBytes; }
-
 // Noise gradients (computeGradients + filterGradients + quantizeGradients + pack) of the noise
-// bytes staged at the start of the context's upload buffer (noise_staging_bytes of capacity),
-// into d_rgba.
+// bytes staged in the context's upload buffer, into d_rgba.
 static vvlic_status noise_gradients_staged(vvlic_ctx* c, const int m[3], int mode, uint8_t* d_rgba) {
-  const size_t count = (size_t)m[0] * m[1] * m[2];
-  const size_t off = noise_grad_offset(count);
   const float sd[3] = {1.f, 1.f, 1.f};
   float w27[27];
   noise_filter_weights(w27);
-  cudaError_t e = launch_noise_gradients((const uint8_t*)c->d_upload, m, mode, sd,
-                                         (float*)((char*)c->d_upload + off), d_rgba, w27, c->stream);
+  cudaError_t e = launch_noise_gradients((const uint8_t*)c->d_upload, m, mode, sd, d_rgba, w27, c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "noise gradients");
   return VVLIC_OK;
 }
@@ -747,7 +733,7 @@ extern "C" vvlic_status vvlic_upload_noise(vvlic_ctx* c, const uint8_t* noise, i
   const int ch = mode == VVLIC_NOISE_SCALAR ? 1 : 4;
   c->tape_valid = false;  // a recorded tape read the previous noise
   if (mode != VVLIC_NOISE_SCALAR) {
-    vvlic_status st = grow(c, &c->d_upload, &c->upload_cap, noise_staging_bytes(count));
+    vvlic_status st = grow(c, &c->d_upload, &c->upload_cap, count);
     if (st) return st;
   }
   // Same extent and layout: rewrite the texels and the cell / texture copies in place once the
@@ -833,9 +819,7 @@ extern "C" vvlic_status vvlic_upload_noise_async(vvlic_ctx* c, const uint8_t* no
   vvlic_status st = ensure_async(c);
   if (st) return st;
   const size_t count = (size_t)mx * my * mz;
-  if ((st = grow_stage(c, &c->d_noise_stage, &c->noise_stage_cap,
-                       mode == VVLIC_NOISE_SCALAR ? count : noise_staging_bytes(count))))
-    return st;
+  if ((st = grow_stage(c, &c->d_noise_stage, &c->noise_stage_cap, count))) return st;
   cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e = cudaStreamWaitEvent(c->copy_stream, c->ev_noise_used, 0);
   if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_noise_stage, noise, count, cudaMemcpyHostToDevice, c->copy_stream);
@@ -848,8 +832,7 @@ extern "C" vvlic_status vvlic_upload_noise_async(vvlic_ctx* c, const uint8_t* no
       const float sd[3] = {1.f, 1.f, 1.f};
       float w27[27];
       noise_filter_weights(w27);
-      e = launch_noise_gradients((const uint8_t*)c->d_noise_stage, m, mode, sd,
-                                 (float*)((char*)c->d_noise_stage + noise_grad_offset(count)), n.d_texels, w27, s);
+      e = launch_noise_gradients((const uint8_t*)c->d_noise_stage, m, mode, sd, n.d_texels, w27, s);
     }
   }
   if (e != cudaSuccess) return cuda_fail(c, e, "upload_noise_async");

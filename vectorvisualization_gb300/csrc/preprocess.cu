@@ -107,88 +107,41 @@ __global__ void field_encode_kernel(const void* xyz, int dtype, size_t count, co
   }
 }
 
-__device__ __forceinline__ float nv(const uint8_t* v, int nx, int ny, int x, int y, int z) {
-  return (float)v[((size_t)z * ny + y) * nx + x];
-}
+// ------------------------------------------------------------------------------------------
+// noise gradients: computeGradients, filterGradients, quantizeGradients and the RGBA pack
+// (gradient.cpp:190-531, dataset.cpp:1270-1286) in one pass over the noise
+// ------------------------------------------------------------------------------------------
+// A CTA owns a 32 x 16 tile of raw gradients and marches it through a run of slices.  A slice's raw
+// gradients go to shared memory once, and every voxel adds its nine neighbours of the slice to
+// the three windows that contain them (those of voxels z + 2, z + 1 and z), so a raw gradient never
+// reaches global memory: 1 byte read and 4 written per voxel remain.  The outputs are the tile
+// without its two low rows and columns, the halo the windows read.
+//
+// Each window's terms are added in the reference's (k, j, i) order with every product and sum
+// rounded by itself, as the reference's CPU code does, so the 81 products and 81 sums of a voxel
+// cannot be merged into FMAs or into a separable filter; x and y go as packed pairs.  Instruction
+// issue is the bound (68 % busy, the FMA pipe 36 %): 430 instructions for a thread's two voxels, a
+// quarter of them for the halo.  512^3 central differences 3604 -> 1405 us, Sobel 2000 us, against
+// the two passes that wrote and re-read 16 bytes of raw gradient per voxel.
+constexpr int kGradTileX = 32, kGradTileY = 16, kGradRows = 2;  // raw gradients per CTA, rows per thread
+constexpr int kGradHalo = 2;
+constexpr int kGradOutX = kGradTileX - kGradHalo, kGradOutY = kGradTileY - kGradHalo;
+constexpr int kGradThreads = kGradTileX * kGradTileY / kGradRows;
 
-// The noise-gradient kernels run one thread per x voxel on a (ceil(nx / kThreads), ny, nz) grid,
-// the y and z extents capped at the grid limit (the kernels step over the rest): a voxel's
-// coordinates come from the block and thread indices without integer division.
-constexpr int kGridYZ = 65535;
-inline dim3 voxel_grid(const int m[3]) {
-  return dim3((unsigned)((m[0] + kThreads - 1) / kThreads), (unsigned)std::min(m[1], kGridYZ),
-              (unsigned)std::min(m[2], kGridYZ));
-}
-
-// computeGradients (gradient.cpp:190-374) for one voxel.
-__global__ void noise_grad_raw_kernel(const uint8_t* v, int nx, int ny, int nz, int mode, float sd0, float sd1,
-                                      float sd2, float4* g) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= nx) return;
-  for (int z = blockIdx.z; z < nz; z += gridDim.z)
-  for (int y = blockIdx.y; y < ny; y += gridDim.y) {
-    const size_t a = ((size_t)z * ny + y) * nx + x;
-    const float sd[3] = {sd0, sd1, sd2};
-    float gp[3];
-    if (mode == VVLIC_NOISE_GRAD_SOBEL && x > 0 && x < nx - 1 && y > 0 && y < ny - 1 && z > 0 && z < nz - 1) {
-      // weights[dir][i+1][j+1][k+1]: the 3x3x3 Sobel masks (gradient.cpp:199-224), summed in
-      // the reference's i, j, k order
-      const int s1[3] = {1, 3, 1}, s2[3] = {3, 6, 3};
-      // the 27 neighbours once; the three masks then run over them in the same i, j, k order
-      float nb[27];
-#pragma unroll
-      for (int i = -1; i < 2; i++)
-#pragma unroll
-        for (int j = -1; j < 2; j++)
-#pragma unroll
-          for (int k = -1; k < 2; k++) nb[((i + 1) * 3 + (j + 1)) * 3 + (k + 1)] = nv(v, nx, ny, x + i, y + j, z + k);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        float acc = 0.0f;
-#pragma unroll
-        for (int i = -1; i < 2; i++)
-#pragma unroll
-          for (int j = -1; j < 2; j++)
-#pragma unroll
-            for (int k = -1; k < 2; k++) {
-              const int o[3] = {i, j, k};
-              const int e = o[d];  // derivative axis offset
-              const int p = o[(d + 1) % 3], q = o[(d + 2) % 3];
-              // mask = sign(e) * w(p) * w(q) with w = (1,3,1) cross (1,3,1) pattern (1,3,1;3,6,3;1,3,1)
-              int w = e == 0 ? 0 : e * ((p == 0 ? s2 : s1)[q + 1]);
-              acc += (float)w * nb[((i + 1) * 3 + (j + 1)) * 3 + (k + 1)];
-            }
-        gp[d] = acc / (2.0f * sd[d]);
-      }
-    } else {
-      // the voxel's neighbours along axis d lie `st[d]` bytes away
-      const uint8_t* cp = v + a;
-      const float c = (float)cp[0];
-      const size_t st[3] = {1, (size_t)nx, (size_t)nx * ny};
-      const int P[3] = {x, y, z}, N[3] = {nx, ny, nz};
-      if (mode == VVLIC_NOISE_GRAD_SOBEL) {
-        // one-sided differences on the border of the Sobel mode
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-          gp[d] = (P[d] < 1) ? ((float)cp[st[d]] - c) / sd[d] : (c - (float)*(cp - st[d])) / sd[d];
-      } else {
-        // central differences (SOBEL 0 branch); the last slice per axis uses a one-sided
-        // difference — those values are never read by the smoothing window below
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          if (P[d] < 1) gp[d] = ((float)cp[st[d]] - c) / sd[d];
-          else if (P[d] >= N[d] - 1) gp[d] = (c - (float)*(cp - st[d])) / sd[d];
-          else gp[d] = ((float)cp[st[d]] - (float)*(cp - st[d])) / sd[d] * 0.5f;
-        }
-      }
-    }
-    g[a] = make_float4(gp[0], gp[1], gp[2], 0.0f);  // padded to 16 bytes: one vector load per filter tap
-  }
-}
-
-struct W27 {
-  float w[27];
+struct GradArgs {
+  const uint8_t* v;
+  uint32_t* out;
+  int nx, ny, nz, zrun;  // slices of output per CTA
+  float sd[3];
+  float w[10];       // window weights by i^2 + j^2 + k^2 (kGradWeight)
+  float minus_zero;  // -0.0f (mul_then_add2)
 };
+// A window weight depends on i^2 + j^2 + k^2 alone (i, j, k in 0..2 from the window's near corner): ten
+// values, kept as register pairs; equal products of a gradient are formed once.
+__host__ __device__ constexpr int grad_weight(int k, int j, int i) {
+  const int d = (2 - k) * (2 - k) + (2 - j) * (2 - j) + (2 - i) * (2 - i);
+  return d < 7 ? d : (d == 8 ? 7 : (d == 9 ? 8 : 9));
+}
 
 // (unsigned char)(((double)c + 1.0) / 2.0 * 255.0), quantizeGradients' conversion of a unit
 // component c (gradient.cpp:466-477), without double arithmetic for almost every input.  The
@@ -209,66 +162,234 @@ __device__ __forceinline__ unsigned char quantize_unit(float c) {
   return quantize_unit_double(c);
 }
 
-// filterGradients + quantize8 + RGBA pack (gradient.cpp:377-478, dataset.cpp:1270-1286).
-__global__ void noise_grad_filter_kernel(const uint8_t* v, const float4* g, int nx, int ny, int nz,
-                                         const __grid_constant__ W27 fw27,
-                                         uint8_t* out) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= nx) return;
-  for (int z = blockIdx.z; z < nz; z += gridDim.z)
-  for (int y = blockIdx.y; y < ny; y += gridDim.y) {
-    const size_t a = ((size_t)z * ny + y) * nx + x;
-    int bd = min(min(min(x, nx - x - 1), min(y, ny - y - 1)), min(z, nz - z - 1));
-    const int fw = min(2, bd);
-    // One pass over the window with the three channel sums side by side: each channel adds its
-    // terms in the reference's (k, j, i) order, so the sums are the per-channel loops' bit for bit.
-    float acc[3] = {0.0f, 0.0f, 0.0f};
-    if (fw == 2) {  // interior: k, j, i in {-2, -1, 0}, table entries (k+2, j+2, i+2)
+// The window sum's RGBA texel as the reference computes it: length, three divisions and the
+// conversion.  In a call of its own: few voxels need it (pack_gradient).
+__device__ __noinline__ uint32_t pack_gradient_exact(float x, float y, float z, unsigned value) {
+  const float len = sqrtf(x * x + y * y + z * z);
+  if (len < 1e-5f) {
+    x = y = z = 0.0f;
+  } else {
+    x /= len;
+    y /= len;
+    z /= len;
+  }
+  return (uint32_t)quantize_unit(x) | ((uint32_t)quantize_unit(y) << 8) | ((uint32_t)quantize_unit(z) << 16) |
+         (value << 24);
+}
+
+// The same texel from one reciprocal square root when no component lies near a step.  With s the
+// float sum of squares, t = fma(c * rsqrt(s), 127.5, 127.5) differs from (q + 1) * 127.5 of the
+// reference's float quotient q by less than 6.2e-5: rsqrtf is good to 2 ulp, the product, the
+// reference's square root and its division to half an ulp each (3.5 * 2^-23 of at most 127.5), and
+// the FMA rounds by 2^-17.  Where t lies more than 2e-4 from an integer both truncate alike; about one
+// voxel in 800 takes the exact form, and those whose length the 1e-5 cut may decide.
+__device__ __forceinline__ uint32_t pack_gradient(float x, float y, float z, unsigned value) {
+  const float s = x * x + y * y + z * z;
+  const float inv = rsqrtf(s);
+  const float tx = fmaf(x * inv, 127.5f, 127.5f), ty = fmaf(y * inv, 127.5f, 127.5f), tz = fmaf(z * inv, 127.5f, 127.5f);
+  const float fx = floorf(tx), fy = floorf(ty), fz = floorf(tz);
+  const float rx = tx - fx, ry = ty - fy, rz = tz - fz;
+  const float lo = fminf(fminf(rx, ry), rz), hi = fmaxf(fmaxf(rx, ry), rz);
+  // (comparisons false for NaN)
+  if (s > 1e-8f && lo > 2e-4f && hi < 1.0f - 2e-4f)
+    return (uint32_t)(int)fx | ((uint32_t)(int)fy << 8) | ((uint32_t)(int)fz << 16) | (value << 24);
+  return pack_gradient_exact(x, y, z, value);
+}
+
+// acc + w * v per component, the product and the sum each rounded.  The assembler merges a packed
+// multiplication and addition into one FMA even in their .rn forms and with -fmad=false (one byte in
+// 10^5 came out off by one), so the product is formed as fma(w, v, -0), whose -0 it cannot see.
+__device__ __forceinline__ float2 mul_then_add2(float2 w, float2 v, float2 acc, float2 minus_zero) {
+  return __fadd2_rn(acc, __ffma2_rn(w, v, minus_zero));
+}
+
+// What a noise slice contributes to raw gradients at one voxel: d along x and y, and for SOBEL the
+// partial sums of the 3x3x3 masks (gradient.cpp:199-224: weight 1, 3 or 6 by the two axes across,
+// 3 times heavier in the derivative's own plane; sums of bytes, exact in float in any order).
+template <bool SOBEL> struct GradSlice;
+template <> struct GradSlice<false> {
+  float c, dx, dy;
+};
+template <> struct GradSlice<true> {
+  float c, x1, x3, y1, y3, s;  // d/dx and d/dy of the (1,3,1) and (3,6,3) sums, sum over the plane
+};
+
+// Both rows of a thread in one slice.  v: the slice (the same for the whole CTA); o: 32-bit offsets of the
+// row below, the two rows and the row above, each that of the nearest row inside; xm, xp: those of
+// the x neighbours (0 outside the volume).  The rows are each other's y neighbours.
+template <bool SOBEL>
+__device__ __forceinline__ void grad_slices(const uint8_t* v, const unsigned (&o)[4], int xm, int xp,
+                                            GradSlice<SOBEL> (&g)[kGradRows]) {
+  if constexpr (SOBEL) {
+    float n[4][3];
 #pragma unroll
-      for (int k = -2; k < 1; ++k)
-#pragma unroll
-        for (int j = -2; j < 1; ++j) {
-          const float4* row = g + ((size_t)(z + k) * ny + (y + j)) * nx + x;
-#pragma unroll
-          for (int i = -2; i < 1; ++i) {
-            const float w = fw27.w[((k + 2) * 3 + (j + 2)) * 3 + (i + 2)];
-            const float4 q = row[i];
-            acc[0] += w * q.x;
-            acc[1] += w * q.y;
-            acc[2] += w * q.z;
-          }
-        }
-    } else {
-      for (int k = -fw; k < fw - 1; ++k)
-        for (int j = -fw; j < fw - 1; ++j)
-          for (int i = -fw; i < fw - 1; ++i) {
-            // the reference indexes its 5x5x5 table with the shrunken fw; only entries with
-            // all three indices in [0, 2] are ever used
-            const int wk = fw + k, wj = fw + j, wi = fw + i;
-            const float w = fw27.w[(wk * 3 + wj) * 3 + wi];
-            const float4 q = g[((size_t)(z + k) * ny + (y + j)) * nx + (x + i)];
-            acc[0] += w * q.x;
-            acc[1] += w * q.y;
-            acc[2] += w * q.z;
-          }
+    for (int i = 0; i < 4; ++i) {
+      n[i][0] = (float)v[o[i] + xm];
+      n[i][1] = (float)v[o[i]];
+      n[i][2] = (float)v[o[i] + xp];
     }
-    float len = sqrtf(acc[0] * acc[0] + acc[1] * acc[1] + acc[2] * acc[2]);
-    if (len < 1e-5f) {
-      acc[0] = acc[1] = acc[2] = 0.0f;
-    } else {
-      acc[0] /= len;
-      acc[1] /= len;
-      acc[2] /= len;
+#pragma unroll
+    for (int q = 0; q < kGradRows; ++q) {
+      const float *lo = n[q], *mi = n[q + 1], *hi = n[q + 2];
+      g[q].c = mi[1];
+      g[q].x1 = (lo[2] - lo[0]) + 3.0f * (mi[2] - mi[0]) + (hi[2] - hi[0]);
+      g[q].x3 = 3.0f * (lo[2] - lo[0]) + 6.0f * (mi[2] - mi[0]) + 3.0f * (hi[2] - hi[0]);
+      g[q].y1 = (hi[0] - lo[0]) + 3.0f * (hi[1] - lo[1]) + (hi[2] - lo[2]);
+      g[q].y3 = 3.0f * (hi[0] - lo[0]) + 6.0f * (hi[1] - lo[1]) + 3.0f * (hi[2] - lo[2]);
+      g[q].s = lo[0] + lo[2] + hi[0] + hi[2] + 3.0f * (lo[1] + mi[0] + mi[2] + hi[1]) + 6.0f * mi[1];
     }
-    uchar4 o;
-    o.x = quantize_unit(acc[0]);
-    o.y = quantize_unit(acc[1]);
-    o.z = quantize_unit(acc[2]);
-    o.w = v[a];
-    reinterpret_cast<uchar4*>(out)[a] = o;
+  } else {
+    g[0].c = (float)v[o[1]];
+    g[1].c = (float)v[o[2]];
+    g[0].dx = (float)v[o[1] + xp] - (float)v[o[1] + xm];
+    g[1].dx = (float)v[o[2] + xp] - (float)v[o[2] + xm];
+    g[0].dy = g[1].c - (float)v[o[0]];
+    g[1].dy = (float)v[o[3]] - g[0].c;
   }
 }
 
+// CTAs per SM: 4 at 64 registers for central differences (512^3 in 1405 us; 3 at 80 registers 1449, 2 at
+// 104 1655), 3 for Sobel, whose slices hold twice the values (1995 us against 2415 at 4).
+template <bool SOBEL, bool UNIT>
+__global__ void __launch_bounds__(kGradThreads, SOBEL ? 3 : 4) noise_gradient_kernel(const __grid_constant__ GradArgs a) {
+  // raw gradients of the current and the previous slice, (x, y) pairs and z; a third buffer lets the
+  // next slice be written while slower warps still read these (one barrier a slice)
+  __shared__ float2 s_xy[3][kGradTileY][kGradTileX];
+  __shared__ float s_z[3][kGradTileY][kGradTileX];
+  const int tx = threadIdx.x, ty = threadIdx.y * kGradRows;
+  const int x = (int)blockIdx.x * kGradOutX - kGradHalo + tx;
+  const int y0 = (int)blockIdx.y * kGradOutY - kGradHalo + ty;
+  const int z0 = (int)blockIdx.z * a.zrun, z1 = min(z0 + a.zrun, a.nz);
+  // voxels outside the volume stand in for the nearest inside; no window reads their gradients
+  const int xc = min(max(x, 0), a.nx - 1);
+  const int xm = xc > 0 ? -1 : 0, xp = xc < a.nx - 1 ? 1 : 0;
+  int yc[4];
+  unsigned o[4];  // below, first row, second row, above
+  yc[1] = min(max(y0, 0), a.ny - 1);
+  yc[2] = min(max(y0 + 1, 0), a.ny - 1);
+  yc[0] = max(yc[1] - 1, 0);
+  yc[3] = min(yc[2] + 1, a.ny - 1);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) o[i] = (unsigned)yc[i] * (unsigned)a.nx + (unsigned)xc;
+  const size_t slice = (size_t)a.nx * a.ny;
+  const bool writes = tx >= kGradHalo && ty >= kGradHalo;
+  int edge[kGradRows];  // distance to the volume's x and y borders, below 0 for rows outside
+#pragma unroll
+  for (int q = 0; q < kGradRows; ++q) edge[q] = min(min(x, a.nx - 1 - x), min(y0 + q, a.ny - 1 - (y0 + q)));
+  const int zs = max(z0 - kGradHalo, 0);
+  const float2 zero = make_float2(0.0f, 0.0f), nz = make_float2(a.minus_zero, a.minus_zero);
+  float2 w2[10];
+#pragma unroll
+  for (int i = 0; i < 10; ++i) w2[i] = make_float2(a.w[i], a.w[i]);
+  // rings of three, their slots named by the phase (s - zs) % 3 so that nothing is moved: noise
+  // slices s - 1, s, s + 1, and the windows of voxels s + 2 (one slice in), s + 1 (two) and s (three)
+  GradSlice<SOBEL> ring[3][kGradRows];
+  float2 xy[3][kGradRows];
+  float zz[3][kGradRows];
+  grad_slices<SOBEL>(a.v + max(zs - 1, 0) * slice, o, xm, xp, ring[0]);
+  grad_slices<SOBEL>(a.v + zs * slice, o, xm, xp, ring[1]);
+  grad_slices<SOBEL>(a.v + min(zs + 1, a.nz - 1) * slice, o, xm, xp, ring[2]);
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int q = 0; q < kGradRows; ++q) {
+      xy[k][q] = zero;
+      zz[k][q] = 0.0f;
+    }
+  const auto step = [&](auto phase, int s) {
+    constexpr int P0 = decltype(phase)::value, P1 = (P0 + 1) % 3, P2 = (P0 + 2) % 3;
+    auto &prev = ring[P0], &cur = ring[P1], &next = ring[P2];
+    GradSlice<SOBEL> ahead[kGradRows];  // two slices on, so that its loads have a slice's time
+    grad_slices<SOBEL>(a.v + min(s + 2, a.nz - 1) * slice, o, xm, xp, ahead);
+#pragma unroll
+    for (int q = 0; q < kGradRows; ++q) {
+      // computeGradients (gradient.cpp:190-374): the Sobel sum inside, one-sided differences on its
+      // border; central differences (SOBEL 0), one-sided on the border
+      float g[3];
+      const int P[3] = {xc, yc[1 + q], s}, N[3] = {a.nx, a.ny, a.nz};
+      if constexpr (SOBEL) {
+        const bool inside = xc > 0 && xc < a.nx - 1 && yc[1 + q] > 0 && yc[1 + q] < a.ny - 1 && s > 0 && s < a.nz - 1;
+        if (inside) {
+          g[0] = prev[q].x1 + cur[q].x3 + next[q].x1;
+          g[1] = prev[q].y1 + cur[q].y3 + next[q].y1;
+          g[2] = next[q].s - prev[q].s;
+#pragma unroll
+          for (int d = 0; d < 3; ++d) g[d] = UNIT ? g[d] * 0.5f : g[d] / (2.0f * a.sd[d]);
+        } else {
+          const uint8_t* cp = a.v + s * slice + o[1 + q];
+          const size_t st[3] = {1, (size_t)a.nx, slice};
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            g[d] = P[d] >= 1 ? cur[q].c - (float)*(cp - st[d]) : (N[d] > 1 ? (float)cp[st[d]] - cur[q].c : 0.0f);
+            if (!UNIT) g[d] = g[d] / a.sd[d];
+          }
+        }
+      } else {
+        // outside neighbours stand in for the voxel itself: the difference is the one-sided one
+        g[0] = cur[q].dx;
+        g[1] = cur[q].dy;
+        g[2] = next[q].c - (s > 0 ? prev[q].c : cur[q].c);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          if (!UNIT) g[d] = g[d] / a.sd[d];
+          if (P[d] >= 1 && P[d] < N[d] - 1) g[d] = g[d] * 0.5f;
+        }
+      }
+      s_xy[P0][ty + q][tx] = make_float2(g[0], g[1]);
+      s_z[P0][ty + q][tx] = g[2];
+      prev[q] = ahead[q];
+    }
+    __syncthreads();
+    if (!writes) return;
+    // rows ty - 2 .. ty + 1 of the slice: row r is window row j = r - q of output row q.  Slots: the
+    // window one slice in is in P2, two in P1, three (finished here) in P0.
+#pragma unroll
+    for (int r = 0; r < kGradRows + 2; ++r) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const float2 gxy = s_xy[P0][ty - 2 + r][tx - 2 + i];
+        const float gz = s_z[P0][ty - 2 + r][tx - 2 + i];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const int slot = k == 0 ? P2 : (k == 1 ? P1 : P0);
+#pragma unroll
+          for (int q = 0; q < kGradRows; ++q) {
+            if (r < q || r - q > 2) continue;
+            const int w = grad_weight(k, r - q, i);
+            xy[slot][q] = mul_then_add2(w2[w], gxy, xy[slot][q], nz);
+            zz[slot][q] = __fadd_rn(zz[slot][q], __fmul_rn(a.w[w], gz));
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kGradRows; ++q) {
+      if (s >= z0 && edge[q] >= 0) {
+        // filterGradients' window shrinks towards the border (gradient.cpp:423-444): whole from two
+        // voxels in, its far corner one voxel in, empty on the border
+        const int bd = min(edge[q], min(s, a.nz - 1 - s));
+        float ax = xy[P0][q].x, ay = xy[P0][q].y, az = zz[P0][q];
+        if (bd < 2) {
+          ax = ay = az = 0.0f;
+          if (bd == 1) {
+            const float2 c = s_xy[P2][ty + q - 1][tx - 1];
+            ax = a.w[9] * c.x;
+            ay = a.w[9] * c.y;
+            az = a.w[9] * s_z[P2][ty + q - 1][tx - 1];
+          }
+        }
+        (a.out + s * slice)[o[1 + q]] = pack_gradient(ax, ay, az, (unsigned)cur[q].c);
+      }
+      xy[P0][q] = zero;
+      zz[P0][q] = 0.0f;
+    }
+  };
+  for (int s = zs; s < z1; s += 3) {
+    step(std::integral_constant<int, 0>(), s);
+    if (s + 1 < z1) step(std::integral_constant<int, 1>(), s + 1);
+    if (s + 2 < z1) step(std::integral_constant<int, 2>(), s + 2);
+  }
+}
 
 // cell c per axis covers texels clamp(c-1), clamp(c): (n+1)^3 cells of 8 texels
 template <int ST>
@@ -432,13 +553,35 @@ cudaError_t launch_encode_field(const void* d_xyz, int dtype, const int n[3], in
   return cudaGetLastError();
 }
 
-cudaError_t launch_noise_gradients(const uint8_t* d_noise, const int m[3], int mode, const float sd[3], float* d_grad,
-                                   uint8_t* d_rgba, const float w27[27], cudaStream_t s) {
-  float4* g4 = reinterpret_cast<float4*>(d_grad);
-  noise_grad_raw_kernel<<<voxel_grid(m), kThreads, 0, s>>>(d_noise, m[0], m[1], m[2], mode, sd[0], sd[1], sd[2], g4);
-  W27 w;
-  for (int i = 0; i < 27; ++i) w.w[i] = w27[i];
-  noise_grad_filter_kernel<<<voxel_grid(m), kThreads, 0, s>>>(d_noise, g4, m[0], m[1], m[2], w, d_rgba);
+cudaError_t launch_noise_gradients(const uint8_t* d_noise, const int m[3], int mode, const float sd[3], uint8_t* d_rgba,
+                                   const float w27[27], cudaStream_t s) {
+  GradArgs a;
+  a.v = d_noise;
+  a.out = reinterpret_cast<uint32_t*>(d_rgba);
+  a.nx = m[0];
+  a.ny = m[1];
+  a.nz = m[2];
+  for (int i = 0; i < 3; ++i) a.sd[i] = sd[i];
+  for (int k = 0; k < 3; ++k)
+    for (int j = 0; j < 3; ++j)
+      for (int i = 0; i < 3; ++i) a.w[grad_weight(k, j, i)] = w27[(k * 3 + j) * 3 + i];
+  a.minus_zero = -0.0f;
+  const int bx = (m[0] + kGradOutX - 1) / kGradOutX, by = (m[1] + kGradOutY - 1) / kGradOutY;
+  // Slices per CTA: two more are computed than written, so long runs, but enough CTAs to fill the
+  // chip four times over at three per SM; at most 65535 runs (grid limit).
+  const long long ctas = 152 * 12;
+  a.zrun = (int)std::min<long long>(std::max<long long>(((long long)m[2] * bx * by + ctas - 1) / ctas, 8), 64);
+  a.zrun = std::max(a.zrun, (m[2] + 65534) / 65535);
+  const dim3 grid((unsigned)bx, (unsigned)by, (unsigned)((m[2] + a.zrun - 1) / a.zrun));
+  const dim3 block(kGradTileX, kGradTileY / kGradRows);
+  const bool unit = sd[0] == 1.0f && sd[1] == 1.0f && sd[2] == 1.0f;  // division by 1 is exact: left out
+  if (mode == VVLIC_NOISE_GRAD_SOBEL) {
+    if (unit) noise_gradient_kernel<true, true><<<grid, block, 0, s>>>(a);
+    else noise_gradient_kernel<true, false><<<grid, block, 0, s>>>(a);
+  } else {
+    if (unit) noise_gradient_kernel<false, true><<<grid, block, 0, s>>>(a);
+    else noise_gradient_kernel<false, false><<<grid, block, 0, s>>>(a);
+  }
   return cudaGetLastError();
 }
 
