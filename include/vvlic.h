@@ -591,8 +591,7 @@ const char* vvlic_io_error(void);
 
 /* computeGradients/filterGradients/quantizeGradients + RGBA pack (gradient.cpp:190-531,
  * dataset.cpp:1270-1286) on device buffers: d_noise (mx*my*mz uint8) -> d_rgba (4 bytes per
- * voxel: quantised gradient xyz, noise).  mode is VVLIC_NOISE_GRAD_SOBEL or _CENTRAL.
- * Allocates a temporary float gradient buffer of 12 bytes per voxel. */
+ * voxel: quantised gradient xyz, noise).  mode is VVLIC_NOISE_GRAD_SOBEL or _CENTRAL. */
 vvlic_status vvlic_noise_gradients_device(const uint8_t* d_noise, int32_t mx, int32_t my,
                                           int32_t mz, int32_t mode, const float* slice_dist,
                                           uint8_t* d_rgba, void* stream);

@@ -52,3 +52,29 @@ def test_texture_copy_holds_every_texel(ctx, storage, dims):
     assert float(ref[..., 3].max()) > 0
     tol = (2e-6 if storage == "f32" else 2.0 ** -11) * max(1.0, 128.0 * p.step_size_vol)
     np.testing.assert_allclose(img, ref, rtol=0, atol=tol)
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16", "bf16", "u8"])
+@pytest.mark.parametrize("dims", [(1, 1, 1), (8, 4, 8), (9, 5, 7), (31, 33, 9), (33, 8, 17), (70, 3, 2)])
+def test_update_writes_texels_and_arrays(ctx, storage, dims):
+    """The update's encode writes texels and texture arrays in one kernel: the frame, and the texels
+    read back, are those of a fresh upload bit for bit (32 x 8 x 8 voxel tiles and their remainders)."""
+    nx, ny, nz = dims
+    rng = np.random.default_rng(sum(dims))
+    a, b = (rng.standard_normal((nz, ny, nx, 3)).astype(np.float32) for _ in range(2))
+    ctx.upload_noise(rng.integers(0, 256, (8, 8, 8)).astype(np.uint8))
+    p = capi.params_default()
+    p.steps_backward = p.steps_forward = 4
+    p.tf_index = capi.TF_INDEX_MAGNITUDE
+    ctx.set_params(p)
+    ext = np.array(dims, np.float64) / max(dims)
+    ctx.set_view(wl.ortho_view(center=(ext[0] / 2, ext[1] / 2, 0.0), right=(ext[0] / 2, 0, 0), up=(0, ext[1] / 2, 0)))
+    updated = ctx.upload_field(a, storage=storage)
+    first = ctx.render(updated, 48, 40)
+    ctx.update_field(updated, b)
+    fresh = ctx.upload_field(b, storage=storage)
+    img = ctx.render(updated, 48, 40)
+    np.testing.assert_array_equal(img, ctx.render(fresh, 48, 40))
+    np.testing.assert_array_equal(ctx.download_field(updated, dims, storage), ctx.download_field(fresh, dims, storage))
+    if nx * ny * nz > 1:
+        assert not np.array_equal(img, first)

@@ -449,7 +449,7 @@ static vvlic_status encode_into_volume(vvlic_ctx* c, const void* d_xyz, int dtyp
   v.texel_bytes = count * texel_bytes(storage);
   cudaError_t e = cudaMalloc(&v.d_texels, v.texel_bytes);
   if (e != cudaSuccess) return cuda_fail(c, e, "field allocation");
-  e = launch_encode_field(d_xyz, dtype, n, storage, v.d_texels, c->d_scratch_word, s);
+  e = launch_encode_field(d_xyz, dtype, n, storage, v.d_texels, c->d_scratch_word, nullptr, s);
   if (e != cudaSuccess) {
     free_volume(v);
     return cuda_fail(c, e, "field encoding");
@@ -523,13 +523,11 @@ extern "C" vvlic_status vvlic_upload_field_interp(vvlic_ctx* c, const void* xyz0
 // Re-encodes the raw vectors at d_xyz into the existing volume and rewrites its cell and texture
 // copies, on the context stream; the caller has waited for renders that read the old texels.
 static vvlic_status reencode_volume(vvlic_ctx* c, int32_t vol_id, Volume& v, const void* d_xyz, int dtype) {
-  cudaError_t e = launch_encode_field(d_xyz, dtype, v.n, v.storage, v.d_texels, c->d_scratch_word, c->stream);
-  if (e != cudaSuccess) return cuda_fail(c, e, "field encoding");
-  vvlic_status st = refresh_volume_layouts(c, v, c->stream);
+  vvlic_status st = encode_volume(c, v, d_xyz, dtype, c->stream);
   if (st) return st;
   v.licvol_valid = false;  // the precomputed LIC volume belongs to the previous field
   if (c->tape_vol == vol_id) c->tape_valid = false;
-  e = cudaStreamSynchronize(c->stream);
+  cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "field update");
   return VVLIC_OK;
 }
@@ -626,9 +624,8 @@ extern "C" vvlic_status vvlic_update_field_async(vvlic_ctx* c, int32_t vol_id, c
   if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_field_stage, xyz, bytes, cudaMemcpyHostToDevice, c->copy_stream);
   if (e == cudaSuccess) e = cudaEventRecord(c->ev_field_copied, c->copy_stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(s, c->ev_field_copied, 0);
-  if (e == cudaSuccess) e = launch_encode_field(c->d_field_stage, dtype, v->n, v->storage, v->d_texels, c->d_scratch_word, s);
   if (e != cudaSuccess) return cuda_fail(c, e, "update_field_async");
-  if ((st = refresh_volume_layouts(c, *v, s))) return st;
+  if ((st = encode_volume(c, *v, c->d_field_stage, dtype, s))) return st;
   e = cudaEventRecord(c->ev_field_used, s);
   if (e != cudaSuccess) return cuda_fail(c, e, "update_field_async");
   v->licvol_valid = false;
@@ -645,9 +642,7 @@ extern "C" vvlic_status vvlic_update_field_device(vvlic_ctx* c, int32_t vol_id, 
   if (st) return st;
   DeviceGuard g(c->device);
   cudaStream_t s = (cudaStream_t)stream;
-  cudaError_t e = launch_encode_field(d_xyz, VVLIC_DTYPE_FLOAT32, v->n, v->storage, v->d_texels, c->d_scratch_word, s);
-  if (e != cudaSuccess) return cuda_fail(c, e, "update_field_device");
-  if ((st = refresh_volume_layouts(c, *v, s))) return st;
+  if ((st = encode_volume(c, *v, d_xyz, VVLIC_DTYPE_FLOAT32, s))) return st;
   v->licvol_valid = false;
   if (c->tape_vol == vol_id) c->tape_valid = false;
   return VVLIC_OK;

@@ -38,15 +38,39 @@ __device__ __forceinline__ float voxel_len(const void* xyz, int dtype, size_t a,
   return len < 1e-5f ? 0.0f : len;
 }
 
-__global__ void field_maxlen_kernel(const void* xyz, int dtype, size_t count, unsigned* maxbits) {
+// The largest magnitude of the field: four FP32 vectors per thread and iteration in three 16-byte
+// loads (VEC: 16-byte aligned input), one atomicMax per CTA.  Bound by memory; one atomic per warp on
+// the single word cost 46 us on a 128^3 field whose vectors take 12 us to read.
+template <bool VEC> __global__ void field_maxlen_kernel(const void* xyz, int dtype, size_t count, unsigned* maxbits) {
   float m = 0.0f;
-  for (size_t a = blockIdx.x * (size_t)blockDim.x + threadIdx.x; a < count; a += (size_t)gridDim.x * blockDim.x) {
+  const size_t first = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+  size_t rest = 0;
+  if (VEC) {
+    const float4* q = reinterpret_cast<const float4*>(xyz);
+    for (size_t g = first; g < count / 4; g += step) {
+      const float4 a = __ldg(q + 3 * g), b = __ldg(q + 3 * g + 1), c = __ldg(q + 3 * g + 2);
+      const float v[4][3] = {{a.x, a.y, a.z}, {a.w, b.x, b.y}, {b.z, b.w, c.x}, {c.y, c.z, c.w}};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float len = vlen_f32(v[i]);
+        m = fmaxf(m, len < 1e-5f ? 0.0f : len);
+      }
+    }
+    rest = count / 4 * 4;
+  }
+  for (size_t a = rest + first; a < count; a += step) {
     unsigned char t[3];
     m = fmaxf(m, voxel_len(xyz, dtype, a, t));
   }
   // non-negative floats order like their bit patterns
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(maxbits, __float_as_uint(m));
+  __shared__ unsigned s_max[kThreads / 32];
+  const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = w;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const unsigned b = __reduce_max_sync(0xffffffffu, threadIdx.x < kThreads / 32 ? s_max[threadIdx.x] : 0u);
+    if (threadIdx.x == 0) atomicMax(maxbits, b);
+  }
 }
 
 // The machine word(s) of one texel.
@@ -56,54 +80,119 @@ template <int ST> struct TexelWord {
 };
 
 template <int ST>
-__device__ __forceinline__ void store_texel(void* out, size_t a, float r, float g, float b, float al) {
-  if (ST == VVLIC_STORAGE_F32) {
-    reinterpret_cast<float4*>(out)[a] = make_float4(r, g, b, al);
-  } else if (ST == VVLIC_STORAGE_F16) {
+__device__ __forceinline__ typename TexelWord<ST>::type encode_texel(float r, float g, float b, float al) {
+  if constexpr (ST == VVLIC_STORAGE_F32) {
+    return make_float4(r, g, b, al);
+  } else if constexpr (ST == VVLIC_STORAGE_F16) {
     __half2 lo = __halves2half2(__float2half_rn(r), __float2half_rn(g));
     __half2 hi = __halves2half2(__float2half_rn(b), __float2half_rn(al));
     uint2 v;
     v.x = *reinterpret_cast<unsigned*>(&lo);
     v.y = *reinterpret_cast<unsigned*>(&hi);
-    reinterpret_cast<uint2*>(out)[a] = v;
-  } else if (ST == VVLIC_STORAGE_UNORM8) {
+    return v;
+  } else if constexpr (ST == VVLIC_STORAGE_UNORM8) {
     // nearest multiple of 1/255 (x*255 rounded in float, then to nearest integer)
     const unsigned q0 = __float2uint_rn(r * 255.0f), q1 = __float2uint_rn(g * 255.0f),
                    q2 = __float2uint_rn(b * 255.0f), q3 = __float2uint_rn(al * 255.0f);
-    reinterpret_cast<uint32_t*>(out)[a] = min(q0, 255u) | (min(q1, 255u) << 8) | (min(q2, 255u) << 16) |
-                                          (min(q3, 255u) << 24);
+    return min(q0, 255u) | (min(q1, 255u) << 8) | (min(q2, 255u) << 16) | (min(q3, 255u) << 24);
   } else {
     __nv_bfloat16 br = __float2bfloat16_rn(r), bg = __float2bfloat16_rn(g), bb = __float2bfloat16_rn(b),
                   ba = __float2bfloat16_rn(al);
     uint2 v;
     v.x = (unsigned)*reinterpret_cast<unsigned short*>(&br) | ((unsigned)*reinterpret_cast<unsigned short*>(&bg) << 16);
     v.y = (unsigned)*reinterpret_cast<unsigned short*>(&bb) | ((unsigned)*reinterpret_cast<unsigned short*>(&ba) << 16);
-    reinterpret_cast<uint2*>(out)[a] = v;
+    return v;
   }
 }
 
+// Voxel tiles of the kernels that write texture arrays: a CTA takes 32 x 8 voxels of kTileZ slices, a warp
+// 8 x 4 of them, so that its writes of 8-byte texels fill 64-byte rows of the arrays' block-linear
+// tiles next to one another.  Bound by memory: 5.8 TB/s of DRAM traffic in the encode, 6.4 in the
+// maximum pass.  512^3 half4 field update and its frame: 1612 us with the arrays filled from the texels,
+// 1322 us filled by an encode in rows of 32 voxels, 960 us so (one slice per thread 1082, four 967).
+constexpr int kTileZ = 8;
+inline dim3 tile_grid(const int n[3]) {
+  return dim3((unsigned)((n[0] + 31) / 32), (unsigned)((n[1] + 7) / 8), (unsigned)((n[2] + kTileZ - 1) / kTileZ));
+}
+__device__ __forceinline__ bool tile_voxel(int nx, int ny, int& x, int& y) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  x = (int)blockIdx.x * 32 + (warp & 3) * 8 + (lane & 7);
+  y = (int)blockIdx.y * 8 + (warp >> 2) * 4 + (lane >> 3);
+  return x < nx && y < ny;
+}
+
+// The texel of voxel (x, y, z) into the volume's texture arrays.
+template <int ST>
+__device__ __forceinline__ void store_array(const FieldSurfaces& s, int x, int y, int z,
+                                            typename TexelWord<ST>::type t) {
+  if constexpr (ST == VVLIC_STORAGE_F32) {
+    surf3Dwrite(make_float2(t.x, t.y), s.rgba, x * 8, y, z);
+    surf3Dwrite(t.z, s.z, x * 4, y, z);
+    surf3Dwrite(t.w, s.w, x * 4, y, z);
+  } else if constexpr (ST == VVLIC_STORAGE_BF16) {
+    const __half2 lo = __floats2half2_rn(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xffff0000u));
+    const __half2 hi = __floats2half2_rn(__uint_as_float(t.y << 16), __uint_as_float(t.y & 0xffff0000u));
+    surf3Dwrite(make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi)), s.rgba,
+                x * 8, y, z);
+  } else if constexpr (ST == VVLIC_STORAGE_F16) {
+    surf3Dwrite(t, s.rgba, x * 8, y, z);
+  } else {
+    surf3Dwrite(t, s.rgba, x * 4, y, z);
+  }
+}
+
+
+// The encoded texel of voxel a (fillTexDataFloatInterp).
+template <int ST>
+__device__ __forceinline__ typename TexelWord<ST>::type encode_voxel(const void* xyz, int dtype, size_t a, float max_len) {
+  unsigned char t[3];
+  float len = voxel_len(xyz, dtype, a, t);
+  float r, g, b;
+  if (len == 0.0f) {
+    r = g = b = 0.5f;
+  } else if (dtype == VVLIC_DTYPE_UINT8) {
+    r = 0.5f * (float)t[0] / len + 0.5f;
+    g = 0.5f * (float)t[1] / len + 0.5f;
+    b = 0.5f * (float)t[2] / len + 0.5f;
+  } else {
+    const float* f = reinterpret_cast<const float*>(xyz) + 3 * a;
+    r = 0.5f * f[0] / len + 0.5f;
+    g = 0.5f * f[1] / len + 0.5f;
+    b = 0.5f * f[2] / len + 0.5f;
+  }
+  float al = max_len > 0.0f ? len / max_len : 0.0f;
+  al = (al > 1.0f) ? 1.0f : ((al < 0.0f) ? 0.0f : al);
+  return encode_texel<ST>(r, g, b, al);
+}
+
+// Voxels run last to first in both encode kernels: the maximum pass before them left the field's end
+// in L2.
 template <int ST>
 __global__ void field_encode_kernel(const void* xyz, int dtype, size_t count, const unsigned* maxbits, void* out) {
   const float max_len = __uint_as_float(*maxbits);
-  for (size_t a = blockIdx.x * (size_t)blockDim.x + threadIdx.x; a < count; a += (size_t)gridDim.x * blockDim.x) {
-    unsigned char t[3];
-    float len = voxel_len(xyz, dtype, a, t);
-    float r, g, b;
-    if (len == 0.0f) {
-      r = g = b = 0.5f;
-    } else if (dtype == VVLIC_DTYPE_UINT8) {
-      r = 0.5f * (float)t[0] / len + 0.5f;
-      g = 0.5f * (float)t[1] / len + 0.5f;
-      b = 0.5f * (float)t[2] / len + 0.5f;
-    } else {
-      const float* f = reinterpret_cast<const float*>(xyz) + 3 * a;
-      r = 0.5f * f[0] / len + 0.5f;
-      g = 0.5f * f[1] / len + 0.5f;
-      b = 0.5f * f[2] / len + 0.5f;
-    }
-    float al = max_len > 0.0f ? len / max_len : 0.0f;
-    al = (al > 1.0f) ? 1.0f : ((al < 0.0f) ? 0.0f : al);
-    store_texel<ST>(out, a, r, g, b, al);
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t a = count - 1 - i;
+    reinterpret_cast<typename TexelWord<ST>::type*>(out)[a] = encode_voxel<ST>(xyz, dtype, a, max_len);
+  }
+}
+
+// The same with the volume's texture arrays.
+template <int ST>
+__global__ void __launch_bounds__(kThreads) field_encode_arrays_kernel(const void* xyz, int dtype, int nx, int ny, int nz,
+                                                                       const unsigned* maxbits, void* out,
+                                                                       const __grid_constant__ FieldSurfaces arr) {
+  const float max_len = __uint_as_float(*maxbits);
+  int x, y;
+  if (!tile_voxel(nx, ny, x, y)) return;
+  const int z1 = nz - (int)blockIdx.z * kTileZ;  // slices z1 - kTileZ .. z1 - 1
+#pragma unroll
+  for (int i = 1; i <= kTileZ; ++i) {
+    const int z = z1 - i;
+    if (z < 0) break;
+    const size_t a = ((size_t)z * ny + y) * nx + x;
+    const auto texel = encode_voxel<ST>(xyz, dtype, a, max_len);
+    reinterpret_cast<typename TexelWord<ST>::type*>(out)[a] = texel;
+    store_array<ST>(arr, x, y, z, texel);
   }
 }
 
@@ -447,63 +536,17 @@ inline int grid_for(size_t count) {
   return (int)(b < 152 * 64 ? (b == 0 ? 1 : b) : 152 * 64);
 }
 
-// Division of a 31-bit index by a fixed extent as a multiply-high and a shift.
-struct FastDiv {
-  unsigned mul, shift, d;
-};
-inline FastDiv fast_div(unsigned d) {
-  FastDiv f;
-  f.d = d;
-  f.shift = 0;
-  while ((1ull << f.shift) < d) ++f.shift;
-  f.mul = (unsigned)((((1ull << f.shift) - d) << 32) / d + 1);
-  return f;
-}
-__device__ __forceinline__ unsigned quotient(unsigned a, const FastDiv& f) { return (__umulhi(a, f.mul) + a) >> f.shift; }
-
-// Voxel index -> coordinates.
-struct VoxelMap {
-  FastDiv nx, ny;
-};
-__device__ __forceinline__ void voxel_xyz(unsigned a, const VoxelMap& m, int& x, int& y, int& z) {
-  const unsigned row = quotient(a, m.nx), slice = quotient(row, m.ny);
-  x = (int)(a - row * m.nx.d);
-  y = (int)(row - slice * m.ny.d);
-  z = (int)slice;
-}
-inline VoxelMap voxel_map(const int n[3]) { return VoxelMap{fast_div((unsigned)n[0]), fast_div((unsigned)n[1])}; }
-
-// The texel of voxel (x, y, z) into the volume's texture arrays.
+// Texels -> texture arrays through surface writes (a volume's first TEXTURE or HYBRID render).
 template <int ST>
-__device__ __forceinline__ void store_array(const FieldSurfaces& s, int x, int y, int z,
-                                            typename TexelWord<ST>::type t) {
-  if constexpr (ST == VVLIC_STORAGE_F32) {
-    surf3Dwrite(make_float2(t.x, t.y), s.rgba, x * 8, y, z);
-    surf3Dwrite(t.z, s.z, x * 4, y, z);
-    surf3Dwrite(t.w, s.w, x * 4, y, z);
-  } else if constexpr (ST == VVLIC_STORAGE_BF16) {
-    const __half2 lo = __floats2half2_rn(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xffff0000u));
-    const __half2 hi = __floats2half2_rn(__uint_as_float(t.y << 16), __uint_as_float(t.y & 0xffff0000u));
-    surf3Dwrite(make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi)), s.rgba,
-                x * 8, y, z);
-  } else if constexpr (ST == VVLIC_STORAGE_F16) {
-    surf3Dwrite(t, s.rgba, x * 8, y, z);
-  } else {
-    surf3Dwrite(t, s.rgba, x * 4, y, z);
-  }
-}
-
-// Texels -> texture arrays through surface writes, one voxel per thread and iteration.  Bound by
-// memory; it replaces a cudaMemcpy3D per array: a 512^3 half4 field update, whose last pass this is,
-// went from 1762 to 1556 us.
-template <int ST>
-__global__ void fill_arrays_kernel(const void* texels, unsigned count, const __grid_constant__ VoxelMap m,
-                                   const __grid_constant__ FieldSurfaces arr) {
+__global__ void __launch_bounds__(kThreads) fill_arrays_kernel(const void* texels, int nx, int ny, int nz,
+                                                               const __grid_constant__ FieldSurfaces arr) {
+  int x, y;
+  if (!tile_voxel(nx, ny, x, y)) return;
   const auto* t = reinterpret_cast<const typename TexelWord<ST>::type*>(texels);
-  for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < count; a += gridDim.x * blockDim.x) {
-    int x, y, z;
-    voxel_xyz(a, m, x, y, z);
-    store_array<ST>(arr, x, y, z, t[a]);
+#pragma unroll
+  for (int i = 0; i < kTileZ; ++i) {
+    const int z = (int)blockIdx.z * kTileZ + i;
+    if (z < nz) store_array<ST>(arr, x, y, z, t[((size_t)z * ny + y) * nx + x]);
   }
 }
 
@@ -535,21 +578,29 @@ cudaError_t launch_interp_field(const void* d_a0, const void* d_a1, int dtype, c
   return cudaGetLastError();
 }
 
+template <int ST>
+static void launch_encode(const void* d_xyz, int dtype, const int n[3], void* d_texels, const unsigned* d_maxbits,
+                          const FieldSurfaces* arr, cudaStream_t s) {
+  const size_t count = (size_t)n[0] * n[1] * n[2];
+  if (arr)
+    field_encode_arrays_kernel<ST><<<tile_grid(n), kThreads, 0, s>>>(d_xyz, dtype, n[0], n[1], n[2], d_maxbits, d_texels, *arr);
+  else field_encode_kernel<ST><<<grid_for(count), kThreads, 0, s>>>(d_xyz, dtype, count, d_maxbits, d_texels);
+}
+
 cudaError_t launch_encode_field(const void* d_xyz, int dtype, const int n[3], int storage, void* d_texels,
-                                unsigned* d_maxbits, cudaStream_t s) {
+                                unsigned* d_maxbits, const FieldSurfaces* arr, cudaStream_t s) {
   const size_t count = (size_t)n[0] * n[1] * n[2];
   cudaError_t e = cudaMemsetAsync(d_maxbits, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
-  field_maxlen_kernel<<<grid_for(count), kThreads, 0, s>>>(d_xyz, dtype, count, d_maxbits);
-  if (storage == VVLIC_STORAGE_F32)
-    field_encode_kernel<VVLIC_STORAGE_F32><<<grid_for(count), kThreads, 0, s>>>(d_xyz, dtype, count, d_maxbits, d_texels);
-  else if (storage == VVLIC_STORAGE_F16)
-    field_encode_kernel<VVLIC_STORAGE_F16><<<grid_for(count), kThreads, 0, s>>>(d_xyz, dtype, count, d_maxbits, d_texels);
+  const bool vec = dtype == VVLIC_DTYPE_FLOAT32 && (reinterpret_cast<uintptr_t>(d_xyz) & 15) == 0;
+  const int grid = std::min(grid_for(vec ? (count + 3) / 4 : count), 152 * 8);
+  if (vec) field_maxlen_kernel<true><<<grid, kThreads, 0, s>>>(d_xyz, dtype, count, d_maxbits);
+  else field_maxlen_kernel<false><<<grid, kThreads, 0, s>>>(d_xyz, dtype, count, d_maxbits);
+  if (storage == VVLIC_STORAGE_F32) launch_encode<VVLIC_STORAGE_F32>(d_xyz, dtype, n, d_texels, d_maxbits, arr, s);
+  else if (storage == VVLIC_STORAGE_F16) launch_encode<VVLIC_STORAGE_F16>(d_xyz, dtype, n, d_texels, d_maxbits, arr, s);
   else if (storage == VVLIC_STORAGE_UNORM8)
-    field_encode_kernel<VVLIC_STORAGE_UNORM8><<<grid_for(count), kThreads, 0, s>>>(d_xyz, dtype, count, d_maxbits,
-                                                                                    d_texels);
-  else
-    field_encode_kernel<VVLIC_STORAGE_BF16><<<grid_for(count), kThreads, 0, s>>>(d_xyz, dtype, count, d_maxbits, d_texels);
+    launch_encode<VVLIC_STORAGE_UNORM8>(d_xyz, dtype, n, d_texels, d_maxbits, arr, s);
+  else launch_encode<VVLIC_STORAGE_BF16>(d_xyz, dtype, n, d_texels, d_maxbits, arr, s);
   return cudaGetLastError();
 }
 
@@ -601,15 +652,14 @@ cudaError_t launch_build_field_cells(const void* d_texels, const int n[3], int s
 
 cudaError_t launch_fill_arrays(const void* d_texels, const int n[3], int storage, const FieldSurfaces& arr,
                                cudaStream_t s) {
-  const unsigned count = (unsigned)n[0] * (unsigned)n[1] * (unsigned)n[2];  // < 2^31 (valid_dims)
-  const VoxelMap m = voxel_map(n);
-  const int g = grid_for(count);
-  if (storage == VVLIC_STORAGE_F32) fill_arrays_kernel<VVLIC_STORAGE_F32><<<g, kThreads, 0, s>>>(d_texels, count, m, arr);
+  const dim3 g = tile_grid(n);
+  if (storage == VVLIC_STORAGE_F32)
+    fill_arrays_kernel<VVLIC_STORAGE_F32><<<g, kThreads, 0, s>>>(d_texels, n[0], n[1], n[2], arr);
   else if (storage == VVLIC_STORAGE_F16)
-    fill_arrays_kernel<VVLIC_STORAGE_F16><<<g, kThreads, 0, s>>>(d_texels, count, m, arr);
+    fill_arrays_kernel<VVLIC_STORAGE_F16><<<g, kThreads, 0, s>>>(d_texels, n[0], n[1], n[2], arr);
   else if (storage == VVLIC_STORAGE_UNORM8)
-    fill_arrays_kernel<VVLIC_STORAGE_UNORM8><<<g, kThreads, 0, s>>>(d_texels, count, m, arr);
-  else fill_arrays_kernel<VVLIC_STORAGE_BF16><<<g, kThreads, 0, s>>>(d_texels, count, m, arr);
+    fill_arrays_kernel<VVLIC_STORAGE_UNORM8><<<g, kThreads, 0, s>>>(d_texels, n[0], n[1], n[2], arr);
+  else fill_arrays_kernel<VVLIC_STORAGE_BF16><<<g, kThreads, 0, s>>>(d_texels, n[0], n[1], n[2], arr);
   return cudaGetLastError();
 }
 

@@ -40,15 +40,12 @@ vvlic_status ensure_noise_cells(vvlic_ctx* c, NoiseTex& n, cudaStream_t s) {
   return VVLIC_OK;
 }
 
-// Copies the volume's texels into its texture arrays (allocated by ensure_texture).
-vvlic_status fill_textures(vvlic_ctx* c, Volume& v, cudaStream_t s) {
+FieldSurfaces surfaces(const Volume& v) {
   FieldSurfaces arr;
   arr.rgba = v.surf[0];
   arr.z = v.surf[1];
   arr.w = v.surf[2];
-  const cudaError_t e = launch_fill_arrays(v.d_texels, v.n, v.storage, arr, s);
-  if (e != cudaSuccess) return cuda_fail(c, e, "texture array fill");
-  return VVLIC_OK;
+  return arr;
 }
 
 // Texture copy of a volume.  128-bit texels filter at an eighth of the texture unit's rate, so F32
@@ -79,8 +76,8 @@ vvlic_status ensure_texture(vvlic_ctx* c, Volume& v, cudaStream_t s) {
     e = cudaCreateTextureObject(&v.tex[i], &rd, &td, nullptr);
     if (e != cudaSuccess) return cuda_fail(c, e, "texture object");
   }
-  const vvlic_status st = fill_textures(c, v, s);
-  if (st) return st;
+  const cudaError_t e = launch_fill_arrays(v.d_texels, v.n, v.storage, surfaces(v), s);
+  if (e != cudaSuccess) return cuda_fail(c, e, "texture array fill");
   v.array_bytes = (size_t)v.n[0] * v.n[1] * v.n[2] * texel_bytes(v.storage);
   return VVLIC_OK;
 }
@@ -126,12 +123,15 @@ vvlic_status ensure_noise_texture(vvlic_ctx* c, NoiseTex& n, cudaStream_t s) {
 
 namespace vvlic {
 
-vvlic_status refresh_volume_layouts(vvlic_ctx* c, Volume& v, cudaStream_t s) {
+vvlic_status encode_volume(vvlic_ctx* c, Volume& v, const void* d_xyz, int dtype, cudaStream_t s) {
+  const FieldSurfaces arr = surfaces(v);
+  cudaError_t e = launch_encode_field(d_xyz, dtype, v.n, v.storage, v.d_texels, c->d_scratch_word,
+                                      v.array_bytes ? &arr : nullptr, s);
+  if (e != cudaSuccess) return cuda_fail(c, e, "field encoding");
   if (v.d_cells) {
-    cudaError_t e = launch_build_field_cells(v.d_texels, v.n, v.storage, v.d_cells, s);
+    e = launch_build_field_cells(v.d_texels, v.n, v.storage, v.d_cells, s);
     if (e != cudaSuccess) return cuda_fail(c, e, "cell layout rebuild");
   }
-  if (v.array_bytes) return fill_textures(c, v, s);
   return VVLIC_OK;
 }
 

@@ -166,9 +166,11 @@ vvlic_status ensure_illum_luts(vvlic_ctx* c);
 // Orders the context stream after the context's last launch (device-table updates).
 cudaError_t after_launches(vvlic_ctx* c);
 vvlic_status cuda_fail(vvlic_ctx* c, cudaError_t e, const char* what);
-// Rewrite the cell and texture copies that exist from the texels, in place (render.cu).
 void free_textures(Volume& v);  // texture objects, surfaces and arrays of the texture copy
-vvlic_status refresh_volume_layouts(vvlic_ctx* c, Volume& v, cudaStream_t s);
+// Encode new raw vectors into the texels and the cell and texture copies that exist, in place
+// (render.cu).
+vvlic_status encode_volume(vvlic_ctx* c, Volume& v, const void* d_xyz, int dtype, cudaStream_t s);
+// Rewrite the noise's cell and texture copies that exist from its texels, in place (render.cu).
 vvlic_status refresh_noise_layouts(vvlic_ctx* c, NoiseTex& n, cudaStream_t s);
 Geometry make_geometry(const int n[3], const float* slice_dist);
 vvlic_status derive_taps(const vvlic_ctx* c, int lb, int lf, float* taps, float* inv_area);

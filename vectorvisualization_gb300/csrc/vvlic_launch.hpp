@@ -98,10 +98,15 @@ cudaError_t launch_brick(int storage, const RenderArgs& a, const BrickArgs& b, i
 
 // Preprocessing (preprocess.cu, compiled without FMA contraction so results match the
 // reference's CPU arithmetic bit for bit).
-// Field encoding of fillTexDataFloatInterp into `storage` texels; d_maxbits is a 4-byte
-// device scratch word.
+// Surfaces of a volume's texture arrays: `rgba` (half4 for F16 and BF16, uchar4 for UNORM8), or for
+// F32 the (x, y), z and w arrays (vvlic_device.cuh, Field<F32, kTexture>).
+struct FieldSurfaces {
+  cudaSurfaceObject_t rgba = 0, z = 0, w = 0;
+};
+// Field encoding of fillTexDataFloatInterp into `storage` texels and, where `arr` is given, the
+// volume's texture arrays; d_maxbits is a 4-byte device scratch word.
 cudaError_t launch_encode_field(const void* d_xyz, int dtype, const int n[3], int storage, void* d_texels,
-                                unsigned* d_maxbits, cudaStream_t s);
+                                unsigned* d_maxbits, const FieldSurfaces* arr, cudaStream_t s);
 // Time interpolation of two raw vector fields at t = interpIndex / InterpSize.
 cudaError_t launch_interp_field(const void* d_a0, const void* d_a1, int dtype, const int n[3], float t, void* d_out,
                                 cudaStream_t s);
@@ -114,11 +119,6 @@ cudaError_t launch_build_field_cells(const void* d_texels, const int n[3], int s
 cudaError_t launch_build_noise_cells(const uint8_t* d_texels, const int m[3], int ch, uint8_t* d_cells,
                                      cudaStream_t s);
 
-// Surfaces of a volume's texture arrays: `rgba` (half4 for F16 and BF16, uchar4 for UNORM8), or for
-// F32 the (x, y), z and w arrays (vvlic_device.cuh, Field<F32, kTexture>).
-struct FieldSurfaces {
-  cudaSurfaceObject_t rgba = 0, z = 0, w = 0;
-};
 // Texels into the texture arrays.  A BF16 volume's array holds half-precision copies of its texels
 // (the texture unit has no bf16 format): exact for every texel value in [2^-14, 65504]; smaller
 // magnitudes round to the nearest half subnormal (absolute error <= 2^-25).
