@@ -183,8 +183,7 @@ enum { VVLIC_TECHNIQUE_VOLUME = 0, VVLIC_TECHNIQUE_RAYCAST = 1, VVLIC_TECHNIQUE_
 
 /* Work distribution of a render launch.  Forward ray-casts run one raster grid of small CTAs, a warp
  * on 2x2 (or 2x1) rays with 8 (16) consecutive samples of each side by side, under either value;
- * adjoints pull 8x4-pixel tiles, longest ray chord first, from a device work queue (no spin-waits: one
- * atomic per tile). */
+ * adjoints pull 2x2-ray tiles from a device counter (no spin-waits: one atomic per tile). */
 enum { VVLIC_SCHEDULE_QUEUE = 0, VVLIC_SCHEDULE_STATIC = 1 };
 
 /* View.  PERSPECTIVE follows Camera::setCamera (camera.cpp:56-67) followed by

@@ -3,15 +3,16 @@
 //
 // The forward render records a tape: per sample (intensity I, TF coordinate), with gradient
 // lighting also the LIC gradient sum G (4 halves), and every kSegment samples a checkpoint
-// (position, dest before the sample).  Per ray this kernel walks the segments last to first: it
-// recomputes the segment's compositing states from its checkpoint into a local array (cheap:
-// no streamline work), then backpropagates sample by sample through clamp, blend, alpha
-// correction, the opacity lookup, the shading (illumZoeckler / illumMallo factors recomputed
-// from the field sample) and the TF lookup.  The cotangents of I and G are
-// pushed onto the filter taps by walking the sample's streamlines once more
-// (dL/dw_j = sum_k S dL/dI_k n_kj + dL/dG_k . g_kj).
+// (position, dest before the sample).  A warp takes four rays, eight consecutive samples of each
+// side by side (the forward's groups), and walks their segments last to first.  From the
+// checkpoint it recomputes the compositing states (cheap: no streamline work), the lanes forming
+// the sources and every lane of a ray blending them in order; going back, every lane of a ray carries
+// the image cotangent through the blends and each lane keeps what its own sample needs.  The
+// samples' cotangents (clamp, blend, alpha correction, opacity lookup, shading, TF lookup) and
+// their streamlines are then one lane each: the cotangents of I and G are pushed onto the filter taps by
+// walking the streamlines once more (dL/dw_j = sum_k S dL/dI_k n_kj + dL/dG_k . g_kj).
 //
-// Reductions are deterministic: per-tap sums are formed by a fixed-order warp butterfly, and
+// Reductions are deterministic: per-tap sums are formed by fixed-order warp exchanges, and
 // every contribution enters 64-bit fixed-point accumulators (scale 2^30) by integer atomics,
 // which are associative — so the result does not depend on scheduling.
 #pragma once
@@ -20,32 +21,31 @@
 
 namespace vvlic {
 
-// Minimum resident CTAs per SM requested for the adjoint kernels (register cap 65536 / (128 * n)):
-// 6 (80 registers, a few spilled bytes) measured 1786 ms against 1951 ms for 5 (93 registers)
-// on the lit 512^3 RK4 frame with one sample per pass and one warp butterfly per tap sum.
+// Minimum resident CTAs per SM requested for the adjoint kernels (register cap 65536 / (128 * n)): 6
+// (80 registers).  At 7 / 6 / 5 / 4: four-view fit step of 128^3 43.1 / 42.7 / 44.2 / 48.0 ms; RK4, lit,
+// L = 60: 128.2 at 3, 118.7 at 4, 118.0 at 5, 117.4 at 6.
 #ifndef VVLIC_ADJ_MIN_BLOCKS
 #define VVLIC_ADJ_MIN_BLOCKS 6
 #endif
-// Samples whose streamlines one thread re-walks together in the RK4 adjoint: 1 or 2 (four
-// independent gather chains, as the forward's trace_pixel2).  On frames 0 / 40 of the lit 512^3
-// RK4 orbit (2048^2) the adjoint took 1309 / 1532 ms with two samples at 6 CTAs per SM (80
-// registers, 100 spilled bytes), 1335 / 1550 ms at 5 (96 registers), 1353 / 1579 ms at 4 (127
-// registers) and 1518 / 1762 ms with one sample at 6.  Two samples per pass measured slower for
-// the Heun forward, so the other integrators keep one.
-#ifndef VVLIC_ADJ_RK4_SAMPLES_PER_PASS
-#define VVLIC_ADJ_RK4_SAMPLES_PER_PASS 2
-#endif
-
-template <int INTEG> __host__ __device__ constexpr int adj_samples_per_pass() {
-  return INTEG == VVLIC_RK4 ? VVLIC_ADJ_RK4_SAMPLES_PER_PASS : 1;
-}
 
 constexpr float kFixedScale = 1073741824.0f;  // 2^30
 constexpr int kAccTF = 0, kAccOpac = 4 * VVLIC_TF_ENTRIES, kAccTaps = 5 * VVLIC_TF_ENTRIES;
 constexpr int kAccSize = kAccTaps + kMaxTaps;
 
+// Adds v to a 64-bit fixed-point accumulator in shared memory, as two 32-bit atomics: the low word's
+// old value tells each addition its own carry, so the sum is the 64-bit one in any order.  (64-bit
+// shared atomics are compare-and-swap loops, and neighbouring samples hit the same table entries: fit
+// step of four 512^2 views 42.7 ms with them, 38.7 so, 38.1 without any.)  |v| < 1 converts in 32
+// bits.
 __device__ __forceinline__ void fixed_add(long long* slot, float v) {
-  if (v != 0.0f) atomicAdd(reinterpret_cast<unsigned long long*>(slot), (unsigned long long)__float2ll_rn(v * kFixedScale));
+  if (v == 0.0f) return;
+  const float f = v * kFixedScale;
+  const long long q = fabsf(v) < 1.0f ? (long long)__float2int_rn(f) : __float2ll_rn(f);
+  const unsigned lo = (unsigned)q;
+  unsigned hi = (unsigned)((unsigned long long)q >> 32);
+  unsigned* w = reinterpret_cast<unsigned*>(slot);
+  hi += atomicAdd(w, lo) + lo < lo ? 1u : 0u;
+  if (hi) atomicAdd(w + 1, hi);
 }
 
 // Sum over the warp (fixed butterfly order); lane 0 adds it to the block accumulator.
@@ -55,18 +55,55 @@ __device__ __forceinline__ void warp_fixed_add(long long* slot, float v) {
   if ((threadIdx.x & 31) == 0) fixed_add(slot, v);
 }
 
-// Two warp sums in five shuffles (fixed order): the first exchange leaves lanes 0-15 holding
-// pair sums of `va` and lanes 16-31 pair sums of `vb`; each half then reduces on its own.  Lane 0
-// adds the sum of `va` to slot_a (when use_a), lane 16 the sum of `vb` to slot_b (when use_b).
-__device__ __forceinline__ void warp_fixed_add2(long long* slot_a, bool use_a, float va, long long* slot_b, bool use_b,
-                                                float vb) {
-  const int lane = threadIdx.x & 31;
-  const bool lo = lane < 16;
-  float x = (lo ? va : vb) + __shfl_xor_sync(0xffffffffu, lo ? vb : va, 16);
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  if ((lane == 0 && use_a) || (lane == 16 && use_b)) fixed_add(lo ? slot_a : slot_b, x);
+// One exchange of a warp reduction of two values: lanes with bit `o` clear keep `a`, the others
+// `b`, each plus its partner's.
+__device__ __forceinline__ float exchange(float a, float b, int o) {
+  const bool lo = ((threadIdx.x & 31) & o) == 0;
+  return (lo ? a : b) + __shfl_xor_sync(0xffffffffu, lo ? b : a, o);
 }
+
+// Warp sums of the tap contributions of both streamline directions, one pair per step, reduced 32 at a
+// time: step 2^n merges with the step before it at distance 16 >> n, so 16 steps (32 sums) take 31
+// exchanges and leave each lane with one finished sum, which it adds to its tap; a butterfly per step
+// takes five shuffles and a 64-bit shared atomic for every pair.  Every lane of the warp calls.
+struct TapSums {
+  float h1, h2, h3, h4;  // waiting for their partner at each level
+  __device__ __forceinline__ void step(int i, float vb, float vf, int lb, int lf, long long* s_taps) {  // i = 1, 2, ...
+    const int n = i - 1;
+    float x = exchange(vb, vf, 16);
+    if (!(n & 1)) {
+      h1 = x;
+      return;
+    }
+    x = exchange(h1, x, 8);
+    if (!(n & 2)) {
+      h2 = x;
+      return;
+    }
+    x = exchange(h2, x, 4);
+    if (!(n & 4)) {
+      h3 = x;
+      return;
+    }
+    x = exchange(h3, x, 2);
+    if (!(n & 8)) {
+      h4 = x;
+      return;
+    }
+    x = exchange(h4, x, 1);
+    const int lane = threadIdx.x & 31;
+    const int j = (n & ~15) + 1 + (((lane >> 3) & 1) | ((lane >> 1) & 2) | ((lane << 1) & 4) | ((lane << 3) & 8));
+    if (lane & 16) {
+      if (j <= lf) fixed_add(s_taps + lb + j, x);
+    } else if (j <= lb) {
+      fixed_add(s_taps + lb - j, x);
+    }
+  }
+  // the steps after the last one, up to a whole block of 16
+  __device__ __forceinline__ void finish(int i, int lb, int lf, long long* s_taps) {
+    for (; (i - 1) & 15; ++i) step(i, 0.0f, 0.0f, lb, lf, s_taps);
+  }
+};
 
 // 1D LINEAR + CLAMP_TO_EDGE lookup decomposed: entries i0, i1, weight t of i1, and whether the
 // coordinate lies strictly inside the interpolation range (derivative in s = 256 there, else 0).
@@ -112,12 +149,6 @@ __device__ __forceinline__ Src unlit_source(const RenderArgs& a, const float* s_
 __device__ __forceinline__ float4 premultiplied(const Src& s) {
   return make_float4(s.col.x * s.alpha, s.col.y * s.alpha, s.col.z * s.alpha, s.alpha);
 }
-// The source as blend() takes it (colour not yet multiplied by alpha), matching shade().
-__device__ __forceinline__ float4 unlit_source_rgba(const RenderArgs& a, const float* s_tf, float I, float tfc) {
-  const Src s = unlit_source(a, s_tf, I, tfc);
-  return make_float4(s.col.x, s.col.y, s.col.z, s.alpha);
-}
-
 // illumGradient (inc_illum.glsl:1-41) intermediates: N = n(-G), R = n(2 (L.N) N - L),
 // df = sat(L.N) * illumScale, spf = sat(R.V)^e.
 struct LitT {
@@ -178,141 +209,112 @@ __device__ __forceinline__ float3 tape_gradient(const RenderArgs& a, size_t idx)
   return f3(xy.x, xy.y, z0.x);
 }
 
+// gI * n + gG . g of a tap
+template <bool GRAD> __device__ __forceinline__ float tap_dot(float4 n, float gI, float3 gG) {
+  return GRAD ? fmaf(gI, n.w, gG.x * n.x + gG.y * n.y + gG.z * n.z) : gI * n.w;
+}
+
 // Walk the streamlines of the LIC at `pos` once more and add gI * n_j (+ gG . g_j with noise
 // gradients) to the tap accumulators.  Every lane of the warp takes part in each reduction;
 // lanes with zero cotangents skip the fetches.
 template <int ST, int FL, int NL, int INTEG, bool GRAD>
-__device__ __forceinline__ float tap_dot(float4 n, float gI, float3 gG) {
-  return GRAD ? fmaf(gI, n.w, gG.x * n.x + gG.y * n.y + gG.z * n.z) : gI * n.w;
-}
-template <int ST, int FL, int NL, int INTEG, bool GRAD>
 __device__ __forceinline__ void tap_gradients(const RenderArgs& a, float3 pos, float gI, float3 gG, long long* s_taps) {
   const bool act = gI != 0.0f || (GRAD && (gG.x != 0.0f || gG.y != 0.0f || gG.z != 0.0f));
-  const int lb = a.lb, lf = a.lf, L = max(lb, lf);
+  const int lb = a.lb, lf = a.lf, both = min(lb, lf), L = max(lb, lf);
   float4 f0 = make_float4(0.f, 0.f, 0.f, 0.f);
   float v0 = 0.0f;
   if (act) {
     f0 = Field<ST, FL>::sample(a, pos);
-    v0 = tap_dot<ST, FL, NL, INTEG, GRAD>(noise_tap<NL, GRAD>(a, pos), gI, gG);
+    v0 = tap_dot<GRAD>(noise_tap<NL, GRAD>(a, pos), gI, gG);
   }
   warp_fixed_add(s_taps + lb, v0);
   float3 pb = pos, pf = pos;
   float4 sb = f0, sf = f0;
-  for (int i = 1; i <= L; ++i) {
-    float vb = 0.0f, vf = 0.0f;
-    if (act) {
-      if (i <= lb) {
-        pb = lic_step<ST, FL, INTEG>(a, pb, sb, -1.0f);
-        vb = tap_dot<ST, FL, NL, INTEG, GRAD>(noise_tap<NL, GRAD>(a, pb), gI, gG);
-      }
-      if (i <= lf) {
-        pf = lic_step<ST, FL, INTEG>(a, pf, sf, 1.0f);
-        vf = tap_dot<ST, FL, NL, INTEG, GRAD>(noise_tap<NL, GRAD>(a, pf), gI, gG);
-      }
-    }
-    warp_fixed_add2(s_taps + lb - i, i <= lb, vb, s_taps + lb + i, i <= lf, vf);
-  }
-}
-
-// tap_gradients of two samples at once: four independent streamline chains per thread, and
-// per tap the two samples' contributions are added in the lane before the warp sum.  A lane
-// walks both samples' streamlines when either has a non-zero cotangent; the other sample's
-// terms are then zero (its cotangents are zero and its noise values finite).
-template <int ST, int FL, int NL, int INTEG, bool GRAD>
-__device__ __forceinline__ void tap_gradients2(const RenderArgs& a, float3 pa, float gIa, float3 gGa, float3 pc,
-                                               float gIc, float3 gGc, long long* s_taps) {
-  const bool act = gIa != 0.0f || gIc != 0.0f ||
-                   (GRAD && (gGa.x != 0.0f || gGa.y != 0.0f || gGa.z != 0.0f || gGc.x != 0.0f || gGc.y != 0.0f ||
-                             gGc.z != 0.0f));
-  const int lb = a.lb, lf = a.lf, L = max(lb, lf);
-  float4 fa = make_float4(0.f, 0.f, 0.f, 0.f), fc = fa;
-  float v0 = 0.0f;
-  if (act) {
-    fa = Field<ST, FL>::sample(a, pa);
-    fc = Field<ST, FL>::sample(a, pc);
-    v0 = tap_dot<ST, FL, NL, INTEG, GRAD>(noise_tap<NL, GRAD>(a, pa), gIa, gGa) +
-         tap_dot<ST, FL, NL, INTEG, GRAD>(noise_tap<NL, GRAD>(a, pc), gIc, gGc);
-  }
-  warp_fixed_add(s_taps + lb, v0);
-  float3 p0 = pa, p1 = pa, p2 = pc, p3 = pc;
-  float4 s0 = fa, s1 = fa, s2 = fc, s3 = fc;
-  const int both = min(lb, lf);
+  TapSums sums;
   int i = 1;
   for (; i <= both; ++i) {
     float vb = 0.0f, vf = 0.0f;
     if (act) {
-      p0 = lic_step<ST, FL, INTEG>(a, p0, s0, -1.0f);
-      p1 = lic_step<ST, FL, INTEG>(a, p1, s1, 1.0f);
-      p2 = lic_step<ST, FL, INTEG>(a, p2, s2, -1.0f);
-      p3 = lic_step<ST, FL, INTEG>(a, p3, s3, 1.0f);
-      vb = tap_dot<ST, FL, NL, INTEG, GRAD>(noise_tap<NL, GRAD>(a, p0), gIa, gGa) +
-           tap_dot<ST, FL, NL, INTEG, GRAD>(noise_tap<NL, GRAD>(a, p2), gIc, gGc);
-      vf = tap_dot<ST, FL, NL, INTEG, GRAD>(noise_tap<NL, GRAD>(a, p1), gIa, gGa) +
-           tap_dot<ST, FL, NL, INTEG, GRAD>(noise_tap<NL, GRAD>(a, p3), gIc, gGc);
+      float2 n[4];
+      pb = lic_step<ST, FL, INTEG>(a, pb, sb, -1.0f);
+      pf = lic_step<ST, FL, INTEG>(a, pf, sf, 1.0f);
+      noise_tap2<NL, GRAD>(a, pb, pf, n);
+      vb = GRAD ? tap_dot<true>(make_float4(n[0].x, n[1].x, n[2].x, n[3].x), gI, gG) : gI * n[3].x;
+      vf = GRAD ? tap_dot<true>(make_float4(n[0].y, n[1].y, n[2].y, n[3].y), gI, gG) : gI * n[3].y;
     }
-    warp_fixed_add2(s_taps + lb - i, true, vb, s_taps + lb + i, true, vf);
+    sums.step(i, vb, vf, lb, lf, s_taps);
   }
   for (; i <= L; ++i) {
     float vb = 0.0f, vf = 0.0f;
     if (act) {
       if (i <= lb) {
-        p0 = lic_step<ST, FL, INTEG>(a, p0, s0, -1.0f);
-        p2 = lic_step<ST, FL, INTEG>(a, p2, s2, -1.0f);
-        vb = tap_dot<ST, FL, NL, INTEG, GRAD>(noise_tap<NL, GRAD>(a, p0), gIa, gGa) +
-             tap_dot<ST, FL, NL, INTEG, GRAD>(noise_tap<NL, GRAD>(a, p2), gIc, gGc);
-      }
-      if (i <= lf) {
-        p1 = lic_step<ST, FL, INTEG>(a, p1, s1, 1.0f);
-        p3 = lic_step<ST, FL, INTEG>(a, p3, s3, 1.0f);
-        vf = tap_dot<ST, FL, NL, INTEG, GRAD>(noise_tap<NL, GRAD>(a, p1), gIa, gGa) +
-             tap_dot<ST, FL, NL, INTEG, GRAD>(noise_tap<NL, GRAD>(a, p3), gIc, gGc);
+        pb = lic_step<ST, FL, INTEG>(a, pb, sb, -1.0f);
+        vb = tap_dot<GRAD>(noise_tap<NL, GRAD>(a, pb), gI, gG);
+      } else {
+        pf = lic_step<ST, FL, INTEG>(a, pf, sf, 1.0f);
+        vf = tap_dot<GRAD>(noise_tap<NL, GRAD>(a, pf), gI, gG);
       }
     }
-    warp_fixed_add2(s_taps + lb - i, i <= lb, vb, s_taps + lb + i, i <= lf, vf);
+    sums.step(i, vb, vf, lb, lf, s_taps);
   }
+  sums.finish(i, lb, lf, s_taps);
 }
 
-// Reverse step through one sample (kk of segment seg): clamp, blend, alpha correction, opacity
-// and TF lookups and the shading, from the recomputed compositing state Dloc[kk].  Adds the TF
-// and opacity cotangents to the block accumulators, updates the image cotangent g to the one
-// before the sample and returns the cotangents of the sample's LIC intensity (gIraw, already
-// scaled by the intensity scale) and gradient sum (gG), and its position.  Samples at or past
-// cnt leave everything zero.
+// A sample's source recomputed from its tape record: what the blend, the lookups and the shading
+// need again in the reverse step.
+template <bool GRAD> struct Sample {
+  Src s;
+  LitT lt;       // GRAD
+  float3 ld;     // line lighting: colour = tf.rgb * I * ld + ...
+  float I;
+};
 template <int ST, int FL, bool GRAD>
-__device__ __forceinline__ void sample_cotangent(const RenderArgs& a, const float* s_tf, bool line, float3 dir,
-                                                 const float4* Dloc, const float3* Ploc, int px, int py, int seg,
-                                                 int kk, int cnt, float4& g, long long* s_acc, float& gIraw,
-                                                 float3& gG, float3& pk) {
-  gIraw = 0.0f;
-  gG = f3(0.f, 0.f, 0.f);
-  pk = f3(0.f, 0.f, 0.f);
-  if (kk < 0 || kk >= cnt) return;
-  const size_t idx = tape_entry_checked(a, px, py, seg * kSegment + kk);
+__device__ __forceinline__ Sample<GRAD> tape_sample(const RenderArgs& a, const float* s_tf, bool line, size_t idx,
+                                                    float3 pos, float3 dir) {
+  Sample<GRAD> q;
   const float2 rec = a.tape_is[idx];
-  const float I = rec.x;
-  Src s = unlit_source(a, s_tf, I, rec.y);
-  LitT lt;
-  float3 ld = f3(0.f, 0.f, 0.f);
+  q.I = rec.x;
+  q.s = unlit_source(a, s_tf, rec.x, rec.y);
   if (GRAD) {
-    lt = lit_setup(a, tape_gradient(a, idx), Ploc[kk], dir);
-    s.col = lit_color(a, lt, s.tf, I);
-  } else if (line) {  // colour = tf.rgb * I * d + s (d, s independent of TF, taps and I)
+    q.lt = lit_setup(a, tape_gradient(a, idx), pos, dir);
+    q.s.col = lit_color(a, q.lt, q.s.tf, q.I);
+  } else if (line) {  // (ld and the specular part are independent of TF, taps and I)
     float3 sf;
-    line_factors(a, Ploc[kk], dir, Field<ST, FL>::sample(a, Ploc[kk]), ld, sf);
-    s.col = f3(s.tf.x * I * ld.x + sf.x, s.tf.y * I * ld.y + sf.y, s.tf.z * I * ld.z + sf.z);
+    line_factors(a, pos, dir, Field<ST, FL>::sample(a, pos), q.ld, sf);
+    q.s.col = f3(q.s.tf.x * q.I * q.ld.x + sf.x, q.s.tf.y * q.I * q.ld.y + sf.y, q.s.tf.z * q.I * q.ld.z + sf.z);
   }
-  const float4 sv = premultiplied(s);
-  const float4 Dp = Dloc[kk];
-  pk = Ploc[kk];
+  return q;
+}
+// The source as blend() takes it (colour not yet multiplied by alpha), matching shade().
+__device__ __forceinline__ float4 source_rgba(const Src& s) { return make_float4(s.col.x, s.col.y, s.col.z, s.alpha); }
+
+__device__ __forceinline__ float4 shfl4(float4 v, int from) {
+  return make_float4(__shfl_sync(0xffffffffu, v.x, from), __shfl_sync(0xffffffffu, v.y, from),
+                     __shfl_sync(0xffffffffu, v.z, from), __shfl_sync(0xffffffffu, v.w, from));
+}
+
+// The image cotangent g through clamp((1 - Dp.a) * sv + Dp) (derivative 1 on [0, 1]) to the
+// one before the sample; ds: the cotangent of the premultiplied source.
+__device__ __forceinline__ float4 blend_vjp(float4 g, float4 sv, float4 Dp, float4& ds) {
   const float om = 1.0f - Dp.w;
-  // clamp((1 - Dp.a) * s + Dp) per channel: derivative 1 on [0, 1]
-  const float ux = fmaf(om, sv.x, Dp.x), uy = fmaf(om, sv.y, Dp.y), uz = fmaf(om, sv.z, Dp.z),
-              uw = fmaf(om, sv.w, Dp.w);
+  const float ux = fmaf(om, sv.x, Dp.x), uy = fmaf(om, sv.y, Dp.y), uz = fmaf(om, sv.z, Dp.z), uw = fmaf(om, sv.w, Dp.w);
   const float gx = (ux >= 0.f && ux <= 1.f) ? g.x : 0.f, gy = (uy >= 0.f && uy <= 1.f) ? g.y : 0.f,
               gz = (uz >= 0.f && uz <= 1.f) ? g.z : 0.f, gw = (uw >= 0.f && uw <= 1.f) ? g.w : 0.f;
-  const float4 ds = make_float4(om * gx, om * gy, om * gz, om * gw);
+  ds = make_float4(om * gx, om * gy, om * gz, om * gw);
   float4 gp = make_float4(gx, gy, gz, gw);
   gp.w -= gx * sv.x + gy * sv.y + gz * sv.z + gw * sv.w;
+  return gp;
+}
+
+// Reverse step of one sample from the cotangent ds of its premultiplied source: alpha correction,
+// opacity and TF lookups and the shading.  Adds the TF and opacity cotangents to the block
+// accumulators and returns those of the LIC intensity (gI, scaled by the intensity scale) and of
+// the gradient sum (gG).
+template <bool GRAD>
+__device__ __forceinline__ void sample_cotangent(const RenderArgs& a, const float* s_tf, bool line,
+                                                 const Sample<GRAD>& q, float4 ds, long long* s_acc, float& gI,
+                                                 float3& gG) {
+  const Src& s = q.s;
   // s = (col * alpha, alpha)
   const float dcx = ds.x * s.alpha, dcy = ds.y * s.alpha, dcz = ds.z * s.alpha;
   const float dalpha = ds.x * s.col.x + ds.y * s.col.y + ds.z * s.col.z + ds.w;
@@ -328,15 +330,15 @@ __device__ __forceinline__ void sample_cotangent(const RenderArgs& a, const floa
   dtf[3] = dtfa;
   if (GRAD) {
     float dIc;
-    lit_vjp(a, lt, s.tf, I, f3(dcx, dcy, dcz), dtf, &dIc, &gG);
+    lit_vjp(a, q.lt, s.tf, q.I, f3(dcx, dcy, dcz), dtf, &dIc, &gG);
     dI += dIc;
   } else if (line) {
-    dtf[0] = dcx * I * ld.x;
-    dtf[1] = dcy * I * ld.y;
-    dtf[2] = dcz * I * ld.z;
-    dI += dcx * s.tf.x * ld.x + dcy * s.tf.y * ld.y + dcz * s.tf.z * ld.z;
+    dtf[0] = dcx * q.I * q.ld.x;
+    dtf[1] = dcy * q.I * q.ld.y;
+    dtf[2] = dcz * q.I * q.ld.z;
+    dI += dcx * s.tf.x * q.ld.x + dcy * s.tf.y * q.ld.y + dcz * s.tf.z * q.ld.z;
   } else {  // col = I * tf.rgb * illumScale
-    const float ci = I * a.illum_scale;
+    const float ci = q.I * a.illum_scale;
     dtf[0] = dcx * ci;
     dtf[1] = dcy * ci;
     dtf[2] = dcz * ci;
@@ -347,93 +349,97 @@ __device__ __forceinline__ void sample_cotangent(const RenderArgs& a, const floa
     fixed_add(s_acc + kAccTF + 4 * s.lt.i0 + ch, dtf[ch] * (1.0f - s.lt.t));
     fixed_add(s_acc + kAccTF + 4 * s.lt.i1 + ch, dtf[ch] * s.lt.t);
   }
-  gIraw = dI * a.intensity_scale;
-  g = gp;
+  gI = dI * a.intensity_scale;
 }
 
 template <int ST, int FL, int NL, int INTEG, bool GRAD>
-__global__ void __launch_bounds__(kThreads, VVLIC_ADJ_MIN_BLOCKS) adjoint_kernel(const __grid_constant__ RenderArgs a,
-                                                           const float4* __restrict__ g_img, long long* acc,
-                                                           const uint32_t* __restrict__ order, int ntiles,
-                                                           unsigned* __restrict__ next) {
+__global__ void __launch_bounds__(kThreads, VVLIC_ADJ_MIN_BLOCKS)
+    adjoint_kernel(const __grid_constant__ RenderArgs a, const float4* __restrict__ g_img, long long* acc, unsigned ntiles,
+                   unsigned* __restrict__ next) {
   __shared__ __align__(16) float s_tf[5 * VVLIC_TF_ENTRIES];
   __shared__ long long s_acc[kAccSize];
   for (int i = threadIdx.x; i < kAccSize; i += blockDim.x) s_acc[i] = 0;
   load_tf(a, s_tf);  // includes __syncthreads
-  const int lane = threadIdx.x & 31;
-  const int tiles_x = (a.W + kWarpTileW - 1) / kWarpTileW;
+  constexpr int S = 8, R = 32 / S;
+  const int lane = threadIdx.x & 31, k = lane / R, r = lane % R;
+  const unsigned tiles_x = (a.W + 1) / 2;
   const bool line = !GRAD && (a.illum == VVLIC_ILLUM_ZOECKLER || a.illum == VVLIC_ILLUM_MALLO);
-  float4 Dloc[kSegment];
-  float3 Ploc[kSegment];
   for (;;) {
     unsigned t = 0;
     if (lane == 0) t = atomicAdd(next, 1u);
     t = __shfl_sync(0xffffffffu, t, 0);
-    if (t >= (unsigned)ntiles) break;
-    const unsigned tile = __ldg(order + t);
-    const int px = (int)(tile % tiles_x) * kWarpTileW + (lane & (kWarpTileW - 1));
-    const int py = (int)(tile / tiles_x) * kWarpTileH + (lane / kWarpTileW);
-    const bool in_image = px < a.W && py < a.H;
-    const size_t ray = in_image ? (size_t)py * a.W + px : 0;
+    if (t >= ntiles) break;
+    const int px = (int)(t % tiles_x) * 2 + (r & 1), py = (int)(t / tiles_x) * 2 + (r >> 1);
     float3 pos0 = f3(0.f, 0.f, 0.f), dir = f3(0.f, 0.f, 0.f);
-    int S = 0;
+    int n = 0;  // samples of this lane's ray
     float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (in_image && ray_setup(a, px, py, pos0, dir)) {
-      S = (int)min(a.tape_n[ray], (uint32_t)a.tape_stride);
+    if (px < a.W && py < a.H && ray_setup(a, px, py, pos0, dir)) {
+      const size_t ray = (size_t)py * a.W + px;
+      n = (int)min(a.tape_n[ray], (uint32_t)a.tape_stride);
       g = g_img[ray];
     }
-    const int nseg = (S + kSegment - 1) / kSegment;
-    const int nseg_warp = __reduce_max_sync(0xffffffffu, (unsigned)nseg);
-    for (int seg = nseg_warp - 1; seg >= 0; --seg) {
-      const bool act_seg = seg < nseg;
-      int cnt = 0;
-      if (act_seg) {
+    const int most = (int)__reduce_max_sync(0xffffffffu, (unsigned)n);
+    for (int seg = (most + kSegment - 1) / kSegment - 1; seg >= 0; --seg) {
+      const int cnt = min(max(n - seg * kSegment, 0), kSegment), top = min(most - seg * kSegment, kSegment);
+      float4 D = make_float4(0.f, 0.f, 0.f, 0.f);
+      float3 p0 = f3(0.f, 0.f, 0.f);
+      if (cnt > 0) {
         size_t ce = tape_ck_entry(a, px, py, seg);
         if (!in_range(a, (long long)ce + 32, tape_ck_entries(a), VVLIC_CHECK_TAPE)) ce = 0;
-        const float4* ck = a.tape_ck + ce;
-        const float4 p4 = ck[0];
-        float3 p = f3(p4.x, p4.y, p4.z);
-        float4 D = ck[32];
-        cnt = min(kSegment, S - seg * kSegment);
-        for (int kk = 0; kk < cnt; ++kk) {
-          Ploc[kk] = p;
-          Dloc[kk] = D;
-          const size_t idx = tape_entry_checked(a, px, py, seg * kSegment + kk);
-          const float2 rec = a.tape_is[idx];
-          float4 src;
-          if (GRAD) {
-            const Src us = unlit_source(a, s_tf, rec.x, rec.y);
-            const float3 col = lit_color(a, lit_setup(a, tape_gradient(a, idx), p, dir), us.tf, rec.x);
-            src = make_float4(col.x, col.y, col.z, us.alpha);
-          } else if (line) {
-            const Src us = unlit_source(a, s_tf, rec.x, rec.y);
-            float3 d, sf;
-            line_factors(a, p, dir, Field<ST, FL>::sample(a, p), d, sf);
-            src = make_float4(us.tf.x * rec.x * d.x + sf.x, us.tf.y * rec.x * d.y + sf.y, us.tf.z * rec.x * d.z + sf.z,
-                              us.alpha);
-          } else {
-            src = unlit_source_rgba(a, s_tf, rec.x, rec.y);
-          }
-          D = blend(D, src);
-          p = add3(p, scl3(dir, a.step_size));
-        }
+        const float4 p4 = a.tape_ck[ce];
+        p0 = f3(p4.x, p4.y, p4.z);
+        D = a.tape_ck[ce + 32];
       }
-      for (int kk = kSegment - 1; kk >= 0; kk -= adj_samples_per_pass<INTEG>()) {
-        float gIraw;
-        float3 gG, pk;
-        sample_cotangent<ST, FL, GRAD>(a, s_tf, line, dir, Dloc, Ploc, px, py, seg, kk, cnt, g, s_acc, gIraw, gG, pk);
-        bool need = gIraw != 0.0f || (GRAD && (gG.x != 0.0f || gG.y != 0.0f || gG.z != 0.0f));
-        if constexpr (adj_samples_per_pass<INTEG>() == 2) {
-          float gIraw1;
-          float3 gG1, pk1;
-          sample_cotangent<ST, FL, GRAD>(a, s_tf, line, dir, Dloc, Ploc, px, py, seg, kk - 1, cnt, g, s_acc, gIraw1,
-                                         gG1, pk1);
-          need = need || gIraw1 != 0.0f || (GRAD && (gG1.x != 0.0f || gG1.y != 0.0f || gG1.z != 0.0f));
-          if (__any_sync(0xffffffffu, need))
-            tap_gradients2<ST, FL, NL, INTEG, GRAD>(a, pk, gIraw, gG, pk1, gIraw1, gG1, s_acc + kAccTaps);
-        } else {
-          if (__any_sync(0xffffffffu, need)) tap_gradients<ST, FL, NL, INTEG, GRAD>(a, pk, gIraw, gG, s_acc + kAccTaps);
+      for (int j = 0; j < k; ++j) p0 = march(p0, dir, a.step_size);  // of this lane's sample in chunk 0
+      // compositing state at the start of each chunk: chunk c's in the lanes of sample c
+      const int last = (top + S - 1) / S - 1;
+      float4 Dstart = D;
+      float3 p = p0;
+      for (int c = 0; c < last; ++c) {
+        float4 src = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c * S + k < cnt)
+          src = source_rgba(
+              tape_sample<ST, FL, GRAD>(a, s_tf, line, tape_entry_checked(a, px, py, seg * kSegment + c * S + k), p, dir).s);
+        for (int j = 0; j < S; ++j) {
+          const float4 s = shfl4(src, j * R + r);
+          if (c * S + j < cnt) D = blend(D, s);
         }
+        if (k == c + 1) Dstart = D;
+        for (int j = 0; j < S; ++j) p = march(p, dir, a.step_size);
+      }
+      for (int c = last; c >= 0; --c) {
+        p = p0;
+        for (int j = 0; j < c * S; ++j) p = march(p, dir, a.step_size);
+        const bool valid = c * S + k < cnt;
+        Sample<GRAD> q;
+        float4 src = make_float4(0.f, 0.f, 0.f, 0.f), sv = src;
+        if (valid) {
+          q = tape_sample<ST, FL, GRAD>(a, s_tf, line, tape_entry_checked(a, px, py, seg * kSegment + c * S + k), p, dir);
+          src = source_rgba(q.s);
+          sv = premultiplied(q.s);
+        }
+        // state before each sample; this lane keeps its own sample's
+        float4 Dmine = shfl4(Dstart, c * R + r);
+        D = Dmine;
+        for (int j = 0; j < S; ++j) {
+          const float4 s = shfl4(src, j * R + r);
+          if (j == k) Dmine = D;
+          if (c * S + j < cnt) D = blend(D, s);
+        }
+        float4 ds = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = S - 1; j >= 0; --j) {
+          const float4 svj = shfl4(sv, j * R + r), Dj = shfl4(Dmine, j * R + r);
+          if (c * S + j < cnt) {
+            float4 dsj;
+            g = blend_vjp(g, svj, Dj, dsj);
+            if (j == k) ds = dsj;
+          }
+        }
+        float gI = 0.0f;
+        float3 gG = f3(0.f, 0.f, 0.f);
+        if (valid) sample_cotangent<GRAD>(a, s_tf, line, q, ds, s_acc, gI, gG);
+        const bool need = gI != 0.0f || (GRAD && (gG.x != 0.0f || gG.y != 0.0f || gG.z != 0.0f));
+        if (__any_sync(0xffffffffu, need)) tap_gradients<ST, FL, NL, INTEG, GRAD>(a, p, gI, gG, s_acc + kAccTaps);
       }
     }
   }
@@ -443,43 +449,45 @@ __global__ void __launch_bounds__(kThreads, VVLIC_ADJ_MIN_BLOCKS) adjoint_kernel
 }
 
 template <int ST, int FL, int NL, int INTEG, bool GRAD>
-static cudaError_t launch_adjoint_one(const RenderArgs& a, const float4* g_img, long long* acc, const Schedule& sch,
-                                      cudaStream_t s) {
+static cudaError_t launch_adjoint_one(const RenderArgs& a, const float4* g_img, long long* acc, unsigned* next,
+                                      int num_sms, cudaStream_t s) {
   auto kern = adjoint_kernel<ST, FL, NL, INTEG, GRAD>;
   int per_sm = 0;
   cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, 0);
   if (e != cudaSuccess) return e;
-  kern<<<std::max(1, per_sm) * sch.num_sms, kThreads, 0, s>>>(a, g_img, acc, sch.order, sch.ntiles, sch.next);
+  const unsigned ntiles = (unsigned)((a.W + 1) / 2) * (unsigned)((a.H + 1) / 2);
+  const int grid = (int)std::min<unsigned>((ntiles + kWarps - 1) / kWarps, (unsigned)(std::max(1, per_sm) * num_sms));
+  kern<<<grid, kThreads, 0, s>>>(a, g_img, acc, ntiles, next);
   return cudaGetLastError();
 }
 
 template <int ST, int FL, int NL, bool GRAD>
 static cudaError_t launch_adjoint_integ(const RenderArgs& a, int integ, const float4* g_img, long long* acc,
-                                        const Schedule& sch, cudaStream_t s) {
-  if (integ == VVLIC_EULER) return launch_adjoint_one<ST, FL, NL, VVLIC_EULER, GRAD>(a, g_img, acc, sch, s);
-  if (integ == VVLIC_HEUN) return launch_adjoint_one<ST, FL, NL, VVLIC_HEUN, GRAD>(a, g_img, acc, sch, s);
-  return launch_adjoint_one<ST, FL, NL, VVLIC_RK4, GRAD>(a, g_img, acc, sch, s);
+                                        unsigned* next, int num_sms, cudaStream_t s) {
+  if (integ == VVLIC_EULER) return launch_adjoint_one<ST, FL, NL, VVLIC_EULER, GRAD>(a, g_img, acc, next, num_sms, s);
+  if (integ == VVLIC_HEUN) return launch_adjoint_one<ST, FL, NL, VVLIC_HEUN, GRAD>(a, g_img, acc, next, num_sms, s);
+  return launch_adjoint_one<ST, FL, NL, VVLIC_RK4, GRAD>(a, g_img, acc, next, num_sms, s);
 }
 
 template <int ST, int FL, int NL>
 static cudaError_t launch_adjoint_layout(const RenderArgs& a, int integ, bool lit, const float4* g_img,
-                                         long long* acc, const Schedule& sch, cudaStream_t s) {
-  return lit ? launch_adjoint_integ<ST, FL, NL, true>(a, integ, g_img, acc, sch, s)
-             : launch_adjoint_integ<ST, FL, NL, false>(a, integ, g_img, acc, sch, s);
+                                         long long* acc, unsigned* next, int num_sms, cudaStream_t s) {
+  return lit ? launch_adjoint_integ<ST, FL, NL, true>(a, integ, g_img, acc, next, num_sms, s)
+             : launch_adjoint_integ<ST, FL, NL, false>(a, integ, g_img, acc, next, num_sms, s);
 }
 
 template <int ST>
 static cudaError_t launch_adjoint_storage(const RenderArgs& a, int sampler, int integ, bool lit, const float4* g_img,
-                                          long long* acc, const Schedule& sch, cudaStream_t s) {
+                                          long long* acc, unsigned* next, int num_sms, cudaStream_t s) {
   switch (sampler) {
-    case VVLIC_SAMPLER_GATHER: return launch_adjoint_layout<ST, kGather, kGather>(a, integ, lit, g_img, acc, sch, s);
-    case VVLIC_SAMPLER_CELL: return launch_adjoint_layout<ST, kCell, kCell>(a, integ, lit, g_img, acc, sch, s);
+    case VVLIC_SAMPLER_GATHER: return launch_adjoint_layout<ST, kGather, kGather>(a, integ, lit, g_img, acc, next, num_sms, s);
+    case VVLIC_SAMPLER_CELL: return launch_adjoint_layout<ST, kCell, kCell>(a, integ, lit, g_img, acc, next, num_sms, s);
     case VVLIC_SAMPLER_TEXTURE:
       if constexpr (ST == VVLIC_STORAGE_BF16) return cudaErrorNotSupported;  // runs as F16 (kernel_storage)
-      else return launch_adjoint_layout<ST, kTexture, kTexture>(a, integ, lit, g_img, acc, sch, s);
+      else return launch_adjoint_layout<ST, kTexture, kTexture>(a, integ, lit, g_img, acc, next, num_sms, s);
     case VVLIC_SAMPLER_HYBRID:
       if constexpr (ST == VVLIC_STORAGE_BF16) return cudaErrorNotSupported;
-      else return launch_adjoint_layout<ST, kTexture, kCellFast>(a, integ, lit, g_img, acc, sch, s);
+      else return launch_adjoint_layout<ST, kTexture, kCellFast>(a, integ, lit, g_img, acc, next, num_sms, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -4,8 +4,8 @@
 namespace vvlic {
 
 cudaError_t launch_adjoint_bf16(const RenderArgs& a, int sampler, int integ, bool lit, const float4* g_img,
-                                long long* acc, const Schedule& sch, cudaStream_t s) {
-  return launch_adjoint_storage<VVLIC_STORAGE_BF16>(a, sampler, integ, lit, g_img, acc, sch, s);
+                               long long* acc, unsigned* next, int num_sms, cudaStream_t s) {
+  return launch_adjoint_storage<VVLIC_STORAGE_BF16>(a, sampler, integ, lit, g_img, acc, next, num_sms, s);
 }
 
 }  // namespace vvlic

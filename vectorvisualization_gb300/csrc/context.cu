@@ -399,7 +399,6 @@ extern "C" vvlic_status vvlic_destroy(vvlic_ctx* c) {
   for (cudaEvent_t ev : {c->ev_field_copied, c->ev_field_used, c->ev_noise_copied, c->ev_noise_used})
     if (ev) cudaEventDestroy(ev);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
-  if (c->d_sched) cudaFree(c->d_sched);
   if (c->d_tape) cudaFree(c->d_tape);
   if (c->d_tape_flag) cudaFree(c->d_tape_flag);
   if (c->d_acc) cudaFree(c->d_acc);

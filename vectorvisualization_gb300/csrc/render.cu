@@ -307,106 +307,9 @@ cudaError_t launch_raycast(const RenderArgs& a, int storage, int sampler, int in
   }
 }
 
-// ------------------------------------------------------------------------------------------
-// longest-first tile order for the adjoint's queue
-// ------------------------------------------------------------------------------------------
-namespace {
-
-constexpr int kBuckets = 1024;
-
-// One warp per 8x4 tile: the tile's cost is its longest ray's sample count (the warp runs until
-// that ray finishes), estimated from the ray-box chord: samples ~ chord / spacing + 1.
-__global__ void tile_cost_kernel(const __grid_constant__ RenderArgs a, int ntiles, int tiles_x, int shift,
-                                 unsigned* bucket, unsigned* hist) {
-  const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < ntiles; t += warps) {
-    const int px = (t % tiles_x) * 8 + (lane & 7), py = (t / tiles_x) * 4 + (lane >> 3);
-    unsigned cost = 0;
-    float o[3], d[3], tn, tf;
-    if (px < a.W && py < a.H && ray_interval(a, px, py, o, d, tn, tf)) {
-      const float len = (tf - tn) * sqrtf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-      cost = (unsigned)fminf(len / a.step_size + 1.0f, 4.0e9f);
-    }
-    cost = __reduce_max_sync(0xffffffffu, cost);
-    if (lane == 0) {
-      const unsigned b = kBuckets - 1 - min(cost >> shift, (unsigned)(kBuckets - 1));  // descending
-      bucket[t] = b;
-      atomicAdd(hist + b, 1u);
-    }
-  }
-}
-
-// Exclusive scan of the bucket histogram into start offsets (one CTA of kBuckets threads).
-__global__ void bucket_scan_kernel(const unsigned* hist, unsigned* offsets) {
-  __shared__ unsigned s[kBuckets];
-  const int i = threadIdx.x;
-  s[i] = hist[i];
-  __syncthreads();
-  for (int d = 1; d < kBuckets; d <<= 1) {
-    unsigned v = i >= d ? s[i - d] : 0u;
-    __syncthreads();
-    s[i] += v;
-    __syncthreads();
-  }
-  offsets[i] = s[i] - hist[i];
-}
-
-__global__ void tile_scatter_kernel(int ntiles, const unsigned* bucket, unsigned* offsets, unsigned* order) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x)
-    order[atomicAdd(offsets + bucket[t], 1u)] = (unsigned)t;
-}
-
-}  // namespace
-
-cudaError_t launch_tile_order(const RenderArgs& a, int ntiles, int tiles_x, int shift, unsigned* scratch,
-                              cudaStream_t s) {
-  unsigned* bucket = scratch;
-  unsigned* order = scratch + ntiles;
-  unsigned* hist = scratch + 2 * (size_t)ntiles;
-  unsigned* offsets = hist + kBuckets;
-  cudaError_t e = cudaMemsetAsync(hist, 0, kBuckets * sizeof(unsigned), s);
-  if (e != cudaSuccess) return e;
-  const int warps_per_block = 8;
-  const int blocks = std::min((ntiles + warps_per_block - 1) / warps_per_block, 152 * 16);
-  tile_cost_kernel<<<blocks, 32 * warps_per_block, 0, s>>>(a, ntiles, tiles_x, shift, bucket, hist);
-  bucket_scan_kernel<<<1, kBuckets, 0, s>>>(hist, offsets);
-  tile_scatter_kernel<<<std::min((ntiles + 255) / 256, 152 * 8), 256, 0, s>>>(ntiles, bucket, offsets, order);
-  return cudaGetLastError();
-}
-
 }  // namespace vvlic
 
 namespace {
-
-// Adjoint queue for one image: longest-first tile order in the context's scratch.
-vvlic_status make_schedule(vvlic_ctx* c, const RenderArgs& a, const Geometry& gm, int w, int h, cudaStream_t s,
-                           Schedule& sch) {
-  const int tiles_x = (w + 7) / 8, ntiles = tiles_x * ((h + 3) / 4);
-  const size_t words = 2 * (size_t)ntiles + 2 * 1024 + 1;
-  if (c->sched_cap < words) {
-    if (c->d_sched) cudaFree(c->d_sched);
-    c->d_sched = nullptr;
-    c->sched_cap = 0;
-    cudaError_t e = cudaMalloc(&c->d_sched, words * sizeof(unsigned));
-    if (e != cudaSuccess) return cuda_fail(c, e, "schedule allocation");
-    c->sched_cap = words;
-  }
-  // cost buckets of 2^shift samples so the longest possible chord fits 1024 buckets
-  const double diag = std::sqrt((double)gm.extent[0] * gm.extent[0] + (double)gm.extent[1] * gm.extent[1] +
-                                (double)gm.extent[2] * gm.extent[2]);
-  const double maxcost = diag / a.step_size + 2.0;
-  int shift = 0;
-  while ((maxcost / (double)(1u << shift)) >= 1024.0 && shift < 31) ++shift;
-  unsigned* scratch = c->d_sched;
-  cudaError_t e = launch_tile_order(a, ntiles, tiles_x, shift, scratch, s);
-  sch.order = scratch + ntiles;
-  sch.ntiles = ntiles;
-  sch.next = scratch + 2 * (size_t)ntiles + 2 * 1024;
-  if (e == cudaSuccess) e = cudaMemsetAsync(sch.next, 0, sizeof(unsigned), s);
-  if (e != cudaSuccess) return cuda_fail(c, e, "schedule");
-  return VVLIC_OK;
-}
 
 // Tape buffers for a recording render: per ray `stride` samples (the longest march / spacing,
 // capped by the two loop bounds) and a checkpoint every kSegment samples.  A ray marches in
@@ -576,29 +479,25 @@ extern "C" vvlic_status vvlic_render_adjoint(vvlic_ctx* c, int32_t vol_id, const
   const int acc_size = 5 * VVLIC_TF_ENTRIES + kMaxTaps;
   cudaError_t e = cudaSuccess;
   if (!c->d_acc) {
-    e = cudaMalloc(&c->d_acc, acc_size * sizeof(long long));
+    e = cudaMalloc(&c->d_acc, (acc_size + 1) * sizeof(long long));  // the accumulators and the queue counter
     if (e != cudaSuccess) return cuda_fail(c, e, "adjoint accumulators");
   }
-  e = cudaMemsetAsync(c->d_acc, 0, acc_size * sizeof(long long), s);
+  e = cudaMemsetAsync(c->d_acc, 0, (acc_size + 1) * sizeof(long long), s);
   if (e != cudaSuccess) return cuda_fail(c, e, "adjoint");
   const RenderArgs& a = c->tape_args;
-  Schedule sch;
-  sch.num_sms = c->num_sms;
-  auto vt = c->vols.find(vol_id);
-  if (vt == c->vols.end()) return fail(c, VVLIC_ERR_INVALID_ARGUMENT, "render_adjoint: unknown volume %d", vol_id);
-  vvlic_status st = make_schedule(c, a, vt->second.geom, w, h, s, sch);
-  if (st) return st;
+  unsigned* next = reinterpret_cast<unsigned*>(c->d_acc + acc_size);
+  const int sms = c->num_sms;
   e = cudaEventRecord(c->ev0, s);
   const float4* gi = (const float4*)d_dl_drgba;
   if (e == cudaSuccess) {
     const bool lit = c->tape_illum == VVLIC_ILLUM_GRADIENT;
     switch (kernel_storage(c->tape_storage, c->tape_sampler)) {
-      case VVLIC_STORAGE_F32: e = launch_adjoint_f32(a, c->tape_sampler, c->tape_integ, lit, gi, c->d_acc, sch, s); break;
-      case VVLIC_STORAGE_F16: e = launch_adjoint_f16(a, c->tape_sampler, c->tape_integ, lit, gi, c->d_acc, sch, s); break;
+      case VVLIC_STORAGE_F32: e = launch_adjoint_f32(a, c->tape_sampler, c->tape_integ, lit, gi, c->d_acc, next, sms, s); break;
+      case VVLIC_STORAGE_F16: e = launch_adjoint_f16(a, c->tape_sampler, c->tape_integ, lit, gi, c->d_acc, next, sms, s); break;
       case VVLIC_STORAGE_UNORM8:
-        e = launch_adjoint_u8(a, c->tape_sampler, c->tape_integ, lit, gi, c->d_acc, sch, s);
+        e = launch_adjoint_u8(a, c->tape_sampler, c->tape_integ, lit, gi, c->d_acc, next, sms, s);
         break;
-      default: e = launch_adjoint_bf16(a, c->tape_sampler, c->tape_integ, lit, gi, c->d_acc, sch, s); break;
+      default: e = launch_adjoint_bf16(a, c->tape_sampler, c->tape_integ, lit, gi, c->d_acc, next, sms, s); break;
     }
   }
   if (e == cudaSuccess) e = cudaEventRecord(c->ev1, s);

@@ -127,8 +127,6 @@ struct vvlic_ctx {
   size_t field_stage_cap = 0;
   void* d_noise_stage = nullptr;
   size_t noise_stage_cap = 0;
-  unsigned* d_sched = nullptr;    // tile order scratch of the adjoint's queue
-  size_t sched_cap = 0;           // in 4-byte words
   int num_sms = 1;
   // adjoint tape of the last recording render
   void* d_tape = nullptr;

@@ -23,15 +23,6 @@ cudaError_t launch_technique_bf16(const RenderArgs& a, const TechArgs& t, int sa
 cudaError_t launch_technique_u8(const RenderArgs& a, const TechArgs& t, int sampler, int integ, bool grad,
                                 cudaStream_t s);
 
-// Work queue of an adjoint launch: persistent CTAs pull `ntiles` 8x4-pixel tiles in `order` through
-// the counter `next`.
-struct Schedule {
-  const uint32_t* order = nullptr;
-  int ntiles = 0;
-  unsigned* next = nullptr;
-  int num_sms = 1;
-};
-
 // Forward ray-cast, one launcher per field storage (render_<storage>.cu).
 cudaError_t launch_raycast_f32(const RenderArgs& a, int sampler, int integ, bool grad, int num_sms, cudaStream_t s);
 cudaError_t launch_raycast_f16(const RenderArgs& a, int sampler, int integ, bool grad, int num_sms, cudaStream_t s);
@@ -39,15 +30,16 @@ cudaError_t launch_raycast_bf16(const RenderArgs& a, int sampler, int integ, boo
 cudaError_t launch_raycast_u8(const RenderArgs& a, int sampler, int integ, bool grad, int num_sms, cudaStream_t s);
 
 // Adjoint of the unlit (lit == false) or gradient-lit render (adjoint_<storage>.cu):
-// accumulates 64-bit fixed-point gradients into acc (TF 1024, opacity 256, taps).
+// accumulates 64-bit fixed-point gradients into acc (TF 1024, opacity 256, taps).  `next`: the
+// launch's work queue counter, zero.
 cudaError_t launch_adjoint_f32(const RenderArgs& a, int sampler, int integ, bool lit, const float4* g_img,
-                               long long* acc, const Schedule& sch, cudaStream_t s);
+                               long long* acc, unsigned* next, int num_sms, cudaStream_t s);
 cudaError_t launch_adjoint_f16(const RenderArgs& a, int sampler, int integ, bool lit, const float4* g_img,
-                               long long* acc, const Schedule& sch, cudaStream_t s);
+                               long long* acc, unsigned* next, int num_sms, cudaStream_t s);
 cudaError_t launch_adjoint_bf16(const RenderArgs& a, int sampler, int integ, bool lit, const float4* g_img,
-                                long long* acc, const Schedule& sch, cudaStream_t s);
+                                long long* acc, unsigned* next, int num_sms, cudaStream_t s);
 cudaError_t launch_adjoint_u8(const RenderArgs& a, int sampler, int integ, bool lit, const float4* g_img,
-                              long long* acc, const Schedule& sch, cudaStream_t s);
+                              long long* acc, unsigned* next, int num_sms, cudaStream_t s);
 
 // Batched render (batch_<storage>.cu): one persistent launch over (job, tile) items.
 struct BatchLaunch {
@@ -84,11 +76,6 @@ inline BatchScratch batch_scratch(unsigned* base, int njobs, int ntiles) {
 // Job-major (job, tile) order over a batch (batch.cu); start[] holds njobs+1 entries
 // (exclusive prefix of tiles per job).
 cudaError_t launch_batch_order(const BatchScratch& b, int njobs, int ntiles, cudaStream_t s);
-
-// Longest-first tile order for the adjoint's queue (render.cu): per-tile chord cost, a
-// counting sort over 1024 cost buckets, scatter.  `scratch` holds 2*ntiles + 2048 + 1 words.
-cudaError_t launch_tile_order(const RenderArgs& a, int ntiles, int tiles_x, int shift, unsigned* scratch,
-                              cudaStream_t s);
 
 // BRICK sampler (brick.cu): brick shapes and TMA maps for a render of volume v, and its launch.
 struct BrickArgs;
