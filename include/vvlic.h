@@ -474,19 +474,21 @@ typedef struct vvlic_job {
   int32_t filter_clamp;
 } vvlic_job;
 
-/* Render n jobs in one persistent launch: every (job, 8x4 tile) item goes into one device work
- * queue in job-major order (jobs in submission order, each job's tiles in raster order), so the
- * warps in flight share one or two volumes' texels in cache.  All jobs must share the field storage,
- * sampler, integrator and lighting (they are compiled variants); LIC length, step sizes,
- * filter, view, image size, TF index and the other runtime parameters may differ.  The noise,
- * scalar volume and transfer function are the context's.  The launch sequence is captured in a
- * CUDA graph the first time a batch of a given shape is rendered and replayed afterwards
- * (only the job table is re-uploaded).  `stream` must not be the legacy default stream (NULL
- * selects the context's stream).  Asynchronous; vvlic_get_stats reports the batch totals. */
+/* Render n jobs side by side.  Jobs of 30 x 30 pixels and more (on average) are launched one by one over
+ * `stream` and streams of the context, joined back into `stream`.  Smaller ones go through one persistent
+ * launch: every (job, 8x4 tile) item enters one device work queue in job-major order (jobs in
+ * submission order, each job's tiles in raster order), and the launch sequence is captured in a
+ * CUDA graph the first time a batch of a given shape is rendered and replayed afterwards (only the
+ * job table is re-uploaded).  All jobs must share the field storage, sampler, integrator and
+ * lighting (they are compiled variants); LIC length, step sizes, filter, view, image size, TF
+ * index and the other runtime parameters may differ.  The noise, scalar volume and transfer function
+ * are the context's.  `stream` must not be the legacy default stream (NULL selects the context's
+ * stream).  Asynchronous; vvlic_get_stats reports the batch totals. */
 vvlic_status vvlic_batch_render(vvlic_ctx* ctx, const vvlic_job* jobs, int32_t n, void* stream);
 
-/* Time the batch under each warp tile shape (8x4, 4x8, 16x2, 32x1 pixels) and each exact-noise
- * sampler (HYBRID, CELL) that the jobs' storage supports, keep the fastest for later batches of
+/* Time the batch under each warp tile shape of the persistent launch (8x4, 4x8, 16x2, 32x1 pixels; jobs
+ * launched one by one have none and report 8) and each exact-noise sampler (HYBRID, CELL) that the
+ * jobs' storage supports, keep the fastest for later batches of
  * this context and report it (tile width, sampler, milliseconds).  Renders the batch several
  * times.  Synchronous. */
 vvlic_status vvlic_batch_autotune(vvlic_ctx* ctx, const vvlic_job* jobs, int32_t n, void* stream,

@@ -1,5 +1,6 @@
-// Batched rendering: job table, job-major (job, tile) order over the whole batch, the
-// CUDA-graph-captured launch sequence and the tile-shape / sampler autotuner.
+// Batched rendering: jobs launched one by one over eight streams or, small ones, in one persistent launch
+// (job table, job-major (job, tile) order, CUDA-graph-captured launch sequence); the tile-shape /
+// sampler autotuner.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -148,6 +149,52 @@ vvlic_status prepare_batch(vvlic_ctx* c, const vvlic_job* jobs, int n, int tw, i
   return VVLIC_OK;
 }
 
+// Jobs of some size are launched one by one, dealt to the caller's stream and seven of the context's so
+// that one job's tail runs beside the next ones' starts.  A kernel of its own reads its arguments
+// from the constant bank, as operands; the persistent kernel has to hold them in shared memory and loads
+// them again and again through the pipe that also serves the noise cells.  24 views of 8 uneven
+// volumes, one by one / persistent: 86.5 / 105.6 ms at 512^2 (lit 136 / 223), 26.5 / 37.1 at 256^2, 3.2 /
+// 12.7 at 64^2; 320 views at 32^2 14.9 / 21.9 ms, 800 at 16^2 27.6 / 13.6 (launches).  The line lies at a mean
+// of a sixteenth of the resident warps in 2x2-ray tiles, 30^2 pixels.
+bool job_by_job(const vvlic_ctx* c, const vvlic_job* jobs, int n) {
+  double tiles = 0.0;
+  for (int j = 0; j < n; ++j) tiles += (double)((jobs[j].w + 1) / 2) * (double)((jobs[j].h + 1) / 2);
+  return tiles >= 24.0 / 16.0 * c->num_sms * n;
+}
+
+vvlic_status launch_jobs(vvlic_ctx* c, int n, int storage, int sampler, int integ, bool grad, cudaStream_t s) {
+  constexpr int B = vvlic_ctx::kBatchStreams;
+  cudaError_t e = cudaSuccess;
+  if (!c->ev_batch_fork) {
+    for (int b = 0; b < B && e == cudaSuccess; ++b) {
+      if (!c->batch_streams[b]) e = cudaStreamCreateWithFlags(&c->batch_streams[b], cudaStreamNonBlocking);
+      if (e == cudaSuccess && !c->ev_batch_join[b]) e = cudaEventCreateWithFlags(&c->ev_batch_join[b], cudaEventDisableTiming);
+    }
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_batch_fork, cudaEventDisableTiming);
+    if (e != cudaSuccess) return cuda_fail(c, e, "batch streams");
+  }
+  const int used = std::min(n - 1, B);
+  e = cudaMemsetAsync(c->d_counters, 0, 4 * sizeof(unsigned long long), s);
+  if (e == cudaSuccess) e = cudaEventRecord(c->ev0, s);
+  if (e == cudaSuccess) e = cudaEventRecord(c->ev_batch_fork, s);
+  for (int b = 0; b < used && e == cudaSuccess; ++b) e = cudaStreamWaitEvent(c->batch_streams[b], c->ev_batch_fork, 0);
+  for (int j = 0; j < n && e == cudaSuccess; ++j) {
+    RenderArgs& a = c->h_jobs[j];
+    a.count_steps = 1;
+    const int b = j % (used + 1);
+    e = launch_raycast(a, storage, sampler, integ, grad, c->num_sms, b == 0 ? s : c->batch_streams[b - 1]);
+  }
+  // joined even after a failed launch: nothing on the side streams outlives the caller's stream
+  for (int b = 0; b < used; ++b) {
+    cudaError_t ej = cudaEventRecord(c->ev_batch_join[b], c->batch_streams[b]);
+    if (ej == cudaSuccess) ej = cudaStreamWaitEvent(s, c->ev_batch_join[b], 0);
+    if (e == cudaSuccess) e = ej;
+  }
+  if (e == cudaSuccess) e = cudaEventRecord(c->ev1, s);
+  if (e != cudaSuccess) return cuda_fail(c, e, "batch launch");
+  return VVLIC_OK;
+}
+
 vvlic_status batch_render(vvlic_ctx* c, const vvlic_job* jobs, int n, cudaStream_t s, int tw, int sampler_override) {
   int storage, sampler, integ, ntiles;
   bool grad;
@@ -155,6 +202,14 @@ vvlic_status batch_render(vvlic_ctx* c, const vvlic_job* jobs, int n, cudaStream
   vvlic_status st = prepare_batch(c, jobs, n, tw, sampler_override, s, &storage, &sampler, &integ, &grad, &ntiles,
                                   start);
   if (st) return st;
+  if (job_by_job(c, jobs, n)) {
+    if ((st = launch_jobs(c, n, storage, sampler, integ, grad, s))) return st;
+    c->stats_pending = true;
+    c->tape_flag_pending = false;
+    c->last_was_batch = true;
+    c->tape_valid = false;
+    return VVLIC_OK;
+  }
   // device buffers; a reallocation invalidates the captured graph
   const void* old_jobs = c->d_jobs;
   const void* old_batch = c->d_batch;
@@ -236,8 +291,10 @@ extern "C" vvlic_status vvlic_batch_autotune(vvlic_ctx* c, const vvlic_job* jobs
   const int tws[4] = {8, 4, 16, 32};
   float best = 1e30f;
   int bt = c->batch_tile_w, bs = jobs[0].params.sampler;
+  const bool shaped = !job_by_job(c, jobs, n);  // launched one by one, the jobs have no tile shape
   for (int smp : samplers) {
     for (int tw : tws) {
+      if (!shaped && tw != tws[0]) continue;
       float ms = 0.f;
       for (int rep = 0; rep < 2; ++rep) {  // the first render builds layouts and the graph
         vvlic_status st = batch_render(c, jobs, n, s, tw, smp);

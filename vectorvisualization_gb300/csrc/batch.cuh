@@ -1,9 +1,9 @@
-// Batched LIC ray-cast: many render jobs (volume x view x image, each with its own LIC
-// parameters and filter) in one persistent launch.  Warps pull (job, tile) items from one
-// device work queue in job-major order (batch.cu) and trace a tile's rays in groups of four samples
-// (trace_group); on a job switch a warp copies that
-// job's argument block into its own shared-memory slot and traces the tile from there.  The
-// transfer function is the context's and is shared by every job.
+// Batched LIC ray-cast of small images: many render jobs (volume x view x image, each with its own LIC
+// parameters and filter) in one persistent launch (batch.cu, job_by_job).  Warps pull (job, tile)
+// items from one device work queue in job-major order and trace a tile's rays in groups of four
+// samples (trace_group); on a job switch a warp copies that job's argument block into its own
+// shared-memory slot and traces the tile from there.  The transfer function is the context's and
+// is shared by every job.
 #pragma once
 
 #include "render_fwd.cuh"

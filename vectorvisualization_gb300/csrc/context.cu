@@ -407,6 +407,11 @@ extern "C" vvlic_status vvlic_destroy(vvlic_ctx* c) {
   if (c->d_jobs) cudaFree(c->d_jobs);
   if (c->d_batch) cudaFree(c->d_batch);
   if (c->ev_jobs) cudaEventDestroy(c->ev_jobs);
+  for (cudaStream_t b : c->batch_streams)
+    if (b) cudaStreamDestroy(b);
+  for (cudaEvent_t ev : c->ev_batch_join)
+    if (ev) cudaEventDestroy(ev);
+  if (c->ev_batch_fork) cudaEventDestroy(c->ev_batch_fork);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->stream) cudaStreamDestroy(c->stream);

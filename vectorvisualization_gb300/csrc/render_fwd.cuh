@@ -54,6 +54,7 @@ __device__ __forceinline__ void flush_counters(const RenderArgs& a, uint32_t sam
   unsigned h = __reduce_add_sync(0xffffffffu, hits);
   if ((threadIdx.x & 31) == 0) {
     if (s) atomicAdd(a.counters + 0, (unsigned long long)s);
+    if (s && a.count_steps) atomicAdd(a.counters + 2, (unsigned long long)s * (unsigned)(a.lb + a.lf));
     if (h) atomicAdd(a.counters + 1, (unsigned long long)h);
   }
 }

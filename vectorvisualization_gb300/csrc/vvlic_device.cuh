@@ -35,7 +35,8 @@ struct RenderArgs {
   const float* tf;            // 256 RGBA entries followed by 256 opacity entries
   float* out;                 // W*H RGBA
   uint32_t* samples;          // optional per-pixel sample counts
-  unsigned long long* counters;  // [0] samples, [1] rays
+  unsigned long long* counters;  // [0] samples, [1] rays, [2] sample-steps (count_steps)
+  int count_steps;               // batches: jobs of different lengths share the counters
   int W, H;
   float o0[3], o1[3], o2[3], d0[3], d1[3], d2[3];
   int clamp0;

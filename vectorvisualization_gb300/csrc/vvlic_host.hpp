@@ -150,6 +150,10 @@ struct vvlic_ctx {
   int batch_tile_w = 8;                 // warp tile width (autotuned)
   int batch_sampler_override = -1;      // sampler chosen by the autotuner (-1: the jobs')
   bool last_was_batch = false;
+  // streams of batches whose jobs are launched one by one (batch.cu), created on first use
+  static constexpr int kBatchStreams = 7;
+  cudaStream_t batch_streams[kBatchStreams] = {};
+  cudaEvent_t ev_batch_fork = nullptr, ev_batch_join[kBatchStreams] = {};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   bool stats_pending = false;
   uint64_t stats_steps_per_sample = 0;

@@ -29,6 +29,10 @@ cudaError_t launch_raycast_f16(const RenderArgs& a, int sampler, int integ, bool
 cudaError_t launch_raycast_bf16(const RenderArgs& a, int sampler, int integ, bool grad, int num_sms, cudaStream_t s);
 cudaError_t launch_raycast_u8(const RenderArgs& a, int sampler, int integ, bool grad, int num_sms, cudaStream_t s);
 
+// The same by storage (render.cu).
+cudaError_t launch_raycast(const RenderArgs& a, int storage, int sampler, int integ, bool grad, int num_sms,
+                           cudaStream_t s);
+
 // Adjoint of the unlit (lit == false) or gradient-lit render (adjoint_<storage>.cu):
 // accumulates 64-bit fixed-point gradients into acc (TF 1024, opacity 256, taps).  `next`: the
 // launch's work queue counter, zero.
