@@ -288,11 +288,6 @@ __device__ __forceinline__ Sample<GRAD> tape_sample(const RenderArgs& a, const f
 // The source as blend() takes it (colour not yet multiplied by alpha), matching shade().
 __device__ __forceinline__ float4 source_rgba(const Src& s) { return make_float4(s.col.x, s.col.y, s.col.z, s.alpha); }
 
-__device__ __forceinline__ float4 shfl4(float4 v, int from) {
-  return make_float4(__shfl_sync(0xffffffffu, v.x, from), __shfl_sync(0xffffffffu, v.y, from),
-                     __shfl_sync(0xffffffffu, v.z, from), __shfl_sync(0xffffffffu, v.w, from));
-}
-
 // The image cotangent g through clamp((1 - Dp.a) * sv + Dp) (derivative 1 on [0, 1]) to the
 // one before the sample; ds: the cotangent of the premultiplied source.
 __device__ __forceinline__ float4 blend_vjp(float4 g, float4 sv, float4 Dp, float4& ds) {

@@ -288,12 +288,12 @@ vvlic_status build_render_args_ex(vvlic_ctx* c, Volume& v, int W, int H, cudaStr
 }
 
 cudaError_t launch_technique(int storage, const RenderArgs& a, const TechArgs& t, int sampler, int integ, bool grad,
-                             cudaStream_t s) {
+                             int num_sms, cudaStream_t s) {
   switch (kernel_storage(storage, sampler)) {
-    case VVLIC_STORAGE_F32: return launch_technique_f32(a, t, sampler, integ, grad, s);
-    case VVLIC_STORAGE_F16: return launch_technique_f16(a, t, sampler, integ, grad, s);
-    case VVLIC_STORAGE_UNORM8: return launch_technique_u8(a, t, sampler, integ, grad, s);
-    default: return launch_technique_bf16(a, t, sampler, integ, grad, s);
+    case VVLIC_STORAGE_F32: return launch_technique_f32(a, t, sampler, integ, grad, num_sms, s);
+    case VVLIC_STORAGE_F16: return launch_technique_f16(a, t, sampler, integ, grad, num_sms, s);
+    case VVLIC_STORAGE_UNORM8: return launch_technique_u8(a, t, sampler, integ, grad, num_sms, s);
+    default: return launch_technique_bf16(a, t, sampler, integ, grad, num_sms, s);
   }
 }
 
@@ -397,7 +397,8 @@ extern "C" vvlic_status vvlic_render_device(vvlic_ctx* c, int32_t vol_id, float*
     if (e == cudaSuccess) e = cudaEventRecord(c->ev0, s);
     if (e == cudaSuccess)
       e = launch_technique(v.storage, a, t, c->params.sampler, c->params.integrator,
-                           c->params.illum == VVLIC_ILLUM_GRADIENT && t.technique == VVLIC_TECHNIQUE_SLICING, s);
+                           c->params.illum == VVLIC_ILLUM_GRADIENT && t.technique == VVLIC_TECHNIQUE_SLICING, c->num_sms,
+                           s);
     if (e == cudaSuccess) e = cudaEventRecord(c->ev1, s);
     if (e != cudaSuccess) return cuda_fail(c, e, "render launch");
     c->stats_pending = true;
@@ -628,7 +629,7 @@ extern "C" vvlic_status vvlic_compute_lic_volume(vvlic_ctx* c, int32_t vol_id, i
   for (int i = 0; i < 3; ++i) a.scale_vol[i] = v.geom.scale[i];
   cudaError_t e = cudaMemsetAsync(c->d_counters, 0, 4 * sizeof(unsigned long long), s);
   if (e == cudaSuccess) e = cudaEventRecord(c->ev0, s);
-  if (e == cudaSuccess) e = launch_technique(v.storage, a, t, c->params.sampler, c->params.integrator, false, s);
+  if (e == cudaSuccess) e = launch_technique(v.storage, a, t, c->params.sampler, c->params.integrator, false, c->num_sms, s);
   if (e == cudaSuccess) e = cudaEventRecord(c->ev1, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(c, e, "compute_lic_volume");

@@ -31,7 +31,7 @@ constexpr int kThreads = 128, kWarps = kThreads / 32;
 #define VVLIC_RK4_MIN_BLOCKS 5
 #endif
 template <int INTEG> constexpr int min_blocks() { return INTEG == VVLIC_RK4 ? VVLIC_RK4_MIN_BLOCKS : VVLIC_MIN_BLOCKS; }
-template <int INTEG> constexpr int cast_threads() { return INTEG == VVLIC_RK4 ? 128 : 256; }
+template <int INTEG> __host__ __device__ constexpr int cast_threads() { return INTEG == VVLIC_RK4 ? 128 : 256; }
 
 __device__ __forceinline__ void load_tf(const RenderArgs& a, float* s_tf) {
   for (int i = threadIdx.x; i < 5 * VVLIC_TF_ENTRIES; i += blockDim.x) s_tf[i] = __ldg(a.tf + i);
@@ -106,17 +106,22 @@ __global__ void __launch_bounds__(cast_threads<INTEG>(), min_blocks<INTEG>() * 1
 //   128 threads otherwise.
 // RK4 grids run up strips of 16 CTAs, so that the rays in flight are a block of the image and not a
 // few rows: 2048^2 orbit frame 1379 against 1404 ms, 1024^2 447 against 453 (Heun: 59.6 against 58.9).
+inline long long cast_tiles(const RenderArgs& a) { return (long long)((a.W + 1) / 2) * ((a.H + 1) / 2); }
+inline long long resident_warps(int num_sms) { return 24ll * num_sms; }
+template <int INTEG, bool GRAD> static int cast_cta_threads(const RenderArgs& a, int num_sms) {
+  const long long tiles = cast_tiles(a), resident = resident_warps(num_sms);
+  return tiles <= 2 * resident ? 64 : (GRAD && INTEG != VVLIC_RK4 && tiles >= 16 * resident ? 256 : 128);
+}
+
 template <int ST, int FL, int NL, int INTEG, bool GRAD>
 static cudaError_t launch_one(const RenderArgs& a, int num_sms, cudaStream_t stream) {
-  const long long resident = 24ll * num_sms;
-  const long long tiles = (long long)((a.W + 1) / 2) * ((a.H + 1) / 2);
-  const int threads = tiles <= 2 * resident ? 64 : (GRAD && INTEG != VVLIC_RK4 && tiles >= 16 * resident ? 256 : 128);
+  const int threads = cast_cta_threads<INTEG, GRAD>(a, num_sms);
   const int strip = INTEG == VVLIC_RK4 ? 16 : 0;
   const CtaShape cta = cta_shape(threads);
   const auto grid = [&](int th) {
     return dim3((unsigned)((a.W + 2 * cta.wx - 1) / (2 * cta.wx)), (unsigned)((a.H + th * cta.wy - 1) / (th * cta.wy)));
   };
-  if (2 * tiles <= resident)
+  if (2 * cast_tiles(a) <= resident_warps(num_sms))
     raycast_kernel<ST, FL, NL, INTEG, GRAD, 16><<<grid(GroupTile<16>::h), threads, 0, stream>>>(a, strip);
   else
     raycast_kernel<ST, FL, NL, INTEG, GRAD, 8><<<grid(GroupTile<8>::h), threads, 0, stream>>>(a, strip);

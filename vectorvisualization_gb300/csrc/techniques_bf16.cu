@@ -4,8 +4,8 @@
 namespace vvlic {
 
 cudaError_t launch_technique_bf16(const RenderArgs& a, const TechArgs& t, int sampler, int integ, bool grad,
-                                 cudaStream_t s) {
-  return launch_tech_storage<VVLIC_STORAGE_BF16>(a, t, sampler, integ, grad, s);
+                                  int num_sms, cudaStream_t s) {
+  return launch_tech_storage<VVLIC_STORAGE_BF16>(a, t, sampler, integ, grad, num_sms, s);
 }
 
 }  // namespace vvlic

@@ -1044,6 +1044,11 @@ __device__ __forceinline__ void record_sample(const RenderArgs& a, int px, int p
   }
 }
 
+__device__ __forceinline__ float4 shfl4(float4 v, int from) {
+  return make_float4(__shfl_sync(0xffffffffu, v.x, from), __shfl_sync(0xffffffffu, v.y, from),
+                     __shfl_sync(0xffffffffu, v.z, from), __shfl_sync(0xffffffffu, v.w, from));
+}
+
 __device__ __forceinline__ float3 march(float3 p, float3 dir, float step) {
   return f3(fmaf(dir.x, step, p.x), fmaf(dir.y, step, p.y), fmaf(dir.z, step, p.z));
 }
@@ -1100,8 +1105,7 @@ __device__ __forceinline__ float4 trace_group(const RenderArgs& a, const float* 
 #pragma unroll (S < 8 ? S : 8)
     for (int j = 0; j < S; ++j) {
       const int from = j * R + r;
-      const float4 s = make_float4(__shfl_sync(0xffffffffu, src.x, from), __shfl_sync(0xffffffffu, src.y, from),
-                                   __shfl_sync(0xffffffffu, src.z, from), __shfl_sync(0xffffffffu, src.w, from));
+      const float4 s = shfl4(src, from);
       if (alive && from <= last) {
         dest = blend(dest, s);
         ++samples;

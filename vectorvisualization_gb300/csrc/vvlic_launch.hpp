@@ -15,13 +15,13 @@ struct TechArgs;
 
 // Slicing, vector-field DVR, LIC-volume precompute and DVR (techniques_<storage>.cu).
 cudaError_t launch_technique_f32(const RenderArgs& a, const TechArgs& t, int sampler, int integ, bool grad,
-                                 cudaStream_t s);
+                                 int num_sms, cudaStream_t s);
 cudaError_t launch_technique_f16(const RenderArgs& a, const TechArgs& t, int sampler, int integ, bool grad,
-                                 cudaStream_t s);
+                                 int num_sms, cudaStream_t s);
 cudaError_t launch_technique_bf16(const RenderArgs& a, const TechArgs& t, int sampler, int integ, bool grad,
-                                  cudaStream_t s);
+                                 int num_sms, cudaStream_t s);
 cudaError_t launch_technique_u8(const RenderArgs& a, const TechArgs& t, int sampler, int integ, bool grad,
-                                cudaStream_t s);
+                                 int num_sms, cudaStream_t s);
 
 // Forward ray-cast, one launcher per field storage (render_<storage>.cu).
 cudaError_t launch_raycast_f32(const RenderArgs& a, int sampler, int integ, bool grad, int num_sms, cudaStream_t s);
