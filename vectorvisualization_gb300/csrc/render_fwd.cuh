@@ -30,8 +30,17 @@ constexpr int kThreads = 128, kWarps = kThreads / 32;
 #ifndef VVLIC_RK4_MIN_BLOCKS
 #define VVLIC_RK4_MIN_BLOCKS 5
 #endif
-template <int INTEG> constexpr int min_blocks() { return INTEG == VVLIC_RK4 ? VVLIC_RK4_MIN_BLOCKS : VVLIC_MIN_BLOCKS; }
+template <int INTEG> __host__ __device__ constexpr int min_blocks() {
+  return INTEG == VVLIC_RK4 ? VVLIC_RK4_MIN_BLOCKS : VVLIC_MIN_BLOCKS;
+}
+// Lit FP32 kernels take two texture fetches and a 32-byte cell per evaluation: up to 128 registers (2 CTAs of
+// 256 threads per SM) against 80, 256^3 frame at 128^2 / 256^2 / 512^2 / 1024^2 4.07 / 8.89 / 26.4 / 93.8 against
+// 3.94 / 9.65 / 27.3 / 93.7 ms, Euler at 512^2 15.9 against 16.6.  Unlit ones lose on small frames (128^2
+// preview 214 against 188 us, 256^2 Euler 1447 against 1428) what they gain on a 512^2 one (30.1 against 32.6 ms).
 template <int INTEG> __host__ __device__ constexpr int cast_threads() { return INTEG == VVLIC_RK4 ? 128 : 256; }
+template <int ST, int INTEG, bool GRAD> __host__ __device__ constexpr int cast_min_ctas() {
+  return ST == VVLIC_STORAGE_F32 && GRAD && INTEG != VVLIC_RK4 ? 2 : min_blocks<INTEG>() * 128 / cast_threads<INTEG>();
+}
 
 __device__ __forceinline__ void load_tf(const RenderArgs& a, float* s_tf) {
   for (int i = threadIdx.x; i < 5 * VVLIC_TF_ENTRIES; i += blockDim.x) s_tf[i] = __ldg(a.tf + i);
@@ -71,7 +80,7 @@ __host__ __device__ inline CtaShape cta_shape(int threads) {
 }
 
 template <int ST, int FL, int NL, int INTEG, bool GRAD, int S>
-__global__ void __launch_bounds__(cast_threads<INTEG>(), min_blocks<INTEG>() * 128 / cast_threads<INTEG>())
+__global__ void __launch_bounds__(cast_threads<INTEG>(), cast_min_ctas<ST, INTEG, GRAD>())
     raycast_kernel(const __grid_constant__ RenderArgs a, int strip) {
   __shared__ __align__(16) float s_tf[5 * VVLIC_TF_ENTRIES];
   load_tf(a, s_tf);
