@@ -44,3 +44,40 @@ def test_batch_images_and_totals(ctx, sizes, illum):
             np.testing.assert_array_equal(out.cpu().numpy(), ref)
         st = ctx.stats()
         assert (st.samples, st.rays, st.sample_steps) == tuple(totals)
+
+
+def test_batch_in_a_capture_is_refused(ctx):
+    """Jobs launched one by one on a stream the caller is capturing are an error that leaves the capture
+    as it was, and the next batch renders."""
+    import torch
+
+    size = 48
+
+    ctx.upload_noise(wl.dense_noise(16, seed=4))
+    vid = ctx.upload_field(wl.vortex_field(12, seed=1), storage="f16")
+    p = capi.params_default()
+    p.steps_backward = p.steps_forward = 4
+    table = capi.make_filter_table("cos2", 64)
+    outs = [torch.zeros(size, size, 4, device="cuda") for _ in range(2)]
+    jobs = [capi.make_job(vid, o.data_ptr(), size, size, wl.perspective_view(distance=2.0 + k), p, table)
+            for k, o in enumerate(outs)]
+    stream = torch.cuda.Stream()
+    ctx.batch_render(jobs, stream.cuda_stream)
+    stream.synchronize()
+    first = [o.cpu().numpy() for o in outs]
+    scratch = torch.zeros(4, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        graph.capture_begin(capture_error_mode="thread_local")
+        scratch.add_(1)
+        with pytest.raises(capi.VVLICError):
+            ctx.batch_render(jobs, stream.cuda_stream)
+        graph.capture_end()
+    for o in outs:
+        o.zero_()
+    torch.cuda.synchronize()
+    ctx.batch_render(jobs, torch.cuda.Stream().cuda_stream)
+    torch.cuda.synchronize()
+    for o, ref in zip(outs, first):
+        np.testing.assert_array_equal(o.cpu().numpy(), ref)

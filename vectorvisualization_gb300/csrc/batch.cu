@@ -203,6 +203,10 @@ vvlic_status batch_render(vvlic_ctx* c, const vvlic_job* jobs, int n, cudaStream
                                   start);
   if (st) return st;
   if (job_by_job(c, jobs, n)) {
+    // refused as the captured sequence below is: a stream that the caller is capturing
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+      return cuda_fail(c, cudaErrorStreamCaptureUnsupported, "batch on a stream that is being captured");
     if ((st = launch_jobs(c, n, storage, sampler, integ, grad, s))) return st;
     c->stats_pending = true;
     c->tape_flag_pending = false;

@@ -16,11 +16,10 @@
 namespace vvlic {
 
 constexpr int kTileW = 16, kTileH = 8;         // techniques.cuh: one CTA of 128 threads per tile
-constexpr int kWarpTileW = 8, kWarpTileH = 4;  // adjoint.cuh, batch.cuh: 32 pixels per warp
 constexpr int kThreads = 128, kWarps = kThreads / 32;
 
 // Registers: the ray-cast kernels are compiled for at most 65536 / (128 * VVLIC_MIN_BLOCKS) registers
-// per thread and launched in CTAs of up to kCastThreads threads.  Euler and Heun at 7 / 6 / 5, groups of
+// per thread and launched in CTAs of up to cast_threads() threads.  Euler and Heun at 7 / 6 / 5, groups of
 // four: 512^2 lit frame of 256^3 17.9 / 17.7 / 17.3 ms, 1024^2 61.1 / 60.9 / 62.7 ms, FP32 31.9 / 30.9 /
 // 30.0 ms, unlit 853x481 UNORM8 frame 2.90 / 2.79 / 2.78 ms.  RK4 (four slopes per step), 1024^2 frame
 // of the lit 512^3 orbit, at 6 / 5 / 4: 488 / 474 / 482 ms.

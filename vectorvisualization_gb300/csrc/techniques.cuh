@@ -188,27 +188,20 @@ __global__ void __launch_bounds__(kThreads) volume_kernel(const __grid_constant_
 
 // LIC intensity at every voxel centre of the LIC volume: lic3d_volume_fragment.glsl:2-21 with
 // pos = ((x+.5)/nx, (y+.5)/ny, (z+.5)/nz) * scaleVol (VolumeBuffer::drawSlice).  A warp takes a
-// tile of kLicvolTileW x kLicvolTileH voxels in x, y and kLicvolPairZ consecutive slices; with
-// two slices each thread computes both voxels' LIC together (compute_lic2: four independent
-// streamline chains, results bit-identical to compute_lic).  On the 512^3 turbulence field (RK4,
-// L = 60 each way) the 8x4 tiles took 202.7 ms against 217.9 ms for 32-voxel rows; two slices per
-// thread took 211.1 ms in rows and 203.3 ms in tiles, so one slice and 8x4 tiles are the default.
+// tile of kLicvolTileW x kLicvolTileH voxels in x, y.  On the 512^3 turbulence field (RK4, L = 60 each way)
+// the 8x4 tiles took 202.7 ms against 217.9 ms for 32-voxel rows, and two slices per thread 203.3 ms.
 #ifndef VVLIC_LICVOL_TILE
 #define VVLIC_LICVOL_TILE 1
-#endif
-#ifndef VVLIC_LICVOL_PAIR
-#define VVLIC_LICVOL_PAIR 0
 #endif
 #ifndef VVLIC_LICVOL_MIN_BLOCKS
 #define VVLIC_LICVOL_MIN_BLOCKS 1
 #endif
 constexpr int kLicvolTileW = VVLIC_LICVOL_TILE ? 8 : 32, kLicvolTileH = VVLIC_LICVOL_TILE ? 4 : 1;
-constexpr int kLicvolPairZ = VVLIC_LICVOL_PAIR ? 2 : 1;
 
 // warp work items of an nx*ny*nz LIC volume
 __host__ __device__ inline size_t licvol_items(const int ln[3]) {
   return (size_t)((ln[0] + kLicvolTileW - 1) / kLicvolTileW) * (size_t)((ln[1] + kLicvolTileH - 1) / kLicvolTileH) *
-         (size_t)((ln[2] + kLicvolPairZ - 1) / kLicvolPairZ);
+         (size_t)ln[2];
 }
 
 __device__ __forceinline__ float3 licvol_pos(const RenderArgs& a, const TechArgs& t, int x, int y, int z) {
@@ -227,21 +220,12 @@ __global__ void __launch_bounds__(kThreads, VVLIC_LICVOL_MIN_BLOCKS) licvolume_k
   for (size_t wi = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); wi < items; wi += stride) {
     const int x = (int)(wi % tx) * kLicvolTileW + lane % kLicvolTileW;
     const int y = (int)((wi / tx) % ty) * kLicvolTileH + lane / kLicvolTileW;
-    const int z = (int)(wi / ((size_t)tx * ty)) * kLicvolPairZ;
+    const int z = (int)(wi / ((size_t)tx * ty));
     if (x >= nx || y >= ny) continue;
     const size_t v = ((size_t)z * ny + y) * nx + x;
     const float3 p0 = licvol_pos(a, t, x, y, z);
     const float4 f0 = Field<ST, FL>::sample(a, p0);
-    if (kLicvolPairZ == 2 && z + 1 < nz) {
-      const float3 p1 = licvol_pos(a, t, x, y, z + 1);
-      const float4 f1 = Field<ST, FL>::sample(a, p1);
-      float4 i0, i1;
-      compute_lic2<ST, FL, NL, INTEG, false>(a, p0, f0, p1, f1, i0, i1);
-      t.licvol_out[v] = i0.w * a.intensity_scale;
-      t.licvol_out[v + (size_t)nx * ny] = i1.w * a.intensity_scale;
-    } else {
-      t.licvol_out[v] = compute_lic<ST, FL, NL, INTEG, false>(a, p0, f0).w * a.intensity_scale;
-    }
+    t.licvol_out[v] = compute_lic<ST, FL, NL, INTEG, false>(a, p0, f0).w * a.intensity_scale;
   }
 }
 

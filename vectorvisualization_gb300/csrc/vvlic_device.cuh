@@ -777,51 +777,6 @@ __device__ __forceinline__ float4 compute_lic(const RenderArgs& a, float3 pos, f
   return fold<GRAD>(acc);
 }
 
-// computeLIC of two samples at once (four independent gather chains per thread).  Each sample's
-// sums are formed in exactly the order compute_lic uses, so the results are bit-identical.
-template <int ST, int FL, int NL, int INTEG, bool GRAD>
-__device__ __forceinline__ void compute_lic2(const RenderArgs& a, float3 pa, float4 fa, float3 pc, float4 fc,
-                                             float4& out_a, float4& out_c) {
-  const int lb = a.lb, lf = a.lf;
-  const int both = min(lb, lf);
-  const float w0 = a.taps[lb];
-  float2 acca[4], accc[4], n[4];
-  noise_tap2<NL, GRAD>(a, pa, pc, n);
-#pragma unroll
-  for (int c = GRAD ? 0 : 3; c < 4; ++c) {
-    acca[c] = make_float2(n[c].x * w0, 0.f);
-    accc[c] = make_float2(n[c].y * w0, 0.f);
-  }
-  float3 p0 = pa, p1 = pa, p2 = pc, p3 = pc;
-  float4 s0 = fa, s1 = fa, s2 = fc, s3 = fc;
-  int i = 1;
-  for (; i <= both; ++i) {
-    p0 = lic_step<ST, FL, INTEG>(a, p0, s0, -1.0f);
-    p1 = lic_step<ST, FL, INTEG>(a, p1, s1, 1.0f);
-    p2 = lic_step<ST, FL, INTEG>(a, p2, s2, -1.0f);
-    p3 = lic_step<ST, FL, INTEG>(a, p3, s3, 1.0f);
-    const float2 w = make_float2(a.taps[lb - i], a.taps[lb + i]);
-    noise_tap2<NL, GRAD>(a, p0, p1, n);
-    accumulate2<GRAD>(acca, n, w);
-    noise_tap2<NL, GRAD>(a, p2, p3, n);
-    accumulate2<GRAD>(accc, n, w);
-  }
-  for (int j = i; j <= lb; ++j) {
-    p0 = lic_step<ST, FL, INTEG>(a, p0, s0, -1.0f);
-    p2 = lic_step<ST, FL, INTEG>(a, p2, s2, -1.0f);
-    accumulate_one<GRAD>(acca, false, noise_tap<NL, GRAD>(a, p0), a.taps[lb - j]);
-    accumulate_one<GRAD>(accc, false, noise_tap<NL, GRAD>(a, p2), a.taps[lb - j]);
-  }
-  for (int j = i; j <= lf; ++j) {
-    p1 = lic_step<ST, FL, INTEG>(a, p1, s1, 1.0f);
-    p3 = lic_step<ST, FL, INTEG>(a, p3, s3, 1.0f);
-    accumulate_one<GRAD>(acca, true, noise_tap<NL, GRAD>(a, p1), a.taps[lb + j]);
-    accumulate_one<GRAD>(accc, true, noise_tap<NL, GRAD>(a, p3), a.taps[lb + j]);
-  }
-  out_a = fold<GRAD>(acca);
-  out_c = fold<GRAD>(accc);
-}
-
 // ------------------------------------------------------------------------------------------
 // shading: illumLIC (inc_illum.glsl:158-172) and illumGradient (inc_illum.glsl:1-41)
 // ------------------------------------------------------------------------------------------
