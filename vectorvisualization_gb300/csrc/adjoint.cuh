@@ -364,7 +364,17 @@ __global__ void __launch_bounds__(kThreads, VVLIC_ADJ_MIN_BLOCKS)
     if (lane == 0) t = atomicAdd(next, 1u);
     t = __shfl_sync(0xffffffffu, t, 0);
     if (t >= ntiles) break;
-    const int px = (int)(t % tiles_x) * 2 + (r & 1), py = (int)(t / tiles_x) * 2 + (r >> 1);
+    unsigned tx = t % tiles_x, ty = t / tiles_x;
+    if (GRAD && INTEG == VVLIC_RK4) {
+      // up strips of 64 pixels, so that the rays in flight are a block of the image: one 600^2 lit RK4
+      // view of 320^3, forward and adjoint, 194.9 -> 170.5 ms, 1024^2 of 512^3 930 -> 891 (unlit +0.3 %)
+      constexpr unsigned strip = 32;
+      const unsigned tiles_y = (a.H + 1) / 2;
+      const unsigned col = t / (strip * tiles_y) * strip, rest = t - col * tiles_y, width = min(strip, tiles_x - col);
+      tx = col + rest % width;
+      ty = rest / width;
+    }
+    const int px = (int)tx * 2 + (r & 1), py = (int)ty * 2 + (r >> 1);
     float3 pos0 = f3(0.f, 0.f, 0.f), dir = f3(0.f, 0.f, 0.f);
     int n = 0;  // samples of this lane's ray
     float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
