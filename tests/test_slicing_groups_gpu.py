@@ -37,3 +37,35 @@ def test_slicing_queue_edges(ctx, oracle, planes, gate):
         assert float(np.sqrt(np.mean((img.astype(np.float64) - ref) ** 2))) <= 1e-3
         assert abs(int(ctx.stats().samples) - int(smp.sum())) <= 0.01 * smp.sum() + 2
         assert (gate == "none") == (smp.sum() == 0 and float(img.max()) == 0.0) or gate == "few"
+
+
+@pytest.mark.parametrize("integ", [capi.EULER, capi.HEUN, capi.RK4])
+@pytest.mark.parametrize("lit", [False, True])
+def test_slices_do_not_depend_on_the_grid(ctx, integ, lit):
+    """Groups of eight planes (small frames), of two (medium ones) and a lane per pixel (large ones) give a
+    pixel the same value and count, bit for bit: the corner of a larger frame is the smaller frame."""
+    import torch
+
+    vid = ctx.upload_field(wl.vortex_field(24, seed=3), storage="f16")
+    ctx.upload_noise(wl.dense_noise(20, seed=8), capi.NOISE_GRAD_CENTRAL if lit else capi.NOISE_SCALAR)
+    ctx.set_tf(*wl.random_tf(5))
+    p = capi.params_default()
+    p.technique, p.integrator, p.steps_backward, p.steps_forward = capi.TECHNIQUE["slicing"], integ, 3, 5
+    p.step_size_vol = 1.0 / 99.5  # 100 planes
+    p.illum = capi.ILLUM_GRADIENT if lit else capi.ILLUM_NONE
+    ctx.set_params(p)
+
+    def frame(w, h):
+        ctx.set_view(wl.ortho_view(center=(w / 2048, h / 2048, 0.0), right=(w / 2048, 0, 0), up=(0, h / 2048, 0)))
+        out = torch.zeros(h, w, 4, device="cuda")
+        smp = torch.zeros(h, w, dtype=torch.int32, device="cuda")
+        ctx.render_device(vid, out.data_ptr(), w, h, d_samples=smp.data_ptr())
+        torch.cuda.synchronize()
+        return out.cpu().numpy(), smp.cpu().numpy()
+
+    big, sbig = frame(1024, 1024)
+    assert sbig.max() > 8
+    for w, h in ((1, 1), (65, 57), (300, 258), (419, 418), (420, 421), (513, 509), (603, 604), (611, 605)):
+        img, smp = frame(w, h)
+        np.testing.assert_array_equal(smp, sbig[:h, :w])
+        np.testing.assert_array_equal(img, big[:h, :w])

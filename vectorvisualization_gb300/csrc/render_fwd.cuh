@@ -67,9 +67,9 @@ __device__ __forceinline__ void flush_counters(const RenderArgs& a, uint32_t sam
   }
 }
 
-// Pixels of a CTA: warps of (32 / S) rays, two wide and the rest on top of one another.
+// Rays of a warp: 32 / S as 2x1, 2x2, 4x2 or 4x4 pixels.
 template <int S> struct GroupTile {
-  static constexpr int w = 2, h = 16 / S;
+  static constexpr int w = S >= 8 ? 2 : 4, h = 32 / S / w;
 };
 struct CtaShape {
   int wx, wy;  // warps across and up
@@ -126,13 +126,13 @@ static cudaError_t launch_one(const RenderArgs& a, int num_sms, cudaStream_t str
   const int threads = cast_cta_threads<INTEG, GRAD>(a, num_sms);
   const int strip = INTEG == VVLIC_RK4 ? 16 : 0;
   const CtaShape cta = cta_shape(threads);
-  const auto grid = [&](int th) {
-    return dim3((unsigned)((a.W + 2 * cta.wx - 1) / (2 * cta.wx)), (unsigned)((a.H + th * cta.wy - 1) / (th * cta.wy)));
+  const auto grid = [&](int tw, int th) {
+    return dim3((unsigned)((a.W + tw * cta.wx - 1) / (tw * cta.wx)), (unsigned)((a.H + th * cta.wy - 1) / (th * cta.wy)));
   };
   if (2 * cast_tiles(a) <= resident_warps(num_sms))
-    raycast_kernel<ST, FL, NL, INTEG, GRAD, 16><<<grid(GroupTile<16>::h), threads, 0, stream>>>(a, strip);
+    raycast_kernel<ST, FL, NL, INTEG, GRAD, 16><<<grid(GroupTile<16>::w, GroupTile<16>::h), threads, 0, stream>>>(a, strip);
   else
-    raycast_kernel<ST, FL, NL, INTEG, GRAD, 8><<<grid(GroupTile<8>::h), threads, 0, stream>>>(a, strip);
+    raycast_kernel<ST, FL, NL, INTEG, GRAD, 8><<<grid(GroupTile<8>::w, GroupTile<8>::h), threads, 0, stream>>>(a, strip);
   return cudaGetLastError();
 }
 

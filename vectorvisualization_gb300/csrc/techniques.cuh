@@ -36,28 +36,26 @@ __device__ __forceinline__ float sample_licvol(const TechArgs& t, float3 s) {
   return lerpf(lerpf(c00, c10, ay), lerpf(c01, c11, ay), az);
 }
 
-// SLICING by a warp on 2x2 rays, eight lanes to a ray.  The lanes test eight planes of their ray at a time
-// (inside the slice polygon, TF alpha above 0.05) and queue those that pass; once every ray has eight
+// SLICING by a warp on 32 / S rays, S lanes to a ray.  The lanes test S planes of their ray at a time
+// (inside the slice polygon, TF alpha above 0.05) and queue those that pass; once every ray has S
 // or no planes left, each lane computes one queued plane's LIC and the ray's lanes composite them
 // in order.  So the streamline work, nearly all of the cost, runs in full groups however few planes
-// pass; a lane per pixel idled wherever its own plane did not (18.5 of 32 lanes active).  Planes, order,
+// pass; a lane per pixel idles wherever its own plane does not (18.5 of 32 lanes active).  Planes, order,
 // arithmetic and counts are those of one lane walking the planes; the ones after dest.a reaches 0.95
-// are dropped.  160^3 field, lit 800x600 frame 2.34 -> 1.92 ms, unlit 400x300 1.28 -> 0.55 ms, lit
-// 1400x1000 4.87 -> 4.83 ms (the texture unit's rate).
-constexpr int kSliceGroup = 8, kSliceRays = 32 / kSliceGroup;
-
-template <int ST, int FL, int NL, int INTEG, bool GRAD>
+// are dropped.  launch_tech_one has the rule and the times.
+template <int ST, int FL, int NL, int INTEG, bool GRAD, int S>
 __global__ void __launch_bounds__(cast_threads<INTEG>(), min_blocks<INTEG>() * 128 / cast_threads<INTEG>())
     slicing_kernel(const __grid_constant__ RenderArgs a, const __grid_constant__ TechArgs t) {
-  constexpr int S = kSliceGroup, R = kSliceRays;
+  constexpr int R = 32 / S;
   __shared__ __align__(16) float s_tf[5 * VVLIC_TF_ENTRIES];
   __shared__ int s_queue[cast_threads<INTEG>() / 32][R][2 * S];
   load_tf(a, s_tf);
   const CtaShape cta = cta_shape(blockDim.x);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k = lane / R, r = lane % R;
-  const int px = ((int)blockIdx.x * cta.wx + warp % cta.wx) * 2 + (r & 1);
-  const int py = ((int)blockIdx.y * cta.wy + warp / cta.wx) * 2 + (r >> 1);
-  const unsigned mine = 0x11111111u << r;
+  using T = GroupTile<S>;
+  const int px = ((int)blockIdx.x * cta.wx + warp % cta.wx) * T::w + r % T::w;
+  const int py = ((int)blockIdx.y * cta.wy + warp / cta.wx) * T::h + r / T::w;
+  const unsigned mine = ray_lanes(S) << r;
   int* queue = s_queue[warp][r];
   const bool ray = px < a.W && py < a.H;
   float o[3] = {0.f, 0.f, 0.f}, d[3] = {0.f, 0.f, 0.f}, tn = 0.0f, tf = 0.0f;
@@ -125,6 +123,54 @@ __global__ void __launch_bounds__(cast_threads<INTEG>(), min_blocks<INTEG>() * 1
   const bool store = ray && lane < R;
   if (store) store_pixel(a, px, py, dest, samples);
   flush_counters(a, store ? samples : 0u, store && hit ? 1u : 0u);
+}
+
+// SLICING by one lane per pixel: a warp stays on one plane, whose neighbouring pixels read neighbouring texels.
+template <int ST, int FL, int NL, int INTEG, bool GRAD>
+__device__ __forceinline__ float4 slice_pixel(const RenderArgs& a, const TechArgs& t, const float* s_tf, int px,
+                                              int py, uint32_t& samples, uint32_t& hit) {
+  float4 dest = make_float4(0.f, 0.f, 0.f, 0.f);
+  samples = 0;
+  hit = 0;
+  float o[3], d[3], tn, tf;
+  if (!ray_interval(a, px, py, o, d, tn, tf)) return dest;
+  hit = 1;
+  const float3 O = f3(o[0], o[1], o[2]), D = f3(d[0], d[1], d[2]);
+  const float3 V = f3(t.v[0], t.v[1], t.v[2]), C = f3(t.c[0], t.c[1], t.c[2]);
+  const float vd = dot3(V, D);
+  if (vd == 0.0f) return dest;  // ray parallel to the planes
+  const float voc = dot3(V, sub3(O, C));
+  const float3 sv = f3(a.scale_vol[0], a.scale_vol[1], a.scale_vol[2]);
+  const float3 dir = mul3(norm3(D), sv);
+  const float step = t.depth / (float)t.nslices;
+  for (int i = 0; i < t.nslices; ++i) {
+    if (dest.w >= 0.95f) break;  // lic3d_slicing_fragment.glsl:14 (no later slice changes dest)
+    const float di = -0.5f * t.depth + ((float)i + 0.5f) * step;
+    const float ti = (di - voc) / vd;
+    if (!(ti >= tn && ti <= tf)) continue;  // outside the slice polygon (plane inside the box)
+    const float3 pos = mul3(add3(O, scl3(D, ti)), sv);
+    const float4 f = Field<ST, FL>::sample(a, pos);
+    const float4 tfv = tf_rgba(s_tf, f.w);
+    if (!(tfv.w > 0.05f)) continue;
+    float4 il = compute_lic<ST, FL, NL, INTEG, GRAD>(a, pos, f);
+    ++samples;
+    il.w *= a.intensity_scale;
+    dest = blend(dest, shade<GRAD>(a, s_tf, il, tfv, pos, dir, f));
+  }
+  return dest;
+}
+
+template <int ST, int FL, int NL, int INTEG, bool GRAD>
+__global__ void __launch_bounds__(kThreads, VVLIC_MIN_BLOCKS)
+    slicing_pixel_kernel(const __grid_constant__ RenderArgs a, const __grid_constant__ TechArgs t) {
+  __shared__ __align__(16) float s_tf[5 * VVLIC_TF_ENTRIES];
+  load_tf(a, s_tf);
+  const int px = blockIdx.x * kTileW + (threadIdx.x % kTileW);
+  const int py = blockIdx.y * kTileH + (threadIdx.x / kTileW);
+  uint32_t samples = 0, hit = 0;
+  if (px < a.W && py < a.H)
+    store_pixel(a, px, py, slice_pixel<ST, FL, NL, INTEG, GRAD>(a, t, s_tf, px, py, samples, hit), samples);
+  flush_counters(a, samples, hit);
 }
 
 // VOLUME / LICVOLUME for one pixel.  LICVOLUME keeps four samples' fetches in flight (a texture fetch and
@@ -212,7 +258,7 @@ __device__ __forceinline__ float3 licvol_pos(const RenderArgs& a, const TechArgs
 template <int ST, int FL, int NL, int INTEG>
 __global__ void __launch_bounds__(kThreads, VVLIC_LICVOL_MIN_BLOCKS) licvolume_kernel(const __grid_constant__ RenderArgs a,
                                                                                       const __grid_constant__ TechArgs t) {
-  const int nx = t.ln[0], ny = t.ln[1], nz = t.ln[2];
+  const int nx = t.ln[0], ny = t.ln[1];
   const int tx = (nx + kLicvolTileW - 1) / kLicvolTileW, ty = (ny + kLicvolTileH - 1) / kLicvolTileH;
   const size_t items = licvol_items(t.ln);
   const int lane = threadIdx.x & 31;
@@ -237,10 +283,30 @@ static cudaError_t launch_tech_one(const RenderArgs& a, const TechArgs& t, int n
     licvolume_kernel<ST, FL, NL, INTEG><<<std::max(1, blocks), kThreads, 0, s>>>(a, t);
     return cudaGetLastError();
   }
+  // Slicing frames by W*H pixels on a chip that holds `warps` warps:
+  //   fewer than 1.5 pixels per resident lane: groups of eight planes;
+  //   more pixels than planes * warps: a lane per pixel.  Its tail, a chain of all planes, is then
+  //     short against the whole, and lanes on one plane share more texels than lanes on several;
+  //   groups of two planes between.
+  // FP16, ms by eight / two / lane per pixel: 800x600 lit, 160^3 1.92 / 1.92 / 2.13; Heun, a plane per texel,
+  // 600^2 1.24 / 1.08 / 1.52, 1024^2 3.18 / 2.53 / 2.69, 1600^2 7.26 / 5.52 / 5.36; RK4, 2.5 texels, 300^2
+  // 0.40 / 0.43 / 1.10, 600^2 1.08 / 0.89 / 1.06, 1200^2 3.47 / 2.66 / 2.33; 3.3 texels 300^2 0.22 / 0.23 / 0.39,
+  // 600^2 0.57 / 0.43 / 0.43, 900^2 1.14 / 0.82 / 0.66.
+  const long long pixels = (long long)a.W * a.H, warps = resident_warps(num_sms);
+  if (pixels >= 48 * warps && pixels >= t.nslices * warps) {
+    const dim3 tiles((a.W + kTileW - 1) / kTileW, (a.H + kTileH - 1) / kTileH);
+    slicing_pixel_kernel<ST, FL, NL, INTEG, GRAD><<<tiles, kThreads, 0, s>>>(a, t);
+    return cudaGetLastError();
+  }
   const int threads = cast_cta_threads<INTEG, GRAD>(a, num_sms);
   const CtaShape cta = cta_shape(threads);
-  const dim3 grid((unsigned)((a.W + 2 * cta.wx - 1) / (2 * cta.wx)), (unsigned)((a.H + 2 * cta.wy - 1) / (2 * cta.wy)));
-  slicing_kernel<ST, FL, NL, INTEG, GRAD><<<grid, threads, 0, s>>>(a, t);
+  const auto grid = [&](int tw, int th) {
+    return dim3((unsigned)((a.W + tw * cta.wx - 1) / (tw * cta.wx)), (unsigned)((a.H + th * cta.wy - 1) / (th * cta.wy)));
+  };
+  if (pixels < 48 * warps)
+    slicing_kernel<ST, FL, NL, INTEG, GRAD, 8><<<grid(GroupTile<8>::w, GroupTile<8>::h), threads, 0, s>>>(a, t);
+  else
+    slicing_kernel<ST, FL, NL, INTEG, GRAD, 2><<<grid(GroupTile<2>::w, GroupTile<2>::h), threads, 0, s>>>(a, t);
   return cudaGetLastError();
 }
 

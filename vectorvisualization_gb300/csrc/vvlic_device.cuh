@@ -1020,13 +1020,19 @@ __device__ __forceinline__ float3 march(float3 p, float3 dir, float step) {
 // warp, each as long as its longest ray), keeps lanes together when rays end at different samples,
 // and lets the lanes of a warp read overlapping streamlines: a sample's noise cells are mostly its
 // neighbour's.  `ray` is false for lanes without a pixel.  Every lane of the warp calls.
+// Lanes 0, 32/S, 2 * 32/S, ... of a warp: those of its first ray.
+__host__ __device__ constexpr unsigned ray_lanes(int S) {
+  unsigned m = 0;
+  for (int j = 0; j < S; ++j) m |= 1u << (j * (32 / S));
+  return m;
+}
+
 template <int ST, int FL, int NL, int INTEG, bool GRAD, int S>
 __device__ __forceinline__ float4 trace_group(const RenderArgs& a, const float* s_tf, bool ray, int px, int py,
                                               uint32_t& samples, uint32_t& hit) {
   constexpr int R = 32 / S;
   const int lane = threadIdx.x & 31, k = lane / R, r = lane % R;
-  static_assert(S == 4 || S == 8 || S == 16, "samples per group");
-  const unsigned mine = (S == 4 ? 0x01010101u : (S == 8 ? 0x11111111u : 0x55555555u)) << r;  // this ray's lanes
+  const unsigned mine = ray_lanes(S) << r;
   float4 dest = make_float4(0.f, 0.f, 0.f, 0.f);
   float3 pos = f3(0.f, 0.f, 0.f), dir = pos;
   samples = 0;
