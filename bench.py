@@ -55,8 +55,8 @@ def parse():
     ap.add_argument("--impl", choices=["ours", "reference"], default="ours")
     ap.add_argument("--sampler", default="hybrid", choices=["gather", "cell", "texture", "hybrid"])
     ap.add_argument("--schedule", default="auto", choices=["auto", "queue", "static"],
-                    help="auto: the schedule measured faster per workload (static for the orbit frames, "
-                         "queue for the others)")
+                    help="passed on to the library, which runs the same raster grid for both (BRICK frames "
+                         "excepted); auto: static for the orbit frames, queue for the others")
     ap.add_argument("--size", type=int, default=512, help="orbit field size per axis")
     ap.add_argument("--image", type=int, default=2048, help="orbit image size")
     ap.add_argument("--c2-size", type=int, default=256)
@@ -77,10 +77,8 @@ def parse():
 
 
 def schedule(args, workload: str) -> str:
-    """The work distribution of a section.  Measured on one GB300 (ms per frame): the orbit's
-    2048^2 RK4 frames run about 3 % faster on the static raster grid (1230 / 1419 / 1491 against
-    1268 / 1455 / 1540 for frames 0 / 16 / 40), the lit 1024^2 Heun frame about 3 % faster on
-    the longest-first queue; `auto` takes the faster per workload."""
+    """The schedule a section passes to the library.  Ray-casts run the same raster grid of sample
+    groups under either name; only the BRICK sampler tells them apart."""
     if args.schedule != "auto":
         return args.schedule
     return "static" if workload == "orbit" else "queue"
@@ -476,8 +474,7 @@ def bench_c4(ctx, torch, stream, flush, args):
 def bench_batch(ctx, torch, stream, flush, args, dist):
     """C3: 64 volumes with per-axis dims from {64, 80, ..., 192} (ABC or vortex, own seeds), 1-8
     random views each at 512^2, filters mixed box / triangle / cos^2, L in [15, 60], FP16
-    storage, Heun; one persistent launch per batch, replayed from a CUDA graph.  Under N ranks
-    every rank renders its cost-balanced share of the jobs (replicas, no exchange)."""
+    storage, Heun; the jobs launched one by one over eight streams.  Under N ranks every rank renders its cost-balanced share of the jobs (replicas, no exchange)."""
     from vectorvisualization_gb300 import capi, workloads as wl
     from vectorvisualization_gb300.replicas import shard_by_cost
 
@@ -507,7 +504,7 @@ def bench_batch(ctx, torch, stream, flush, args, dist):
     voxels = sum(int(np.prod(bv.field.shape[:3])) for bv in vols if id(bv) in vids)
     sh = stream.cuda_stream
     tw, smp, tune_ms = ctx.batch_autotune(jobs, sh)
-    ctx.batch_render(jobs, sh)  # capture with the tuned shape
+    ctx.batch_render(jobs, sh)  # the tuned sampler's layouts
     stream.synchronize()
     dist.barrier()
     ms = min(timed(torch, stream, flush, lambda: ctx.batch_render(jobs, sh)) for _ in range(2))
@@ -523,9 +520,9 @@ def bench_batch(ctx, torch, stream, flush, args, dist):
         "sample_steps": int(steps_all), "sharding": f"shard_by_cost over {dist.world} rank(s)",
         "autotune": {"tile": f"{tw}x{32 // tw}", "sampler": [k for k, v in capi.SAMPLER.items() if v == smp][0],
                      "best_ms": tune_ms},
-        "cuda_graph": True, "generation_s": gen_s,
+        "cuda_graph": False, "generation_s": gen_s,
     }
-    # the plain FP32 form: the same jobs from FP32 texels with the gather sampler, one launch
+    # the plain FP32 form: the same jobs from FP32 texels with the gather sampler
     with capi.Context(torch.cuda.current_device()) as pctx:
         pctx.upload_noise(noise)
         pctx.set_tf(*wl.default_tf())
@@ -654,22 +651,18 @@ def bench_rows(ctx, torch, stream, flush, w, vid, ceiling, frame, args):
     ms = min(timed(torch, stream, flush, upd) for _ in range(3))
     vox = nx * ny * nz
     vbytes = ctx.volume_bytes(vid)
-    texels = vox * bytes_per_texel(w.storage)
-    # two passes over the float32 field, every layout of the volume written once, the texels read
-    # once more to build the derived layouts
-    alg = vox * 24 + vbytes + (texels if vbytes > texels else 0)
+    # two passes over the float32 field, every layout of the volume written once
+    alg = vox * 24 + vbytes
     res["field_update_device"] = {
         "ms": ms, "voxels": vox, "volume_bytes": vbytes,
         "roofline": {"bound": "hbm", "unit": "GB/s", "achieved": alg / (ms / 1e3) / 1e9, "peak": peak_hbm,
                      "frac": alg / (ms / 1e3) / 1e9 / peak_hbm, "peak_kind": hbm_kind, "traffic": None,
                      "algorithmic_bytes": alg,
                      "bytes": "24 B per voxel read (the length pass and the encode pass over float32 xyz) + "
-                              "the volume's layouts written (texels, texture copy, cells if any) + the "
-                              "texels read once to build the derived layouts"}}
+                              "the volume's layouts written (texels, texture copy)"}}
     del d_xyz
 
-    # noise gradients: 4 calls per timed region, the first untimed, so that the stream-ordered
-    # scratch of calls 2-4 comes from the pool's free list
+    # noise gradients: 4 calls per timed region, the first untimed
     mz, my, mx = w.noise.shape
     d_noise = torch.from_numpy(np.ascontiguousarray(w.noise)).cuda()
     d_rgba = torch.empty(mx * my * mz * 4, dtype=torch.uint8, device="cuda")
@@ -688,15 +681,14 @@ def bench_rows(ctx, torch, stream, flush, w, vid, ceiling, frame, args):
         torch.cuda.synchronize()
         best = min(best, e0.elapsed_time(e1) / 3)
     nvox = mx * my * mz
-    alg = nvox * 30  # raw pass: 1 B read, 12 B written; filter pass: 12 B + 1 B read, 4 B written
+    alg = nvox * 5  # one pass: 1 B read, 4 B written
     res["noise_gradients"] = {
         "ms": best, "voxels": nvox,
         "roofline": {"bound": "hbm", "unit": "GB/s", "achieved": alg / (best / 1e3) / 1e9, "peak": peak_hbm,
                      "frac": alg / (best / 1e3) / 1e9 / peak_hbm, "peak_kind": hbm_kind, "traffic": None,
                      "algorithmic_bytes": alg,
-                     "bytes": "30 B per voxel: the raw-gradient pass reads the noise byte (its 27-voxel "
-                              "stencil from L1) and writes 12 B; the filter pass reads 12 B (27-voxel "
-                              "stencil from L1) and the noise byte and writes 4 B RGBA"}}
+                     "bytes": "5 B per voxel: the noise byte read, 4 B RGBA written (raw gradients stay in "
+                              "shared memory; the FP32 pipe is the bound)"}}
     del d_noise, d_rgba
     return res
 
@@ -826,8 +818,7 @@ def headline(args, dist, torch, stream, flush, ceiling) -> dict:
         "wall_ms_per_step": t_wall / args.steps * 1e3,
         "image_alpha_mean": float(out[..., 3].mean()),
         "roofline": roof,
-        # per frame: the ray-cast (+ the queue schedule's tile order: cost, bucket scan, scatter)
-        "gpu_launches": args.steps * (4 if schedule(args, "orbit") == "queue" else 1),
+        "gpu_launches": args.steps,  # per frame: the ray-cast
         "clocks": clk,
     }
     del total_samples
