@@ -1,7 +1,7 @@
 """The adjoint's ray groups (eight samples of four rays in a warp) and block-wise tap sums at the
 sizes where they can go wrong: rays that end inside a chunk of eight and a segment of 32, images that
 leave partial 2x2-ray tiles, and streamline lengths around the 16 steps of a sum block, even and
-uneven, for every integrator, against the FP64 adjoint.  Exact sampler and a frame inside (0, 1), away
+uneven, images one tile past a strip of 64 pixels and past two, for every integrator, against the FP64 adjoint.  Exact sampler and a frame inside (0, 1), away
 from the blend's clamp where an FP32 and an FP64 state may take different branches; the tolerances are
 those of the adjoint parity tests (2e-3 of the largest gradient, 1e-2 lit)."""
 import numpy as np
@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("integ", [capi.EULER, capi.HEUN, capi.RK4])
 @pytest.mark.parametrize("lit", [False, True])
 @pytest.mark.parametrize("lb,lf,bound,w,h", [(1, 0, 1, 5, 3), (15, 16, 3, 7, 6), (16, 15, 4, 6, 5), (17, 33, 5, 5, 4),
-                                             (0, 20, 6, 3, 3), (31, 32, 7, 4, 2)])
+                                             (0, 20, 6, 3, 3), (31, 32, 7, 4, 2), (2, 3, 2, 65, 3), (3, 2, 2, 131, 2)])
 def test_adjoint_at_chunk_and_block_edges(ctx, oracle, integ, lit, lb, lf, bound, w, h):
     import torch
 

@@ -108,6 +108,10 @@ __global__ void __launch_bounds__(cast_threads<INTEG>(), cast_min_ctas<ST, INTEG
 //     85 us against 125;
 //   up to twice as many: 64-thread CTAs, which spread over the SMs more evenly (128^2 preview 189 us
 //     against 203 in 128 threads and 234 in 256);
+//   from 8 times as many, lit Euler and Heun kernels of the narrower texels: four samples of 4x2 rays,
+//     which stay closer together where samples are further apart than pixels: 3.3 texels between samples, 600^2
+//     5.01 -> 4.83 ms, 1200^2 16.8 -> 16.2; one texel, 1024^2 57.46 -> 57.44.  (FP32 27.2 -> 28.5, RK4
+//     446 -> 465; unlit 14.0 -> 13.6 with coarse samples, but 853x481 UNORM8 2.68 -> 2.79.)
 //   from 16 times as many, lit Euler and Heun kernels: 256-thread CTAs, whose 4x8 rays share more noise
 //     cells in L1 (FP32 512^2 lit frame 27.3 ms against 29.1; FP16 1024^2 57.7 against 58.9); the unlit ones
 //     read a quarter of the cell bytes and lose 1 % by it;
@@ -129,6 +133,12 @@ static cudaError_t launch_one(const RenderArgs& a, int num_sms, cudaStream_t str
   const auto grid = [&](int tw, int th) {
     return dim3((unsigned)((a.W + tw * cta.wx - 1) / (tw * cta.wx)), (unsigned)((a.H + th * cta.wy - 1) / (th * cta.wy)));
   };
+  if constexpr (GRAD && ST != VVLIC_STORAGE_F32 && INTEG != VVLIC_RK4) {
+    if (cast_tiles(a) >= 8 * resident_warps(num_sms)) {
+      raycast_kernel<ST, FL, NL, INTEG, GRAD, 4><<<grid(GroupTile<4>::w, GroupTile<4>::h), threads, 0, stream>>>(a, strip);
+      return cudaGetLastError();
+    }
+  }
   if (2 * cast_tiles(a) <= resident_warps(num_sms))
     raycast_kernel<ST, FL, NL, INTEG, GRAD, 16><<<grid(GroupTile<16>::w, GroupTile<16>::h), threads, 0, stream>>>(a, strip);
   else
