@@ -1,0 +1,78 @@
+// Wrap form of the noise cells (NoiseCells in vvlic_device.cuh) and the rule that chooses it per
+// launch.  Plain C++, so that a host compiler can test the rule.
+#pragma once
+
+#include <cmath>
+
+#ifdef __CUDACC__
+#define VVLIC_HOST_DEVICE __host__ __device__
+#else
+#define VVLIC_HOST_DEVICE
+#endif
+
+namespace vvlic {
+
+// How a noise cell's index wraps (REPEAT), chosen on the host per launch (choose_noise_wrap):
+//   kWrapMask  every extent a power of two: a mask;
+//   kWrapMul   other extents: a multiply-high by a host-computed reciprocal;
+//   kWrapFar   positions whose noise coordinate may exceed +-2^19 (or an extent of 1 beside odd
+//              ones): floor, conversion and integer remainder.
+// The first two take floor(u) from the rounding of one addition: u + 1.5 * 2^23 rounded down holds
+// floor(u) in its low mantissa bits (exact for |u| < 2^22).  FRND and F2I, the direct forms, issue
+// at an eighth of the FADD rate (15 against 118 lanes per SM clock, three of each per tap).
+enum NoiseWrap : int { kWrapFar = 0, kWrapMask = 1, kWrapMul = 2 };
+constexpr float kFloorMagic = 12582912.0f;    // 1.5 * 2^23
+constexpr unsigned kFloorBits = 0x4B400000u;  // its bit pattern
+constexpr int kWrapReach = 1 << 19;           // |noise coordinate| bound of kWrapMask / kWrapMul
+
+// Wrap constants of an extent m: `clamp` is the coordinate a NaN position reads, congruent
+// to -2^24 modulo m (the lower clamp of the general form) and below every finite coordinate;
+// `off` a multiple of m that makes indices non-negative; `mul` = floor(2^32 / m) + 1, whose quotient
+// is exact for indices below 2^21 (2^21 * 2048 <= 2^32).
+VVLIC_HOST_DEVICE inline void noise_wrap_constants(int m, float* clamp, unsigned* mul, unsigned* off) {
+  const int r = (1 << 24) % m;
+  *clamp = -(float)(((kWrapReach - r) / m) * m + r);
+  *off = (unsigned)(((kWrapReach + m - 1) / m) * m);
+  *mul = m > 1 ? (unsigned)(0x100000000ull / (unsigned)m) + 1u : 0u;
+}
+
+// The larger of the two; NaN if either is.
+inline double larger(double a, double b) { return b > a || b != b ? b : a; }
+
+// Largest |position| a streamline of a ray starts at: inside the box its ray marches through,
+// [0, max(extent * scale_vol, tex_max)] per axis.
+inline double ray_start_bound(const float ext[3], const float scale_vol[3], const float tex_max[3]) {
+  double start = 0.0;
+  for (int i = 0; i < 3; ++i) {
+    const double sv = std::fabs((double)scale_vol[i]);
+    start = larger(start, larger(larger((double)ext[i] * sv, sv), (double)tex_max[i]));
+  }
+  return start;
+}
+
+// The same for the voxel centres of a LIC volume, (0, 1) * scale_vol.
+inline double voxel_start_bound(const float scale_vol[3]) {
+  double start = 0.0;
+  for (int i = 0; i < 3; ++i) start = larger(start, std::fabs((double)scale_vol[i]));
+  return start;
+}
+
+// The form for streamlines that start within `start` of the origin and move by at most `reach` along
+// an axis, under noise texel scales `nscale` (value taps) and `nscale_grad` (gradient taps) and noise
+// extents m: |noise coordinate| is bounded by (start + reach) * scale, with a margin for the
+// rounding of the positions.  NaN positions read the clamp.
+inline int choose_noise_wrap(double start, double reach, const float nscale[3], const float nscale_grad[3],
+                             const int m[3]) {
+  double scale = 0.0;
+  bool mask = true, one = false;
+  for (int i = 0; i < 3; ++i) {
+    scale = larger(scale, larger(std::fabs((double)nscale[i]), std::fabs((double)nscale_grad[i])));
+    mask = mask && (m[i] & (m[i] - 1)) == 0;
+    one = one || m[i] == 1;
+  }
+  const double bound = 1.01 * (start + reach) * scale + 1.0;
+  if (!(bound < (double)(kWrapReach - 4096))) return kWrapFar;  // also for NaN
+  return mask ? kWrapMask : (one ? kWrapFar : kWrapMul);
+}
+
+}  // namespace vvlic

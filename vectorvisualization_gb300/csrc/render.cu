@@ -144,24 +144,12 @@ vvlic_status refresh_noise_layouts(vvlic_ctx* c, NoiseTex& n, cudaStream_t s) {
   return VVLIC_OK;
 }
 
-// Wrap form and constants of the noise cells (NoiseWrap).  A streamline starts inside the box
-// its ray marches through, [0, max(extent * scaleVol, tex_max)] per axis (LIC-volume voxels: scaleVol),
-// and moves at most h_eff per step along an axis (encoded directions lie in [0, 1], magnitudes too), so
-// |noise coordinate| is bounded by (start + reach) * scale; NaN positions read the clamp.
-static void set_noise_wrap(const Geometry& g, double reach, RenderArgs& a) {
-  double start = 0.0, scale = 0.0;
-  bool mask = true, odd1 = false;
-  for (int i = 0; i < 3; ++i) {
-    const double sv = std::fabs((double)a.scale_vol[i]);
-    start = std::max(start, std::max(std::max((double)g.extent[i] * sv, sv), (double)a.tex_max[i]));
-    scale = std::max(scale, std::max(std::fabs((double)a.nscale[i]), std::fabs((double)a.nscale_grad[i])));
-    mask = mask && (a.m[i] & (a.m[i] - 1)) == 0;
-    odd1 = odd1 || a.m[i] == 1;
-    noise_wrap_constants(a.m[i], &a.nclamp[i], &a.nwrap_mul[i], &a.nwrap_off[i]);
-  }
-  const double bound = 1.01 * (start + reach) * scale + 1.0;
-  const bool near = bound < (double)(kWrapReach - 4096);  // false for NaN and infinite bounds
-  a.noise_wrap = !near ? kWrapFar : (mask ? kWrapMask : (odd1 ? kWrapFar : kWrapMul));
+// Wrap form and constants of the noise cells for streamlines that start within `start` of the origin.
+// They move at most h_eff per step along an axis (encoded directions lie in [-1, 1], magnitudes in
+// [0, 1]).
+static void set_noise_wrap(double start, RenderArgs& a) {
+  a.noise_wrap = choose_noise_wrap(start, std::max(a.lb, a.lf) * std::fabs((double)a.h_eff), a.nscale, a.nscale_grad, a.m);
+  for (int i = 0; i < 3; ++i) noise_wrap_constants(a.m[i], &a.nclamp[i], &a.nwrap_mul[i], &a.nwrap_off[i]);
 }
 
 // Fill the kernel argument block for one volume and image size.
@@ -254,7 +242,6 @@ vvlic_status build_render_args_ex(vvlic_ctx* c, Volume& v, int W, int H, cudaStr
     a.nscale[i] = (float)((double)a.freq_scale * a.m[i]);
     a.nscale_grad[i] = nofreq ? (float)a.m[i] : a.nscale[i];
   }
-  set_noise_wrap(v.geom, std::max(lb, lf) * std::fabs((double)h * p.eye_dist_factor), a);
   a.alpha_corr = p.low_res ? 2.0f * p.step_size_vol * 128.0f : p.step_size_vol * 128.0f;
   a.h_eff = h * p.eye_dist_factor;
   a.intensity_scale = inv_area / (float)(lf + lb) * p.gradient_scale;  // licKernel.b * gradient.r
@@ -265,6 +252,7 @@ vvlic_status build_render_args_ex(vvlic_ctx* c, Volume& v, int W, int H, cudaStr
   a.num_iter = p.num_iterations;
   a.lb = lb;
   a.lf = lf;
+  set_noise_wrap(ray_start_bound(a.ext, a.scale_vol, a.tex_max), a);
   a.illum = p.illum;
   a.tf_index = p.tf_index;
   a.sof = p.speed_of_flow;
@@ -627,6 +615,7 @@ extern "C" vvlic_status vvlic_compute_lic_volume(vvlic_ctx* c, int32_t vol_id, i
   // lic3d_volume_fragment.glsl composes inc_lic without inc_illum: the uniform scaleVol is the
   // volume's scale whatever the shading variant
   for (int i = 0; i < 3; ++i) a.scale_vol[i] = v.geom.scale[i];
+  set_noise_wrap(voxel_start_bound(a.scale_vol), a);  // streamlines start at voxels, not on rays
   cudaError_t e = cudaMemsetAsync(c->d_counters, 0, 4 * sizeof(unsigned long long), s);
   if (e == cudaSuccess) e = cudaEventRecord(c->ev0, s);
   if (e == cudaSuccess) e = launch_technique(v.storage, a, t, c->params.sampler, c->params.integrator, false, c->num_sms, s);

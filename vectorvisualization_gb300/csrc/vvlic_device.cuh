@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include "../../include/vvlic.h"
+#include "noise_wrap.hpp"
 
 namespace vvlic {
 
@@ -412,30 +413,6 @@ __host__ __device__ __forceinline__ size_t noise_cell_index(int x, int y, int z,
   return (size_t)(((unsigned)z * (unsigned)m[1] + (unsigned)y) * (unsigned)m[0] + (unsigned)x);
 }
 __host__ __device__ __forceinline__ size_t noise_cell_count(const int m[3]) { return (size_t)m[0] * m[1] * m[2]; }
-
-// How a noise cell's index wraps (REPEAT), chosen on the host per render (set_noise_wrap):
-//   kWrapMask  every extent a power of two: a mask;
-//   kWrapMul   other extents: a multiply-high by a host-computed reciprocal;
-//   kWrapFar   positions whose noise coordinate may exceed +-2^19 (or an extent of 1 beside odd
-//              ones): floor, conversion and integer remainder.
-// The first two take floor(u) from the rounding of one addition: u + 1.5 * 2^23 rounded down holds
-// floor(u) in its low mantissa bits (exact for |u| < 2^22).  FRND and F2I, the direct forms, issue
-// at an eighth of the FADD rate (15 against 118 lanes per SM clock, three of each per tap).
-enum NoiseWrap : int { kWrapFar = 0, kWrapMask = 1, kWrapMul = 2 };
-constexpr float kFloorMagic = 12582912.0f;  // 1.5 * 2^23
-constexpr unsigned kFloorBits = 0x4B400000u;  // its bit pattern
-constexpr int kWrapReach = 1 << 19;           // |noise coordinate| bound of kWrapMask / kWrapMul
-
-// Wrap constants of an extent m: `clamp` is the coordinate a NaN position reads, congruent
-// to -2^24 modulo m (the lower clamp of the general form) and below every finite coordinate;
-// `off` a multiple of m that makes indices non-negative; `mul` = floor(2^32 / m) + 1, whose quotient
-// is exact for indices below 2^21 (2^21 * 2048 <= 2^32).
-__host__ __device__ inline void noise_wrap_constants(int m, float* clamp, unsigned* mul, unsigned* off) {
-  const int r = (1 << 24) % m;
-  *clamp = -(float)(((kWrapReach - r) / m) * m + r);
-  *off = (unsigned)(((kWrapReach + m - 1) / m) * m);
-  *mul = m > 1 ? (unsigned)(0x100000000ull / (unsigned)m) + 1u : 0u;
-}
 
 // The general form, off the fast paths' register allocation: cell index and upper weight.
 static __device__ __noinline__ uint2 wrap_far(float u, int m) {
