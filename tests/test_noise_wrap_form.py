@@ -19,7 +19,9 @@ FAR, MASK, MUL = 0, 1, 2
 SOURCE = """
 #include "noise_wrap.hpp"
 extern "C" {
-double ray_start(const float* e, const float* s, const float* t) { return vvlic::ray_start_bound(e, s, t); }
+double ray_start(const float* e, const float* s, const float* t, double origin, double dir) {
+  return vvlic::ray_start_bound(e, s, t, origin, dir);
+}
 double voxel_start(const float* s) { return vvlic::voxel_start_bound(s); }
 int form(double start, double reach, const float* n, const float* g, const int* m) {
   return vvlic::choose_noise_wrap(start, reach, n, g, m);
@@ -41,6 +43,7 @@ def wrap(tmp_path_factory):
     assert r.returncode == 0, r.stderr
     lib = C.CDLL(str(d / "w.so"))
     lib.ray_start.restype = lib.voxel_start.restype = C.c_double
+    lib.ray_start.argtypes = [C.c_void_p] * 3 + [C.c_double] * 2
     lib.form.argtypes = [C.c_double, C.c_double] + [C.c_void_p] * 3
     return lib
 
@@ -71,7 +74,7 @@ def test_lic_volume_of_a_thin_lit_volume_takes_the_general_form(wrap, n, sd, m, 
     assert form_of(wrap, wrap.voxel_start(f3(*scale)), 0.3, freq, m) == FAR
     # the rays of its lit frames stay near: their scaleVol is the inverse scale
     tex = [a * b for a, b in zip(ext, scale)]
-    assert form_of(wrap, wrap.ray_start(f3(*ext), f3(*inv), f3(*tex)), 0.3, freq, m) == MUL
+    assert form_of(wrap, wrap.ray_start(f3(*ext), f3(*inv), f3(*tex), 2.0, 0.0), 0.3, freq, m) == MUL
 
 
 def test_line_between_the_forms(wrap):
@@ -86,8 +89,71 @@ def test_line_between_the_forms(wrap):
         assert form_of(wrap, bad, 0.0, 1.0, (64, 64, 64)) == FAR
         assert form_of(wrap, 0.0, bad, 1.0, (64, 64, 64)) == FAR
         assert form_of(wrap, wrap.voxel_start(f3(1.0, bad, 1.0)), 0.0, 1.0, (64, 64, 64)) == FAR
-        assert form_of(wrap, wrap.ray_start(f3(1, 1, 1), f3(1, 1, 1), f3(1, bad, 1)), 0.0, 1.0, (64, 64, 64)) == FAR
+        assert form_of(wrap, wrap.ray_start(f3(1, 1, 1), f3(1, 1, 1), f3(1, bad, 1), 1.0, 0.0), 0.0, 1.0, (64, 64, 64)) == FAR
         assert wrap.form(1.0, 0.0, f3(64, bad, 64), f3(64, 64, 64), (C.c_int * 3)(64, 64, 64)) == FAR
+
+
+def entry(o, d, ext, clamp):
+    """Start of a ray as the kernels form it (ray_interval, ray_setup), in FP32."""
+    F = np.float32
+    with np.errstate(all="ignore"):
+        tn, tf = F(-np.inf), F(np.inf)
+        for i in range(3):
+            if d[i] == 0:
+                if o[i] < 0 or o[i] > ext[i]:
+                    return None
+                continue
+            inv = F(1) / d[i]
+            t0, t1 = (F(0) - o[i]) * inv, (ext[i] - o[i]) * inv
+            tn, tf = np.fmax(tn, np.fmin(t0, t1)), np.fmin(tf, np.fmax(t0, t1))
+        if not tn < tf or (clamp and not tf > 0):
+            return None
+        if clamp:
+            tn = np.fmax(tn, F(0))
+        return o + tn * d
+
+
+def test_ray_starts_stay_within_their_bound(wrap):
+    """Directions down to denormals, alone and beside large components, and origins up to 1e30 away:
+    a ray's first position is within the bound, or the bound is infinite."""
+    rng = np.random.default_rng(9)
+    F = np.float32
+    ext = np.array([1.0, 0.25, 0.5], F)
+    one = f3(1, 1, 1)
+    unbounded = finite = outside = 0
+    for k in range(40000):
+        d = (rng.standard_normal(3) * 10.0 ** rng.uniform(-45, 3, 3)).astype(F)
+        if k % 2:
+            d[rng.integers(0, 3, 2)] = 0
+        if k % 3 == 0:
+            d = rng.standard_normal(3).astype(F)
+        if not np.any(d):
+            continue
+        if k % 5 == 0:  # a camera far away, aimed at the box
+            t = 10.0 ** rng.uniform(0, 30)
+            o = (rng.random(3) * ext - t * d.astype(np.float64)).astype(F)
+        else:
+            o = (rng.uniform(-0.2, 1.2, 3) * ext).astype(F)
+        if not np.all(np.isfinite(o)):
+            continue
+        clamp = k % 7 == 0 and float(np.abs(d).max()) >= 0.5
+        pos = entry(o, d, ext, clamp)
+        if pos is None:
+            continue
+        bound = wrap.ray_start(f3(*ext), one, one, float(np.abs(o).max()), 0.0 if clamp else float(np.abs(d).max()))
+        if np.isinf(bound):
+            unbounded += 1
+            continue
+        finite += 1
+        largest = float(np.nanmax(np.abs(pos))) if not np.all(np.isnan(pos)) else 0.0
+        outside += largest > 1.0
+        assert largest <= bound, (o, d, pos, bound)
+    assert unbounded > 100 and finite > 5000 and outside > 100
+    # the view that no bound holds for: a denormal direction from inside the box
+    assert np.isinf(entry(np.array([0.5, 0.1, 0.2], F), np.array([0, 0, -1e-40], F), ext, False)[2])
+    assert wrap.ray_start(f3(*ext), one, one, 0.5, 1e-40) == float("inf")
+    assert form_of(wrap, wrap.ray_start(f3(*ext), one, one, 0.5, 1e-40), 0.0, 1.0, (60, 60, 60)) == FAR
+    assert form_of(wrap, wrap.ray_start(f3(*ext), one, one, 1e12, 1.0), 0.0, 1.0, (60, 60, 60)) == FAR
 
 
 def test_chosen_form_is_exact_within_its_bound(wrap):
@@ -174,3 +240,23 @@ def test_frame_on_each_side_of_the_line(ctx, oracle, sampler, lit, m, freq):
     ref, smp = sc.render(w.params, view, 32, 16)
     assert float(ref[..., :3].max()) > 0.01 and abs(int(ctx.stats().samples) - int(smp.sum())) <= 0.01 * smp.sum() + 2
     assert float(np.sqrt(np.mean((img.astype(np.float64) - ref) ** 2))) <= 1e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("technique", ["raycast", "slicing"])
+@pytest.mark.parametrize("view", [wl.ortho_view(direction=(0.0, 0.0, -1e-40)), wl.ortho_view(direction=(1e-42, 0.0, 1e-40)),
+                                  wl.perspective_view(distance=1.5e8, fovy=4e-7),
+                                  wl.ortho_view(center=(0.5 - 1e5, 0.5 - 2e5, 0.5 - 3e5), direction=(0.1, 0.2, 0.3))])
+def test_views_without_a_bound(ctx, oracle, technique, view):
+    """Directions of denormal components (rays that begin at infinity) and cameras so far away that rays begin
+    outside the box: the cells read what the general gather reads."""
+    w, _, vid = still(ctx, oracle, (16, 16, 16), (1.0, 1.0, 1.0), (60, 30, 60), 4096.0, "cell", False)
+    imgs = []
+    for sampler in ("cell", "gather"):
+        p = w.params
+        p.sampler, p.technique, p.num_iterations = capi.SAMPLER[sampler], capi.TECHNIQUE[technique], 16
+        ctx.set_params(p)
+        ctx.set_view(view)
+        imgs.append(ctx.render(vid, 40, 24))
+        assert technique == "slicing" or view.projection == capi.PERSPECTIVE or ctx.stats().samples > 0
+    np.testing.assert_allclose(imgs[0], imgs[1], rtol=0, atol=1e-5)

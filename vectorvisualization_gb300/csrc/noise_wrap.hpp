@@ -39,13 +39,24 @@ VVLIC_HOST_DEVICE inline void noise_wrap_constants(int m, float* clamp, unsigned
 // The larger of the two; NaN if either is.
 inline double larger(double a, double b) { return b > a || b != b ? b : a; }
 
-// Largest |position| a streamline of a ray starts at: inside the box its ray marches through,
-// [0, max(extent * scale_vol, tex_max)] per axis.
-inline double ray_start_bound(const float ext[3], const float scale_vol[3], const float tex_max[3]) {
-  double start = 0.0;
+// Largest |position| a streamline of a ray starts at.  Every sample but a ray's first lies in the box the
+// ray marches through, [0, tex_max]; the first one, and the planes of a slicing ray, are o + t d for a t
+// of the ray's interval in the object box [0, ext], times scale_vol.  `origin` is the largest |component| of
+// a pixel's ray origin, `dir` that of the direction all rays share, or 0 where the rays start no
+// earlier than t = 0 (perspective views, whose directions have a unit component along the view axis).
+//   Rounding: t and t d are good to a few ulps of (|o| + ext) / d, so a camera far away misses the box's
+//   face by 2^-18 of its distance at most.
+//   Overflow: t stays below far / dir < 1e35 as long as far < 1e35 dir, so an axis whose own 1 / d overflows
+//   (|d| < 2^-128) moves by less than 2^-10.  Otherwise (a direction of denormal components, whose
+//   interval may begin at t = -inf) there is no bound.
+inline double ray_start_bound(const float ext[3], const float scale_vol[3], const float tex_max[3], double origin,
+                              double dir) {
+  double start = 0.0, far = 0.0;
+  for (int i = 0; i < 3; ++i) far = larger(far, origin + std::fabs((double)ext[i]));
+  if (!(far < 1e35 * (dir > 0.0 && dir < 0.5 ? dir : 0.5))) return INFINITY;
   for (int i = 0; i < 3; ++i) {
     const double sv = std::fabs((double)scale_vol[i]);
-    start = larger(start, larger(larger((double)ext[i] * sv, sv), (double)tex_max[i]));
+    start = larger(start, larger((1.0 + 1.0 / 1024.0 + far / 262144.0) * larger((double)ext[i], 1.0) * sv, (double)tex_max[i]));
   }
   return start;
 }

@@ -252,7 +252,12 @@ vvlic_status build_render_args_ex(vvlic_ctx* c, Volume& v, int W, int H, cudaStr
   a.num_iter = p.num_iterations;
   a.lb = lb;
   a.lf = lf;
-  set_noise_wrap(ray_start_bound(a.ext, a.scale_vol, a.tex_max), a);
+  double origin = 0.0, dir = 0.0;
+  for (int i = 0; i < 3; ++i) {
+    origin = larger(origin, std::fabs((double)a.o0[i]) + W * std::fabs((double)a.o1[i]) + H * std::fabs((double)a.o2[i]));
+    if (!a.clamp0) dir = larger(dir, std::fabs((double)a.d0[i]));
+  }
+  set_noise_wrap(ray_start_bound(a.ext, a.scale_vol, a.tex_max, origin, dir), a);
   a.illum = p.illum;
   a.tf_index = p.tf_index;
   a.sof = p.speed_of_flow;
