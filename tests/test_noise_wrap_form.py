@@ -79,7 +79,7 @@ def test_lic_volume_of_a_thin_lit_volume_takes_the_general_form(wrap, n, sd, m, 
 
 def test_line_between_the_forms(wrap):
     limit = (1 << 19) - 4096
-    for m, near in (((64, 64, 64), MASK), ((60, 64, 64), MUL), ((64, 60, 1), FAR)):
+    for m, near in (((64, 64, 64), MASK), ((60, 64, 64), MUL), ((64, 60, 2), MUL)):
         for k in (0, 1):
             freq = (limit - 1) / 1.01 / 64
             assert form_of(wrap, 1.0 - k, float(k), 0.999999 * freq, m) == near
@@ -161,9 +161,9 @@ def test_chosen_form_is_exact_within_its_bound(wrap):
     rng = np.random.default_rng(5)
     near = 0
     for _ in range(400):
-        m = [int(v) for v in rng.integers(1, 2049, 3)]
+        m = [int(v) for v in rng.integers(2, 2049, 3)]
         if rng.random() < 0.3:
-            m = [1 << int(v) for v in rng.integers(0, 12, 3)]
+            m = [1 << int(v) for v in rng.integers(1, 12, 3)]
         freq, start, reach = (float(np.float32(2.0 ** v)) for v in rng.uniform(-4, 12, 3))
         form = form_of(wrap, start, reach, freq, m)
         if form == FAR:
@@ -184,6 +184,20 @@ def test_chosen_form_is_exact_within_its_bound(wrap):
                 b = (bits - BITS + np.uint32(off)).astype(np.uint64)
                 np.testing.assert_array_equal(b - ((b * np.uint64(mul)) >> np.uint64(32)) * np.uint64(k), want)
     assert near > 50
+
+
+def test_single_texels_are_two_cells(tmp_path, wrap):
+    """Extents of one: both cells hold the texel, so every form reads it; the other extents are their own."""
+    src = SOURCE + 'extern "C" int cells(int m) { return vvlic::noise_cell_extent(m); }'
+    (tmp_path / "c.cpp").write_text(src)
+    subprocess.run([shutil.which("g++") or shutil.which("c++"), "-std=c++17", "-shared", "-fPIC", "-I",
+                    os.path.join(ROOT, "vectorvisualization_gb300", "csrc"), str(tmp_path / "c.cpp"), "-o",
+                    str(tmp_path / "c.so")], check=True)
+    cells = C.CDLL(str(tmp_path / "c.so")).cells
+    assert [cells(m) for m in (1, 2, 3, 2048)] == [2, 2, 3, 2048]
+    for m in ((200, 150, 1), (1, 1, 3), (1, 64, 64), (1, 1, 1)):
+        form = form_of(wrap, 1.0, 0.5, 2.0, [cells(k) for k in m])
+        assert form == (MASK if all(k & (k - 1) == 0 for k in m) else MUL)
 
 
 # ------------------------------------------------------------------------------------------
@@ -260,3 +274,26 @@ def test_views_without_a_bound(ctx, oracle, technique, view):
         imgs.append(ctx.render(vid, 40, 24))
         assert technique == "slicing" or view.projection == capi.PERSPECTIVE or ctx.stats().samples > 0
     np.testing.assert_allclose(imgs[0], imgs[1], rtol=0, atol=1e-5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [(20, 15, 1), (1, 15, 20), (12, 1, 1), (1, 1, 1), (16, 32, 1), (1, 7, 2)])
+@pytest.mark.parametrize("freq", [1.0, -2.0, 65536.0])
+def test_noise_of_a_single_texel_along_an_axis(ctx, m, freq):
+    """CELL reads what GATHER reads, in the fast forms and (65536) the general one, also after the noise is
+    replaced in place."""
+    ctx.upload_field(wl.vortex_field(12, seed=3))
+    w = wl.c1(size=12, image=8)
+    vid = wl.setup_context(ctx, w)
+    p = w.params
+    p.steps_backward, p.steps_forward, p.freq_scale, p.step_size_lic = 3, 4, freq, 0.0
+    ctx.set_view(wl.ortho_view())
+    rng = np.random.default_rng(1)
+    for _ in range(2):
+        ctx.upload_noise(rng.integers(0, 256, m[::-1]).astype(np.uint8))
+        imgs = []
+        for sampler in ("cell", "gather"):
+            p.sampler = capi.SAMPLER[sampler]
+            ctx.set_params(p)
+            imgs.append(ctx.render(vid, 33, 18))
+        np.testing.assert_allclose(imgs[0], imgs[1], rtol=0, atol=2e-5)

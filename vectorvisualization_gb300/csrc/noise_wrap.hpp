@@ -15,8 +15,8 @@ namespace vvlic {
 // How a noise cell's index wraps (REPEAT), chosen on the host per launch (choose_noise_wrap):
 //   kWrapMask  every extent a power of two: a mask;
 //   kWrapMul   other extents: a multiply-high by a host-computed reciprocal;
-//   kWrapFar   positions whose noise coordinate may exceed +-2^19 (or an extent of 1 beside odd
-//              ones): floor, conversion and integer remainder.
+//   kWrapFar   positions whose noise coordinate may exceed +-2^19: floor, conversion and mask or integer
+//              remainder.
 // The first two take floor(u) from the rounding of one addition: u + 1.5 * 2^23 rounded down holds
 // floor(u) in its low mantissa bits (exact for |u| < 2^22).  FRND and F2I, the direct forms, issue
 // at an eighth of the FADD rate (15 against 118 lanes per SM clock, three of each per tap).
@@ -24,6 +24,11 @@ enum NoiseWrap : int { kWrapFar = 0, kWrapMask = 1, kWrapMul = 2 };
 constexpr float kFloorMagic = 12582912.0f;    // 1.5 * 2^23
 constexpr unsigned kFloorBits = 0x4B400000u;  // its bit pattern
 constexpr int kWrapReach = 1 << 19;           // |noise coordinate| bound of kWrapMask / kWrapMul
+
+// Extent of the noise cells along an axis of m texels: a single texel is held as two equal cells, so that
+// every extent has a multiply-high form (an 800x600 frame with a 200 x 150 x 1 noise took 7.82 ms in the
+// general form).
+VVLIC_HOST_DEVICE inline int noise_cell_extent(int m) { return m > 1 ? m : 2; }
 
 // Wrap constants of an extent m: `clamp` is the coordinate a NaN position reads, congruent
 // to -2^24 modulo m (the lower clamp of the general form) and below every finite coordinate;
@@ -69,21 +74,20 @@ inline double voxel_start_bound(const float scale_vol[3]) {
 }
 
 // The form for streamlines that start within `start` of the origin and move by at most `reach` along
-// an axis, under noise texel scales `nscale` (value taps) and `nscale_grad` (gradient taps) and noise
+// an axis, under noise texel scales `nscale` (value taps) and `nscale_grad` (gradient taps) and cell
 // extents m: |noise coordinate| is bounded by (start + reach) * scale, with a margin for the
 // rounding of the positions.  NaN positions read the clamp.
 inline int choose_noise_wrap(double start, double reach, const float nscale[3], const float nscale_grad[3],
                              const int m[3]) {
   double scale = 0.0;
-  bool mask = true, one = false;
+  bool mask = true;
   for (int i = 0; i < 3; ++i) {
     scale = larger(scale, larger(std::fabs((double)nscale[i]), std::fabs((double)nscale_grad[i])));
     mask = mask && (m[i] & (m[i] - 1)) == 0;
-    one = one || m[i] == 1;
   }
   const double bound = 1.01 * (start + reach) * scale + 1.0;
   if (!(bound < (double)(kWrapReach - 4096))) return kWrapFar;  // also for NaN
-  return mask ? kWrapMask : (one ? kWrapFar : kWrapMul);
+  return mask ? kWrapMask : kWrapMul;
 }
 
 }  // namespace vvlic

@@ -500,15 +500,16 @@ __global__ void field_cells_kernel(const void* texels, int nx, int ny, int nz, v
   }
 }
 
-// noise cell i per axis covers texels i and (i+1) mod m (REPEAT): m^3 cells
+// noise cell i per axis covers texels i and (i+1) mod m (REPEAT); an axis of one texel has two cells
+// (noise_cell_extent)
 __global__ void noise_cells_kernel(const uint8_t* texels, int mx, int my, int mz, int ch, uint8_t* cells) {
-  const size_t count = (size_t)mx * my * mz;
-  const int m[3] = {mx, my, mz};
+  const int m[3] = {noise_cell_extent(mx), noise_cell_extent(my), noise_cell_extent(mz)};
+  const size_t count = noise_cell_count(m);
   for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < count; v += (size_t)gridDim.x * blockDim.x) {
-    const int x = (int)(v % mx), y = (int)((v / mx) % my), z = (int)(v / ((size_t)mx * my));
+    const int x = (int)(v % m[0]), y = (int)((v / m[0]) % m[1]), z = (int)(v / ((size_t)m[0] * m[1]));
     const size_t a = noise_cell_index(x, y, z, m);
-    const int xs[2] = {x, x + 1 == mx ? 0 : x + 1}, ys[2] = {y, y + 1 == my ? 0 : y + 1},
-              zs[2] = {z, z + 1 == mz ? 0 : z + 1};
+    const int xs[2] = {x < mx ? x : 0, x + 1 < mx ? x + 1 : 0}, ys[2] = {y < my ? y : 0, y + 1 < my ? y + 1 : 0},
+              zs[2] = {z < mz ? z : 0, z + 1 < mz ? z + 1 : 0};
     // the cell is assembled in registers and written with 16-byte (RGBA: 32-byte cells) or one
     // 8-byte (value: 8-byte cells) stores; cells are 32- / 8-byte aligned
     if (ch == 4) {
@@ -665,7 +666,8 @@ cudaError_t launch_fill_arrays(const void* d_texels, const int n[3], int storage
 
 cudaError_t launch_build_noise_cells(const uint8_t* d_texels, const int m[3], int ch, uint8_t* d_cells,
                                      cudaStream_t s) {
-  const size_t count = (size_t)m[0] * m[1] * m[2];
+  const int cells[3] = {noise_cell_extent(m[0]), noise_cell_extent(m[1]), noise_cell_extent(m[2])};
+  const size_t count = noise_cell_count(cells);
   noise_cells_kernel<<<grid_for(count), kThreads, 0, s>>>(d_texels, m[0], m[1], m[2], ch, d_cells);
   return cudaGetLastError();
 }

@@ -32,7 +32,8 @@ vvlic_status ensure_cells(vvlic_ctx* c, Volume& v, cudaStream_t s) {
 
 vvlic_status ensure_noise_cells(vvlic_ctx* c, NoiseTex& n, cudaStream_t s) {
   if (n.d_cells) return VVLIC_OK;
-  const size_t bytes = noise_cell_count(n.m) * 8 * n.ch;
+  const int cells[3] = {noise_cell_extent(n.m[0]), noise_cell_extent(n.m[1]), noise_cell_extent(n.m[2])};
+  const size_t bytes = noise_cell_count(cells) * 8 * n.ch;
   cudaError_t e = cudaMalloc(&n.d_cells, bytes);
   if (e != cudaSuccess) return cuda_fail(c, e, "noise cell allocation");
   e = launch_build_noise_cells(n.d_texels, n.m, n.ch, n.d_cells, s);
@@ -206,8 +207,9 @@ vvlic_status build_render_args_ex(vvlic_ctx* c, Volume& v, int W, int H, cudaStr
       break;
   }
 
+  const bool cells = p.sampler == VVLIC_SAMPLER_CELL || p.sampler == VVLIC_SAMPLER_HYBRID;
   for (int i = 0; i < 3; ++i) {
-    a.m[i] = c->noise.m[i];
+    a.m[i] = cells ? noise_cell_extent(c->noise.m[i]) : c->noise.m[i];
     a.sn[i] = c->sn[i];
   }
   a.noise_ch = c->noise.ch;
@@ -239,8 +241,8 @@ vvlic_status build_render_args_ex(vvlic_ctx* c, Volume& v, int W, int H, cudaStr
   a.freq_scale = p.low_res ? 0.7f * p.freq_scale : p.freq_scale;
   const bool nofreq = (p.quirks & VVLIC_QUIRK_GRAD_NOISE_NO_FREQ) != 0;
   for (int i = 0; i < 3; ++i) {
-    a.nscale[i] = (float)((double)a.freq_scale * a.m[i]);
-    a.nscale_grad[i] = nofreq ? (float)a.m[i] : a.nscale[i];
+    a.nscale[i] = (float)((double)a.freq_scale * c->noise.m[i]);
+    a.nscale_grad[i] = nofreq ? (float)c->noise.m[i] : a.nscale[i];
   }
   a.alpha_corr = p.low_res ? 2.0f * p.step_size_vol * 128.0f : p.step_size_vol * 128.0f;
   a.h_eff = h * p.eye_dist_factor;
