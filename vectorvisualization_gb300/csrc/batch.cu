@@ -199,14 +199,15 @@ vvlic_status batch_render(vvlic_ctx* c, const vvlic_job* jobs, int n, cudaStream
   int storage, sampler, integ, ntiles;
   bool grad;
   std::vector<unsigned> start;
+  // A stream that the caller is capturing is refused before anything is allocated or launched: a layout filled
+  // into the caller's graph would count as filled, and the job table would be read at the graph's launch.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+    return cuda_fail(c, cudaErrorStreamCaptureUnsupported, "batch on a stream that is being captured");
   vvlic_status st = prepare_batch(c, jobs, n, tw, sampler_override, s, &storage, &sampler, &integ, &grad, &ntiles,
                                   start);
   if (st) return st;
   if (job_by_job(c, jobs, n)) {
-    // refused as the captured sequence below is: a stream that the caller is capturing
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
-      return cuda_fail(c, cudaErrorStreamCaptureUnsupported, "batch on a stream that is being captured");
     if ((st = launch_jobs(c, n, storage, sampler, integ, grad, s))) return st;
     c->stats_pending = true;
     c->tape_flag_pending = false;
