@@ -59,3 +59,21 @@ def test_first_batch_inside_a_capture(ctx, size, sampler, mode):
     ctx.batch_render(jobs, torch.cuda.Stream().cuda_stream)
     torch.cuda.synchronize()
     check(ctx, vid, outs, views, size)
+
+
+@pytest.mark.parametrize("size", [16, 48])
+def test_legacy_default_stream_is_refused(ctx, size):
+    import torch
+
+    vid, jobs, outs, views = scene(ctx, size)
+    for _ in range(2):  # also once the shape's launch sequence exists
+        with pytest.raises(capi.VVLICError) as e:
+            ctx.batch_render(jobs, 1)  # cudaStreamLegacy
+        assert e.value.status == capi.ERR_CUDA
+        assert all(float(o.abs().max()) == 0.0 for o in outs)
+        ctx.batch_render(jobs, torch.cuda.Stream().cuda_stream)
+        torch.cuda.synchronize()
+        check(ctx, vid, outs, views, size)
+        for o in outs:
+            o.zero_()
+        torch.cuda.synchronize()

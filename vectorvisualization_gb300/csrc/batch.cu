@@ -204,6 +204,8 @@ vvlic_status batch_render(vvlic_ctx* c, const vvlic_job* jobs, int n, cudaStream
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
     return cuda_fail(c, cudaErrorStreamCaptureUnsupported, "batch on a stream that is being captured");
+  if (s == cudaStreamLegacy)  // which the persistent path cannot capture: refused whatever the jobs' sizes
+    return cuda_fail(c, cudaErrorStreamCaptureUnsupported, "batch on the legacy default stream");
   vvlic_status st = prepare_batch(c, jobs, n, tw, sampler_override, s, &storage, &sampler, &integ, &grad, &ntiles,
                                   start);
   if (st) return st;
