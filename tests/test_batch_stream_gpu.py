@@ -1,4 +1,4 @@
-"""Streams a batch may not run on, and what it does to those it may: a first batch inside a caller's capture is
+"""Streams a batch may not run on, and its use of those it may.  A first batch inside a caller's capture is
 refused before it touches the capture, the context or the layouts."""
 import numpy as np
 import pytest
@@ -76,4 +76,36 @@ def test_legacy_default_stream_is_refused(ctx, size):
         check(ctx, vid, outs, views, size)
         for o in outs:
             o.zero_()
+        torch.cuda.synchronize()
+
+
+def test_batch_keeps_its_streams_priority(ctx, vvlic_lib):
+    """Jobs launched one by one on a high-priority stream, all of them, overtake a long frame of another
+    context on a stream of default priority."""
+    import torch
+
+    vid, jobs, outs, views = scene(ctx, 64, count=16)
+    high = torch.cuda.Stream(priority=-1)
+    low = torch.cuda.Stream(priority=0)
+    ctx.batch_render(jobs, low.cuda_stream)  # layouts, and streams of the other priority
+    ctx.batch_render(jobs, high.cuda_stream)
+    torch.cuda.synchronize()
+    check(ctx, vid, outs, views, 64)
+    with capi.Context(0) as other:
+        other.upload_noise(wl.dense_noise(64, seed=4), capi.NOISE_GRAD_CENTRAL)
+        big = other.upload_field(wl.vortex_field(64, seed=1), storage="f16")
+        p = capi.params_default()
+        p.integrator, p.illum, p.step_size_vol = capi.RK4, capi.ILLUM_GRADIENT, 1.0 / 512
+        p.steps_backward = p.steps_forward = 60
+        other.set_params(p)
+        other.set_view(wl.perspective_view(distance=2.2))
+        img = torch.empty(1024, 1024, 4, device="cuda")
+        other.render_device(big, img.data_ptr(), 64, 64, stream=low.cuda_stream)
+        torch.cuda.synchronize()
+        done = torch.cuda.Event()
+        other.render_device(big, img.data_ptr(), 1024, 1024, stream=low.cuda_stream)
+        done.record(low)
+        ctx.batch_render(jobs, high.cuda_stream)
+        high.synchronize()
+        assert not done.query()
         torch.cuda.synchronize()

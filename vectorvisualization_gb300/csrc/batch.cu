@@ -155,7 +155,8 @@ vvlic_status prepare_batch(vvlic_ctx* c, const vvlic_job* jobs, int n, int tw, i
 // them again and again through the pipe that also serves the noise cells.  24 views of 8 uneven
 // volumes, one by one / persistent: 86.5 / 105.6 ms at 512^2 (lit 136 / 223), 26.5 / 37.1 at 256^2, 3.2 /
 // 12.7 at 64^2; 320 views at 32^2 14.9 / 21.9 ms, 800 at 16^2 27.6 / 13.6 (launches).  The line lies at a mean
-// of a sixteenth of the resident warps in 2x2-ray tiles, 30^2 pixels.
+// of a sixteenth of the resident warps in 2x2-ray tiles, 30^2 pixels.  The context's streams have the priority
+// of the caller's.
 bool job_by_job(const vvlic_ctx* c, const vvlic_job* jobs, int n) {
   double tiles = 0.0;
   for (int j = 0; j < n; ++j) tiles += (double)((jobs[j].w + 1) / 2) * (double)((jobs[j].h + 1) / 2);
@@ -164,29 +165,30 @@ bool job_by_job(const vvlic_ctx* c, const vvlic_job* jobs, int n) {
 
 vvlic_status launch_jobs(vvlic_ctx* c, int n, int storage, int sampler, int integ, bool grad, cudaStream_t s) {
   constexpr int B = vvlic_ctx::kBatchStreams;
-  cudaError_t e = cudaSuccess;
-  if (!c->ev_batch_fork) {
-    for (int b = 0; b < B && e == cudaSuccess; ++b) {
-      if (!c->batch_streams[b]) e = cudaStreamCreateWithFlags(&c->batch_streams[b], cudaStreamNonBlocking);
-      if (e == cudaSuccess && !c->ev_batch_join[b]) e = cudaEventCreateWithFlags(&c->ev_batch_join[b], cudaEventDisableTiming);
-    }
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_batch_fork, cudaEventDisableTiming);
-    if (e != cudaSuccess) return cuda_fail(c, e, "batch streams");
+  int priority = 0;
+  cudaError_t e = cudaStreamGetPriority(s, &priority);
+  if (e != cudaSuccess) return cuda_fail(c, e, "batch stream");
+  auto& side = c->batch_streams[priority];  // value-initialised when new
+  for (int b = 0; b < B && e == cudaSuccess; ++b) {
+    if (!side[b]) e = cudaStreamCreateWithPriority(&side[b], cudaStreamNonBlocking, priority);
+    if (e == cudaSuccess && !c->ev_batch_join[b]) e = cudaEventCreateWithFlags(&c->ev_batch_join[b], cudaEventDisableTiming);
   }
+  if (e == cudaSuccess && !c->ev_batch_fork) e = cudaEventCreateWithFlags(&c->ev_batch_fork, cudaEventDisableTiming);
+  if (e != cudaSuccess) return cuda_fail(c, e, "batch streams");
   const int used = std::min(n - 1, B);
   e = cudaMemsetAsync(c->d_counters, 0, 4 * sizeof(unsigned long long), s);
   if (e == cudaSuccess) e = cudaEventRecord(c->ev0, s);
   if (e == cudaSuccess) e = cudaEventRecord(c->ev_batch_fork, s);
-  for (int b = 0; b < used && e == cudaSuccess; ++b) e = cudaStreamWaitEvent(c->batch_streams[b], c->ev_batch_fork, 0);
+  for (int b = 0; b < used && e == cudaSuccess; ++b) e = cudaStreamWaitEvent(side[b], c->ev_batch_fork, 0);
   for (int j = 0; j < n && e == cudaSuccess; ++j) {
     RenderArgs& a = c->h_jobs[j];
     a.count_steps = 1;
     const int b = j % (used + 1);
-    e = launch_raycast(a, storage, sampler, integ, grad, c->num_sms, b == 0 ? s : c->batch_streams[b - 1]);
+    e = launch_raycast(a, storage, sampler, integ, grad, c->num_sms, b == 0 ? s : side[b - 1]);
   }
   // joined even after a failed launch: nothing on the side streams outlives the caller's stream
   for (int b = 0; b < used; ++b) {
-    cudaError_t ej = cudaEventRecord(c->ev_batch_join[b], c->batch_streams[b]);
+    cudaError_t ej = cudaEventRecord(c->ev_batch_join[b], side[b]);
     if (ej == cudaSuccess) ej = cudaStreamWaitEvent(s, c->ev_batch_join[b], 0);
     if (e == cudaSuccess) e = ej;
   }

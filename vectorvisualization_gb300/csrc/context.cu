@@ -407,8 +407,9 @@ extern "C" vvlic_status vvlic_destroy(vvlic_ctx* c) {
   if (c->d_jobs) cudaFree(c->d_jobs);
   if (c->d_batch) cudaFree(c->d_batch);
   if (c->ev_jobs) cudaEventDestroy(c->ev_jobs);
-  for (cudaStream_t b : c->batch_streams)
-    if (b) cudaStreamDestroy(b);
+  for (auto& streams : c->batch_streams)
+    for (cudaStream_t b : streams.second)
+      if (b) cudaStreamDestroy(b);
   for (cudaEvent_t ev : c->ev_batch_join)
     if (ev) cudaEventDestroy(ev);
   if (c->ev_batch_fork) cudaEventDestroy(c->ev_batch_fork);

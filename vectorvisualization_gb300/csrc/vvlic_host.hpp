@@ -6,6 +6,7 @@
 
 #include <cmath>
 #include <cstdarg>
+#include <array>
 #include <map>
 #include <string>
 
@@ -150,9 +151,10 @@ struct vvlic_ctx {
   int batch_tile_w = 8;                 // warp tile width (autotuned)
   int batch_sampler_override = -1;      // sampler chosen by the autotuner (-1: the jobs')
   bool last_was_batch = false;
-  // streams of batches whose jobs are launched one by one (batch.cu), created on first use
+  // streams of batches whose jobs are launched one by one (batch.cu), created on first use for each
+  // priority of a caller's stream (a device has six)
   static constexpr int kBatchStreams = 7;
-  cudaStream_t batch_streams[kBatchStreams] = {};
+  std::map<int, std::array<cudaStream_t, kBatchStreams>> batch_streams;
   cudaEvent_t ev_batch_fork = nullptr, ev_batch_join[kBatchStreams] = {};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   bool stats_pending = false;
