@@ -319,7 +319,7 @@ extern "C" vvlic_status vvlic_batch_autotune(vvlic_ctx* c, const vvlic_job* jobs
       }
     }
   }
-  c->batch_tile_w = bt;
+  if (shaped) c->batch_tile_w = bt;  // otherwise an earlier tuning of small jobs stands
   c->batch_sampler_override = bs;
   drop_graph(c);
   if (best_tile_w) *best_tile_w = bt;
