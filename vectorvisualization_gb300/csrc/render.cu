@@ -49,16 +49,15 @@ FieldSurfaces surfaces(const Volume& v) {
   return arr;
 }
 
-// Texture copy of a volume.  128-bit texels filter at an eighth of the texture unit's rate, so F32
-// fields are held as a float2 array of (x, y) and two float arrays (Field<F32, kTexture>).
-vvlic_status ensure_texture(vvlic_ctx* c, Volume& v, cudaStream_t s) {
-  if (v.array_bytes) return VVLIC_OK;
+// Arrays, surfaces and textures of the texture copy.  128-bit texels filter at an eighth of the texture
+// unit's rate, so F32 fields are held as a float2 array of (x, y) and two float arrays
+// (Field<F32, kTexture>).
+vvlic_status make_texture(vvlic_ctx* c, Volume& v) {
   const bool f32 = v.storage == VVLIC_STORAGE_F32, u8 = v.storage == VVLIC_STORAGE_UNORM8;
   const cudaChannelFormatDesc desc[3] = {f32 ? cudaCreateChannelDesc<float2>()
                                              : (u8 ? cudaCreateChannelDesc<uchar4>() : cudaCreateChannelDescHalf4()),
                                          cudaCreateChannelDesc<float>(), cudaCreateChannelDesc<float>()};
   const cudaExtent ext = make_cudaExtent(v.n[0], v.n[1], v.n[2]);
-  free_textures(v);  // what an earlier call that failed half way left
   for (int i = 0; i < (f32 ? 3 : 1); ++i) {
     cudaError_t e = cudaMalloc3DArray(&v.array[i], &desc[i], ext, cudaArraySurfaceLoadStore);
     if (e != cudaSuccess) return cuda_fail(c, e, "texture array allocation");
@@ -77,8 +76,20 @@ vvlic_status ensure_texture(vvlic_ctx* c, Volume& v, cudaStream_t s) {
     e = cudaCreateTextureObject(&v.tex[i], &rd, &td, nullptr);
     if (e != cudaSuccess) return cuda_fail(c, e, "texture object");
   }
-  const cudaError_t e = launch_fill_arrays(v.d_texels, v.n, v.storage, surfaces(v), s);
-  if (e != cudaSuccess) return cuda_fail(c, e, "texture array fill");
+  return VVLIC_OK;
+}
+
+vvlic_status ensure_texture(vvlic_ctx* c, Volume& v, cudaStream_t s) {
+  if (v.array_bytes) return VVLIC_OK;
+  vvlic_status st = make_texture(c, v);
+  if (!st) {
+    const cudaError_t e = launch_fill_arrays(v.d_texels, v.n, v.storage, surfaces(v), s);
+    if (e != cudaSuccess) st = cuda_fail(c, e, "texture array fill");
+  }
+  if (st) {
+    free_textures(v);  // nothing stays allocated behind a failed call
+    return st;
+  }
   v.array_bytes = (size_t)v.n[0] * v.n[1] * v.n[2] * texel_bytes(v.storage);
   return VVLIC_OK;
 }
