@@ -39,6 +39,7 @@ vvlic_status fail(vvlic_ctx* c, vvlic_status s, const char* fmt, ...) {
 }
 
 vvlic_status cuda_fail(vvlic_ctx* c, cudaError_t e, const char* what) {
+  cudaGetLastError();  // or the next call's launch check would report this one's failed allocation again
   if (e == cudaErrorMemoryAllocation)
     return fail(c, VVLIC_ERR_OUT_OF_MEMORY, "%s: %s", what, cudaGetErrorString(e));
   return fail(c, VVLIC_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
