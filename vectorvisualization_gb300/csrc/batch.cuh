@@ -6,6 +6,7 @@
 // is shared by every job.
 #pragma once
 
+#include "batch_tiles.hpp"
 #include "render_fwd.cuh"
 
 namespace vvlic {
@@ -31,7 +32,6 @@ __global__ void __launch_bounds__(kThreads, batch_min_blocks<INTEG, GRAD>())
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   RenderArgs& a = s_args[warp];
-  const int th = 32 / tw;
   unsigned cur = 0xffffffffu;
   uint32_t samples_acc = 0, hits_acc = 0;
   unsigned long long steps_acc = 0;
@@ -49,12 +49,11 @@ __global__ void __launch_bounds__(kThreads, batch_min_blocks<INTEG, GRAD>())
       cur = item.x;
     }
     const int tiles_x = (a.W + tw - 1) / tw;
-    // the tile's 32 pixels in four groups of 8 rays (4x2; 8x1 in one-row tiles), four samples at a time
+    // the tile's 32 pixels in four groups of 8 rays, four samples at a time
     constexpr int S = 4, R = 32 / S;
-    const int gw = th == 1 ? R : 4, gx = tw / gw, r = lane % R;
     for (int sub = 0; sub < S; ++sub) {
-      const int px = (int)(item.y % tiles_x) * tw + (sub % gx) * gw + r % gw;
-      const int py = (int)(item.y / tiles_x) * th + (sub / gx) * (R / gw) + r / gw;
+      const BatchPixel pixel = batch_pixel(tw, item.y, tiles_x, sub, lane % R);
+      const int px = pixel.x, py = pixel.y;
       const bool ray = px < a.W && py < a.H;
       if (!__any_sync(0xffffffffu, ray)) continue;
       uint32_t samples, hit;
