@@ -164,6 +164,31 @@ static void set_noise_wrap(double start, RenderArgs& a) {
   for (int i = 0; i < 3; ++i) noise_wrap_constants(a.m[i], &a.nclamp[i], &a.nwrap_mul[i], &a.nwrap_off[i]);
 }
 
+// Whether a sample's alpha can exceed the threshold that ends its ray (shade, with both tables at their extremes;
+// the margin covers the kernels' powf), and the samples of an average ray: the box's volume over its
+// projection along the view axis, in samples.  Work is split by them (launch_one); results do not depend on it.
+static void set_ray_length(const vvlic_ctx* c, RenderArgs& a) {
+  float lo[2] = {c->tf[3], c->tf[4 * VVLIC_TF_ENTRIES]}, hi[2] = {lo[0], lo[1]};
+  for (int i = 0; i < VVLIC_TF_ENTRIES; ++i) {
+    const float v[2] = {c->tf[4 * i + 3], c->tf[4 * VVLIC_TF_ENTRIES + i]};
+    for (int k = 0; k < 2; ++k) {
+      lo[k] = std::min(lo[k], v[k]);
+      hi[k] = std::max(hi[k], v[k]);
+    }
+  }
+  const double al = std::max({(double)hi[0] * hi[1], (double)lo[0] * lo[1], (double)hi[0] * lo[1], (double)lo[0] * hi[1]});
+  a.may_end = !(1.0 - std::pow(std::max(1.0 - al, 0.0), (double)a.alpha_corr) <= (double)a.alpha_thr - 1e-4);
+  double v[3], e[3], len = 0.0, area = 0.0;
+  for (int i = 0; i < 3; ++i) {
+    v[i] = a.d0[i] + 0.5 * a.W * a.d1[i] + 0.5 * a.H * a.d2[i];
+    e[i] = (double)a.tex_max[i] / a.scale_vol[i];  // what the ray marches through, in object space
+    len += v[i] * v[i];
+  }
+  for (int i = 0; i < 3; ++i) area += std::fabs(v[i]) * e[(i + 1) % 3] * e[(i + 2) % 3];
+  const double mean = e[0] * e[1] * e[2] * std::sqrt(len) / area / a.step_size;
+  a.mean_samples = mean > 0.0 && mean < 1e9 ? (float)mean : 1e9f;
+}
+
 // Fill the kernel argument block for one volume and image size.
 vvlic_status build_render_args(vvlic_ctx* c, Volume& v, int W, int H, cudaStream_t s, RenderArgs& a) {
   return build_render_args_ex(c, v, W, H, s, c->params, c->view, nullptr, a);
@@ -260,6 +285,7 @@ vvlic_status build_render_args_ex(vvlic_ctx* c, Volume& v, int W, int H, cudaStr
   a.intensity_scale = inv_area / (float)(lf + lb) * p.gradient_scale;  // licKernel.b * gradient.r
   a.illum_scale = p.illum_scale;
   a.alpha_thr = p.alpha_threshold;
+  set_ray_length(c, a);
   a.gate_lo = p.gate_lo;
   a.gate_hi = p.gate_hi;
   a.num_iter = p.num_iterations;

@@ -1,6 +1,7 @@
 // Forward LIC ray-cast kernels: the lic3d_fragment.glsl main() (lic3d_fragment.glsl:5-99) on a raster
 // grid of small CTAs, each warp on a tile of rays with S consecutive samples of each side by side
-// (trace_group).  Instantiated per field storage in render_f32.cu / render_f16.cu /
+// (trace_group); frames whose rays may end early or are short take one lane to a ray first (head_samples).
+// Instantiated per field storage in render_f32.cu / render_f16.cu /
 // render_bf16.cu / render_u8.cu so the translation units compile in parallel.
 //
 // The raster grid took the place of persistent warps that pulled 8x4-pixel tiles longest ray first
@@ -78,12 +79,16 @@ __host__ __device__ inline CtaShape cta_shape(int threads) {
   return threads >= 128 ? CtaShape{2, threads / 64} : CtaShape{1, threads / 32};
 }
 
-template <int ST, int FL, int NL, int INTEG, bool GRAD, int S>
+// Which part of its rays a kernel marches: all of it, the first `bound` passes (rays that go on leave the
+// composite so far in their pixel, with the sign of alpha set), or the rest of those, behind `bound` samples.
+enum Part : int { kWhole, kHead, kRest };
+
+template <int ST, int FL, int NL, int INTEG, bool GRAD, int S, int PART>
 __global__ void __launch_bounds__(cast_threads<INTEG>(), cast_min_ctas<ST, INTEG, GRAD>())
-    raycast_kernel(const __grid_constant__ RenderArgs a, int strip) {
+    raycast_kernel(const __grid_constant__ RenderArgs a, int strip, uint32_t bound) {
   __shared__ __align__(16) float s_tf[5 * VVLIC_TF_ENTRIES];
-  load_tf(a, s_tf);
   using T = GroupTile<S>;
+  if (PART != kRest) load_tf(a, s_tf);
   const CtaShape cta = cta_shape(blockDim.x);
   unsigned bx = blockIdx.x, by = blockIdx.y;
   if (strip) {  // CTAs run up one strip of `strip` columns after the other
@@ -95,12 +100,27 @@ __global__ void __launch_bounds__(cast_threads<INTEG>(), cast_min_ctas<ST, INTEG
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane % (32 / S);
   const int px = ((int)bx * cta.wx + warp % cta.wx) * T::w + r % T::w;
   const int py = ((int)by * cta.wy + warp / cta.wx) * T::h + r / T::w;
-  const bool ray = px < a.W && py < a.H;
+  bool ray = px < a.W && py < a.H, open;
   uint32_t samples, hit;
-  const float4 dest = trace_group<ST, FL, NL, INTEG, GRAD, S>(a, s_tf, ray, px, py, samples, hit);
+  float4 dest = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4* pixel = reinterpret_cast<float4*>(a.out) + ((size_t)py * a.W + px);
+  if (PART == kRest) {
+    if (ray) {
+      dest = *pixel;
+      ray = signbit(dest.w);
+      dest.w = fabsf(dest.w);
+    }
+    if (!__syncthreads_or(ray)) return;
+    load_tf(a, s_tf);
+  }
+  dest = trace_group<ST, FL, NL, INTEG, GRAD, S>(a, s_tf, ray, px, py, samples, hit, PART == kRest ? bound : 0u, dest,
+                                                 PART == kHead ? bound : 0xffffffffu, open);
   const bool store = ray && lane < 32 / S;
-  if (store) store_pixel(a, px, py, dest, samples);
-  flush_counters(a, store ? samples : 0u, store ? hit : 0u);
+  if (store) {
+    if (PART == kHead && open) *pixel = make_float4(dest.x, dest.y, dest.z, -dest.w);
+    else store_pixel(a, px, py, dest, samples);
+  }
+  flush_counters(a, store ? samples - (PART == kRest ? bound : 0u) : 0u, store && PART != kRest ? hit : 0u);
 }
 
 // CTA and group size by the number of 2x2-ray warp tiles against the warps the chip holds:
@@ -120,30 +140,57 @@ __global__ void __launch_bounds__(cast_threads<INTEG>(), cast_min_ctas<ST, INTEG
 // few rows: 2048^2 orbit frame 1379 against 1404 ms, 1024^2 447 against 453 (Heun: 59.6 against 58.9).
 inline long long cast_tiles(const RenderArgs& a) { return (long long)((a.W + 1) / 2) * ((a.H + 1) / 2); }
 inline long long resident_warps(int num_sms) { return 24ll * num_sms; }
+// Samples that a frame's rays take one at a time, a lane to a ray, before the groups: where rays end after a sample
+// or two, or are no longer than that, seven of a group's eight lanes are lost.
+//   Frames whose samples can end a ray (may_end): the first 1 to 16 by the frame's size, since a lane to a ray is
+//     as fast as groups on a large frame only (192^3, 131 samples a ray, ms by lane / groups: 256^2
+//     3.9 / 1.6, 512^2 6.6 / 5.2, 1024^2 19.4 / 19.3).  All opaque, 1024^2, groups alone / so: unlit 1.23 / 0.23 ms, lit
+//     0.80 / 0.24, FP32 2.24 / 0.40, RK4 2.21 / 0.39.  Rays that go on pay 1 to 3 % for it.
+//   Frames of short rays, up to 1.5 times as many samples on average (thin volumes): all of them, 0xffffffff.
+//     512 x 512 x 1 volume, 2 samples a ray, 1024^2, groups / so: unlit 1.13 / 0.31 ms, lit 0.81 / 0.40, RK4 1.97 / 0.56;
+//     14 samples a ray 2.42 / 2.07, 3.08 / 2.61, 4.46 / 3.96.
+// A recording's checkpoints hold the state before every 32nd sample, which a group knows for its first one only:
+// its rays take a multiple of the groups' eight samples first.
+inline uint32_t head_samples(const RenderArgs& a, int num_sms) {
+  const uint32_t head = (uint32_t)std::min<long long>(16, cast_tiles(a) / (2 * resident_warps(num_sms)));
+  if (head > 0 && a.mean_samples <= 1.5f * head) return 0xffffffffu;
+  return a.may_end ? (a.tape_is ? head / 8 * 8 : head) : 0u;
+}
+static_assert(kSegment % 8 == 0, "checkpoints at the first sample of a group");
 template <int INTEG, bool GRAD> static int cast_cta_threads(const RenderArgs& a, int num_sms) {
   const long long tiles = cast_tiles(a), resident = resident_warps(num_sms);
   return tiles <= 2 * resident ? 64 : (GRAD && INTEG != VVLIC_RK4 && tiles >= 16 * resident ? 256 : 128);
 }
 
-template <int ST, int FL, int NL, int INTEG, bool GRAD>
-static cudaError_t launch_one(const RenderArgs& a, int num_sms, cudaStream_t stream) {
+// One part of a frame in groups of S samples.
+template <int ST, int FL, int NL, int INTEG, bool GRAD, int S, int PART>
+static cudaError_t launch_part(const RenderArgs& a, uint32_t bound, int num_sms, cudaStream_t stream) {
   const int threads = cast_cta_threads<INTEG, GRAD>(a, num_sms);
   const int strip = INTEG == VVLIC_RK4 ? 16 : 0;
   const CtaShape cta = cta_shape(threads);
-  const auto grid = [&](int tw, int th) {
-    return dim3((unsigned)((a.W + tw * cta.wx - 1) / (tw * cta.wx)), (unsigned)((a.H + th * cta.wy - 1) / (th * cta.wy)));
-  };
-  if constexpr (GRAD && ST != VVLIC_STORAGE_F32 && INTEG != VVLIC_RK4) {
-    if (cast_tiles(a) >= 8 * resident_warps(num_sms)) {
-      raycast_kernel<ST, FL, NL, INTEG, GRAD, 4><<<grid(GroupTile<4>::w, GroupTile<4>::h), threads, 0, stream>>>(a, strip);
-      return cudaGetLastError();
-    }
-  }
-  if (2 * cast_tiles(a) <= resident_warps(num_sms))
-    raycast_kernel<ST, FL, NL, INTEG, GRAD, 16><<<grid(GroupTile<16>::w, GroupTile<16>::h), threads, 0, stream>>>(a, strip);
-  else
-    raycast_kernel<ST, FL, NL, INTEG, GRAD, 8><<<grid(GroupTile<8>::w, GroupTile<8>::h), threads, 0, stream>>>(a, strip);
+  const int w = GroupTile<S>::w * cta.wx, h = GroupTile<S>::h * cta.wy;
+  const dim3 grid((unsigned)((a.W + w - 1) / w), (unsigned)((a.H + h - 1) / h));
+  raycast_kernel<ST, FL, NL, INTEG, GRAD, S, PART><<<grid, threads, 0, stream>>>(a, strip, bound);
   return cudaGetLastError();
+}
+
+template <int ST, int FL, int NL, int INTEG, bool GRAD>
+static cudaError_t launch_one(const RenderArgs& a, int num_sms, cudaStream_t stream) {
+  constexpr bool kFours = GRAD && ST != VVLIC_STORAGE_F32 && INTEG != VVLIC_RK4;
+  const bool fours = cast_tiles(a) >= 8 * resident_warps(num_sms);
+  const uint32_t head = head_samples(a, num_sms);
+  if (head > 0) {
+    const cudaError_t e = launch_part<ST, FL, NL, INTEG, GRAD, 1, kHead>(a, head, num_sms, stream);
+    if (e != cudaSuccess || head == 0xffffffffu) return e;
+    if constexpr (kFours)
+      if (fours) return launch_part<ST, FL, NL, INTEG, GRAD, 4, kRest>(a, head, num_sms, stream);
+    return launch_part<ST, FL, NL, INTEG, GRAD, 8, kRest>(a, head, num_sms, stream);
+  }
+  if constexpr (kFours)
+    if (fours) return launch_part<ST, FL, NL, INTEG, GRAD, 4, kWhole>(a, 0u, num_sms, stream);
+  if (2 * cast_tiles(a) <= resident_warps(num_sms))
+    return launch_part<ST, FL, NL, INTEG, GRAD, 16, kWhole>(a, 0u, num_sms, stream);
+  return launch_part<ST, FL, NL, INTEG, GRAD, 8, kWhole>(a, 0u, num_sms, stream);
 }
 
 template <int ST, int FL, int NL>

@@ -67,6 +67,9 @@ struct RenderArgs {
   uint32_t* tape_n;
   unsigned long long* tape_overflow;  // rays with more samples than tape_stride
   int tape_stride, tape_nck;
+  // host rules of the work split (launch_one): whether a sample can end its ray, and the samples of an average ray
+  int may_end;
+  float mean_samples;
   float taps[kMaxTaps];
 };
 
@@ -1001,6 +1004,10 @@ __device__ __forceinline__ float3 march(float3 p, float3 dir, float step) {
 // warp, each as long as its longest ray), keeps lanes together when rays end at different samples,
 // and lets the lanes of a warp read overlapping streamlines: a sample's noise cells are mostly its
 // neighbour's.  `ray` is false for lanes without a pixel.  Every lane of the warp calls.
+//
+// A ray can be marched in two parts (launch_one): the first call stops after `passes` passes with `open` set for
+// rays that have not ended, a second one takes them up with `first` samples behind them and `dest` as it
+// was left.
 // Lanes 0, 32/S, 2 * 32/S, ... of a warp: those of its first ray.
 __host__ __device__ constexpr unsigned ray_lanes(int S) {
   unsigned m = 0;
@@ -1010,20 +1017,20 @@ __host__ __device__ constexpr unsigned ray_lanes(int S) {
 
 template <int ST, int FL, int NL, int INTEG, bool GRAD, int S>
 __device__ __forceinline__ float4 trace_group(const RenderArgs& a, const float* s_tf, bool ray, int px, int py,
-                                              uint32_t& samples, uint32_t& hit) {
+                                              uint32_t& samples, uint32_t& hit, uint32_t first, float4 dest,
+                                              uint32_t passes, bool& open) {
   constexpr int R = 32 / S;
   const int lane = threadIdx.x & 31, k = lane / R, r = lane % R;
   const unsigned mine = ray_lanes(S) << r;
-  float4 dest = make_float4(0.f, 0.f, 0.f, 0.f);
   float3 pos = f3(0.f, 0.f, 0.f), dir = pos;
-  samples = 0;
+  samples = first;
   bool alive = ray && ray_setup(a, px, py, pos, dir);
   hit = alive;
   const uint32_t max_samples =
       a.num_iter > 65535 ? 0xffffffffu : (uint32_t)max(a.num_iter, 0) * (uint32_t)max(a.num_iter, 0);
   alive = alive && max_samples > 0;
-  for (int j = 0; j < k; ++j) pos = march(pos, dir, a.step_size);
-  while (__any_sync(0xffffffffu, alive)) {
+  for (uint32_t j = 0; j < first + k; ++j) pos = march(pos, dir, a.step_size);
+  for (; passes > 0 && __any_sync(0xffffffffu, alive); --passes) {
     const float3 next = march(pos, dir, a.step_size);
     // the ray leaves the box after this sample, or has no samples left
     const bool leaves = outside_box(a, next) || max_samples - samples <= (uint32_t)k + 1;
@@ -1047,7 +1054,7 @@ __device__ __forceinline__ float4 trace_group(const RenderArgs& a, const float* 
 #pragma unroll (S < 8 ? S : 8)
     for (int j = 0; j < S; ++j) {
       const int from = j * R + r;
-      const float4 s = shfl4(src, from);
+      const float4 s = S == 1 ? src : shfl4(src, from);
       if (alive && from <= last) {
         dest = blend(dest, s);
         ++samples;
@@ -1056,7 +1063,17 @@ __device__ __forceinline__ float4 trace_group(const RenderArgs& a, const float* 
     alive = alive && ends == 0;
     for (int j = 0; j < S; ++j) pos = march(pos, dir, a.step_size);
   }
+  open = alive;
   return dest;
+}
+
+// Whole rays.
+template <int ST, int FL, int NL, int INTEG, bool GRAD, int S>
+__device__ __forceinline__ float4 trace_group(const RenderArgs& a, const float* s_tf, bool ray, int px, int py,
+                                              uint32_t& samples, uint32_t& hit) {
+  bool open;
+  return trace_group<ST, FL, NL, INTEG, GRAD, S>(a, s_tf, ray, px, py, samples, hit, 0u, make_float4(0.f, 0.f, 0.f, 0.f),
+                                                 0xffffffffu, open);
 }
 
 }  // namespace vvlic
