@@ -146,3 +146,37 @@ def test_adjoint_of_a_split_recording(ctx, lit, integ, case):
     for g, r in zip(got, want):
         assert np.abs(r).max() > 0
         assert np.abs(g - r).max() <= 1e-5 * np.abs(r).max()
+
+
+@pytest.mark.parametrize("integ,lit,ends,lb,lf", [(capi.RK4, False, True, 3, 4), (capi.RK4, True, True, 17, 5),
+                                                  (capi.RK4, True, False, 2, 18), (capi.HEUN, True, True, 16, 17),
+                                                  (capi.EULER, False, True, 0, 33)])
+def test_adjoint_by_lane_per_ray(ctx, integ, lit, ends, lb, lf):
+    """A 1000 x 980 frame's adjoint takes a lane per ray (RK4: two samples of it at a time), its quarters' groups
+    of eight samples: rays of odd and even lengths within and across segments of 32 samples, streamlines around the
+    16 steps of a block of tap sums."""
+    import torch
+
+    vid = ctx.upload_field(wl.vortex_field(16, seed=3), storage="f16")
+    ctx.upload_noise(wl.dense_noise(20, seed=8), capi.NOISE_GRAD_CENTRAL if lit else capi.NOISE_SCALAR)
+    i = np.arange(256, dtype=np.float32)
+    ctx.set_tf(np.stack([i / 255] * 3 + [(0.2 if ends else 0.01) + 0 * i], 1), i / 255)
+    p = params(integ, lit)
+    p.quirks, p.gradient_scale, p.num_iterations = 0, 2.0, 6 if ends else 7
+    p.steps_backward, p.steps_forward, p.step_size_vol, p.step_size_lic = lb, lf, 1.0 / 128, 0.02
+    p.alpha_threshold = 0.14
+    cot = torch.from_numpy(np.random.default_rng(3).standard_normal((980, 1000, 4)).astype(np.float32)).cuda()
+    got, smp = gradients(ctx, vid, p, cot)
+    assert (len(np.unique(smp)) > 5 and smp.max() == 36) if ends else np.all(smp == 49)
+    # parts small enough for groups: below 16 times the resident warps where rays may end
+    nx, ny = (2, 2) if integ == capi.RK4 else (5, 5)
+    w, h = 1000 // nx, 980 // ny
+    want = [np.zeros(g.shape) for g in got]
+    for y0 in range(0, 980, h):
+        for x0 in range(0, 1000, w):
+            part, _ = gradients(ctx, vid, p, cot[y0:y0 + h, x0:x0 + w], x0, y0)
+            for a, b in zip(want, part):
+                a += b
+    for g, r in zip(got, want):
+        assert np.abs(r).max() > 0
+        assert np.abs(g - r).max() <= 1e-5 * np.abs(r).max()

@@ -4,7 +4,7 @@
 // The forward render records a tape: per sample (intensity I, TF coordinate), with gradient
 // lighting also the LIC gradient sum G (4 halves), and every kSegment samples a checkpoint
 // (position, dest before the sample).  A warp takes four rays, eight consecutive samples of each
-// side by side (the forward's groups), and walks their segments last to first.  From the
+// side by side (the forward's groups; adjoint_ray_kernel 32 rays, a lane each, see lane_per_ray), and walks their segments last to first.  From the
 // checkpoint it recomputes the compositing states (cheap: no streamline work), the lanes forming
 // the sources and every lane of a ray blending them in order; going back, every lane of a ray carries
 // the image cotangent through the blends and each lane keeps what its own sample needs.  The
@@ -260,6 +260,60 @@ __device__ __forceinline__ void tap_gradients(const RenderArgs& a, float3 pos, f
   sums.finish(i, lb, lf, s_taps);
 }
 
+// tap_gradients of two samples of each lane's ray: four independent streamline chains per thread, and per tap the
+// two samples' contributions are added in the lane before the warp sum.  A lane walks both samples' streamlines
+// when either has a non-zero cotangent; the other's terms are then zero.
+template <int ST, int FL, int NL, int INTEG, bool GRAD>
+__device__ __forceinline__ void tap_gradients2(const RenderArgs& a, float3 pa, float gIa, float3 gGa, float3 pc, float gIc,
+                                               float3 gGc, long long* s_taps) {
+  const bool act = gIa != 0.0f || gIc != 0.0f ||
+                   (GRAD && (gGa.x != 0.0f || gGa.y != 0.0f || gGa.z != 0.0f || gGc.x != 0.0f || gGc.y != 0.0f ||
+                             gGc.z != 0.0f));
+  const int lb = a.lb, lf = a.lf, L = max(lb, lf);
+  float4 fa = make_float4(0.f, 0.f, 0.f, 0.f), fc = fa;
+  float v0 = 0.0f;
+  const auto dot2 = [&](const float2 (&n)[4], bool second, float gI, float3 gG) {
+    return second ? (GRAD ? tap_dot<true>(make_float4(n[0].y, n[1].y, n[2].y, n[3].y), gI, gG) : gI * n[3].y)
+                  : (GRAD ? tap_dot<true>(make_float4(n[0].x, n[1].x, n[2].x, n[3].x), gI, gG) : gI * n[3].x);
+  };
+  if (act) {
+    fa = Field<ST, FL>::sample(a, pa);
+    fc = Field<ST, FL>::sample(a, pc);
+    float2 n[4];
+    noise_tap2<NL, GRAD>(a, pa, pc, n);
+    v0 = dot2(n, false, gIa, gGa) + dot2(n, true, gIc, gGc);
+  }
+  warp_fixed_add(s_taps + lb, v0);
+  float3 p0 = pa, p1 = pa, p2 = pc, p3 = pc;
+  float4 s0 = fa, s1 = fa, s2 = fc, s3 = fc;
+  TapSums sums;
+  int i = 1;
+  for (; i <= L; ++i) {
+    float vb = 0.0f, vf = 0.0f;
+    if (act) {
+      float2 n[4];
+      if (i <= lb) {
+        p0 = lic_step<ST, FL, INTEG>(a, p0, s0, -1.0f);
+        p2 = lic_step<ST, FL, INTEG>(a, p2, s2, -1.0f);
+      }
+      if (i <= lf) {
+        p1 = lic_step<ST, FL, INTEG>(a, p1, s1, 1.0f);
+        p3 = lic_step<ST, FL, INTEG>(a, p3, s3, 1.0f);
+      }
+      if (i <= lb) {
+        noise_tap2<NL, GRAD>(a, p0, p2, n);
+        vb = dot2(n, false, gIa, gGa) + dot2(n, true, gIc, gGc);
+      }
+      if (i <= lf) {
+        noise_tap2<NL, GRAD>(a, p1, p3, n);
+        vf = dot2(n, false, gIa, gGa) + dot2(n, true, gIc, gGc);
+      }
+    }
+    sums.step(i, vb, vf, lb, lf, s_taps);
+  }
+  sums.finish(i, lb, lf, s_taps);
+}
+
 // A sample's source recomputed from its tape record: what the blend, the lookups and the shading
 // need again in the reverse step.
 template <bool GRAD> struct Sample {
@@ -458,17 +512,127 @@ __global__ void __launch_bounds__(kThreads, VVLIC_ADJ_MIN_BLOCKS)
     if (s_acc[i] != 0) atomicAdd(reinterpret_cast<unsigned long long*>(acc + i), (unsigned long long)s_acc[i]);
 }
 
+// The same by a lane per ray on 8x4-pixel tiles: a segment's positions and states in a local array, its samples
+// last to first, in RK4 two at a time.  Lit RK4 with up to 96 registers (5 CTAs): 2048^2 view along an axis of a
+// 512^3 field, L = 60, 1274 ms against 1339 with 80 and 1333 with 128.
+template <int INTEG, bool GRAD> constexpr int ray_min_blocks() {
+  return GRAD && INTEG == VVLIC_RK4 ? VVLIC_ADJ_MIN_BLOCKS - 1 : VVLIC_ADJ_MIN_BLOCKS;
+}
 template <int ST, int FL, int NL, int INTEG, bool GRAD>
-static cudaError_t launch_adjoint_one(const RenderArgs& a, const float4* g_img, long long* acc, unsigned* next,
-                                      int num_sms, cudaStream_t s) {
-  auto kern = adjoint_kernel<ST, FL, NL, INTEG, GRAD>;
+__global__ void __launch_bounds__(kThreads, ray_min_blocks<INTEG, GRAD>())
+    adjoint_ray_kernel(const __grid_constant__ RenderArgs a, const float4* __restrict__ g_img, long long* acc,
+                       unsigned ntiles, unsigned* __restrict__ next) {
+  __shared__ __align__(16) float s_tf[5 * VVLIC_TF_ENTRIES];
+  __shared__ long long s_acc[kAccSize];
+  for (int i = threadIdx.x; i < kAccSize; i += blockDim.x) s_acc[i] = 0;
+  load_tf(a, s_tf);  // includes __syncthreads
+  constexpr int P = INTEG == VVLIC_RK4 ? 2 : 1;
+  const int lane = threadIdx.x & 31;
+  const unsigned tiles_x = (a.W + 7) / 8, tiles_y = (a.H + 3) / 4;
+  const bool line = !GRAD && (a.illum == VVLIC_ILLUM_ZOECKLER || a.illum == VVLIC_ILLUM_MALLO);
+  float4 Dloc[kSegment];
+  float3 Ploc[kSegment];
+  for (;;) {
+    unsigned t = 0;
+    if (lane == 0) t = atomicAdd(next, 1u);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if (t >= ntiles) break;
+    constexpr unsigned strip = 8;  // up strips of 64 pixels
+    const unsigned col = t / (strip * tiles_y) * strip, rest = t - col * tiles_y, width = min(strip, tiles_x - col);
+    const int x0 = (int)(col + rest % width) * 8, y0 = (int)(rest / width) * 4;
+    const int px = x0 + (lane & 7), py = y0 + (lane >> 3);
+    float3 pos0 = f3(0.f, 0.f, 0.f), dir = f3(0.f, 0.f, 0.f);
+    int n = 0;
+    float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (px < a.W && py < a.H && ray_setup(a, px, py, pos0, dir)) {
+      const size_t ray = (size_t)py * a.W + px;
+      n = (int)min(a.tape_n[ray], (uint32_t)a.tape_stride);
+      g = g_img[ray];
+    }
+    const int longest = (int)__reduce_max_sync(0xffffffffu, (unsigned)n);
+    for (int seg = (longest + kSegment - 1) / kSegment - 1; seg >= 0; --seg) {
+      const int cnt = min(max(n - seg * kSegment, 0), kSegment), top = min(longest - seg * kSegment, kSegment);
+      if (cnt > 0) {
+        size_t ce = tape_ck_entry(a, px, py, seg);
+        if (!in_range(a, (long long)ce + 32, tape_ck_entries(a), VVLIC_CHECK_TAPE)) ce = 0;
+        const float4 p4 = a.tape_ck[ce];
+        float3 p = f3(p4.x, p4.y, p4.z);
+        float4 D = a.tape_ck[ce + 32];
+        for (int j = 0; j < cnt; ++j) {
+          Ploc[j] = p;
+          Dloc[j] = D;
+          D = blend(D, source_rgba(tape_sample<ST, FL, GRAD>(a, s_tf, line, tape_entry_checked(a, px, py, seg * kSegment + j),
+                                                             p, dir).s));
+          p = march(p, dir, a.step_size);
+        }
+      }
+      // the cotangents of sample j: of its intensity (gI) and gradient sum (gG)
+      const auto back = [&](int j, float& gI, float3& gG, float3& pk) {
+        gI = 0.0f;
+        gG = f3(0.f, 0.f, 0.f);
+        pk = f3(0.f, 0.f, 0.f);
+        if (j < 0 || j >= cnt) return false;
+        pk = Ploc[j];
+        const Sample<GRAD> q =
+            tape_sample<ST, FL, GRAD>(a, s_tf, line, tape_entry_checked(a, px, py, seg * kSegment + j), pk, dir);
+        float4 ds;
+        g = blend_vjp(g, premultiplied(q.s), Dloc[j], ds);
+        sample_cotangent<GRAD>(a, s_tf, line, q, ds, s_acc, gI, gG);
+        return gI != 0.0f || (GRAD && (gG.x != 0.0f || gG.y != 0.0f || gG.z != 0.0f));
+      };
+      for (int j = (top + P - 1) / P * P - 1; j >= 0; j -= P) {
+        float gI, gI1;
+        float3 gG, gG1, p, p1;
+        bool need = back(j, gI, gG, p);
+        if constexpr (P == 2) {
+          need |= back(j - 1, gI1, gG1, p1);
+          if (__any_sync(0xffffffffu, need))
+            tap_gradients2<ST, FL, NL, INTEG, GRAD>(a, p, gI, gG, p1, gI1, gG1, s_acc + kAccTaps);
+        } else {
+          if (__any_sync(0xffffffffu, need)) tap_gradients<ST, FL, NL, INTEG, GRAD>(a, p, gI, gG, s_acc + kAccTaps);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kAccSize; i += blockDim.x)
+    if (s_acc[i] != 0) atomicAdd(reinterpret_cast<unsigned long long*>(acc + i), (unsigned long long)s_acc[i]);
+}
+
+// A lane per ray where groups of eight samples lose:
+//   frames of short rays (head_samples), 512 x 512 x 4 volume, 1024^2, groups / lane per ray: unlit 0.40 / 0.17 ms,
+//     lit 2.35 / 1.27, RK4 2.76 / 2.13; 300^2 0.07 / 0.06, 0.25 / 0.19, 0.30 / 0.27;
+//   frames whose rays may end early, from 16 times as many 2x2-ray tiles as resident warps (RK4: 64): all
+//     opaque, 1024^2, 0.31 / 0.06, 0.44 / 0.09, 0.45 / 0.11 ms; rays that go on 5.3 / 3.3, 33.0 / 24.7, 39.5 / 41.5, but at
+//     450^2 1.1 / 1.4, 6.8 / 6.9, 8.5 / 11.0;
+//   the largest lit RK4 frames, from 192 times as many, or 64 where rows of pixels lie along rows of texels: views of
+//     a 512^3 field so / turned, L = 60, 2048^2 1456 / 1274 and 1494 / 1470 ms (before the groups 1312 and 1491),
+//     1024^2 420 / 400 and 480 / 517 (387 and 512).
+template <int INTEG, bool GRAD> static bool lane_per_ray(const RenderArgs& a, int num_sms) {
+  const long long tiles = cast_tiles(a), resident = resident_warps(num_sms);
+  if (head_samples(a, num_sms) == 0xffffffffu) return true;
+  if (a.may_end && tiles >= (INTEG == VVLIC_RK4 ? 64 : 16) * resident) return true;
+  return GRAD && INTEG == VVLIC_RK4 && tiles >= (a.along_rows ? 64 : 192) * resident;
+}
+
+template <typename Kernel>
+static cudaError_t launch_tiles(Kernel kern, const RenderArgs& a, const float4* g_img, long long* acc, unsigned ntiles,
+                                unsigned* next, int num_sms, cudaStream_t s) {
   int per_sm = 0;
   cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, 0);
   if (e != cudaSuccess) return e;
-  const unsigned ntiles = (unsigned)((a.W + 1) / 2) * (unsigned)((a.H + 1) / 2);
   const int grid = (int)std::min<unsigned>((ntiles + kWarps - 1) / kWarps, (unsigned)(std::max(1, per_sm) * num_sms));
   kern<<<grid, kThreads, 0, s>>>(a, g_img, acc, ntiles, next);
   return cudaGetLastError();
+}
+
+template <int ST, int FL, int NL, int INTEG, bool GRAD>
+static cudaError_t launch_adjoint_one(const RenderArgs& a, const float4* g_img, long long* acc, unsigned* next,
+                                      int num_sms, cudaStream_t s) {
+  const auto tiles = [&](int w, int h) { return (unsigned)((a.W + w - 1) / w) * (unsigned)((a.H + h - 1) / h); };
+  if (lane_per_ray<INTEG, GRAD>(a, num_sms))
+    return launch_tiles(adjoint_ray_kernel<ST, FL, NL, INTEG, GRAD>, a, g_img, acc, tiles(8, 4), next, num_sms, s);
+  return launch_tiles(adjoint_kernel<ST, FL, NL, INTEG, GRAD>, a, g_img, acc, tiles(2, 2), next, num_sms, s);
 }
 
 template <int ST, int FL, int NL, bool GRAD>

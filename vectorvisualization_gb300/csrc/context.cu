@@ -308,6 +308,16 @@ extern "C" vvlic_status vvlic_make_filter_table(int32_t filter, int32_t width, u
 // ------------------------------------------------------------------------------------------
 // context
 // ------------------------------------------------------------------------------------------
+static void sort_tf(vvlic_ctx* c) {
+  float* s = c->tf_sorted;
+  for (int i = 0; i < VVLIC_TF_ENTRIES; ++i) {
+    s[i] = c->tf[4 * i + 3];
+    s[VVLIC_TF_ENTRIES + i] = c->tf[4 * VVLIC_TF_ENTRIES + i];
+  }
+  std::sort(s, s + VVLIC_TF_ENTRIES);
+  std::sort(s + VVLIC_TF_ENTRIES, s + 2 * VVLIC_TF_ENTRIES);
+}
+
 static void default_tables(vvlic_ctx* c) {
   // TransferEdit(): rgb identity, alpha and opacity max(0, i-20) (transferEdit.cpp:76-82)
   for (int i = 0; i < VVLIC_TF_ENTRIES; ++i) {
@@ -315,6 +325,7 @@ static void default_tables(vvlic_ctx* c) {
     c->tf[4 * i + 3] = (float)(i < 20 ? 0 : i - 20) / 255.0f;
     c->tf[4 * VVLIC_TF_ENTRIES + i] = (float)(i < 20 ? 0 : i - 20) / 255.0f;
   }
+  sort_tf(c);
   // LICFilter::createBoxFilter(256) (dataset.cpp:1405-1413), GL_CLAMP
   int w = 0;
   vvlic_make_filter_table(VVLIC_FILTER_BOX, 256, c->filter, &w);
@@ -875,6 +886,7 @@ extern "C" vvlic_status vvlic_set_tf(vvlic_ctx* c, const float* rgba, const floa
   if (opacity) std::memcpy(c->tf + 4 * VVLIC_TF_ENTRIES, opacity, sizeof(float) * VVLIC_TF_ENTRIES);
   for (int i = 0; i < 5 * VVLIC_TF_ENTRIES; ++i)
     if (!std::isfinite(c->tf[i])) return fail(c, VVLIC_ERR_INVALID_ARGUMENT, "set_tf: non-finite entry %d", i);
+  sort_tf(c);
   DeviceGuard g(c->device);
   cudaError_t e = after_launches(c);
   if (e == cudaSuccess)

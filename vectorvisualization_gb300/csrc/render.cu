@@ -164,20 +164,24 @@ static void set_noise_wrap(double start, RenderArgs& a) {
   for (int i = 0; i < 3; ++i) noise_wrap_constants(a.m[i], &a.nclamp[i], &a.nwrap_mul[i], &a.nwrap_off[i]);
 }
 
-// Whether a sample's alpha can exceed the threshold that ends its ray (shade, with both tables at their extremes;
-// the margin covers the kernels' powf), and the samples of an average ray: the box's volume over its
-// projection along the view axis, in samples.  Work is split by them (launch_one); results do not depend on it.
+// What the work split goes by (launch_one, lane_per_ray); results do not depend on it.
+//   may_end: rays may well end early, where a 64th of all pairs of a TF alpha and an opacity exceed the threshold
+//     (shade's alpha correction undone on the threshold).  A lower bar takes in random and default tables whose
+//     extremes alone exceed it, whose rays go on.
+//   along_rows: rows of pixels run (within eight degrees) along x.
+//   mean_samples: the box's volume over its projection along the view axis, in samples.
 static void set_ray_length(const vvlic_ctx* c, RenderArgs& a) {
-  float lo[2] = {c->tf[3], c->tf[4 * VVLIC_TF_ENTRIES]}, hi[2] = {lo[0], lo[1]};
-  for (int i = 0; i < VVLIC_TF_ENTRIES; ++i) {
-    const float v[2] = {c->tf[4 * i + 3], c->tf[4 * VVLIC_TF_ENTRIES + i]};
-    for (int k = 0; k < 2; ++k) {
-      lo[k] = std::min(lo[k], v[k]);
-      hi[k] = std::max(hi[k], v[k]);
-    }
+  const double thr = a.alpha_thr, bar = thr >= 1.0 ? 2.0 : (thr < 0.0 ? -1.0 : 1.0 - std::pow(1.0 - thr, 1.0 / a.alpha_corr));
+  constexpr int n = VVLIC_TF_ENTRIES;
+  const float *alpha = c->tf_sorted, *opacity = c->tf_sorted + n;  // ascending
+  int pairs = 0;
+  for (int i = 0, j = n; i < n; ++i) {  // as alpha grows, ever lower opacities reach the bar
+    while (j > 0 && (double)alpha[i] * opacity[j - 1] > bar) --j;
+    pairs += n - j;
   }
-  const double al = std::max({(double)hi[0] * hi[1], (double)lo[0] * lo[1], (double)hi[0] * lo[1], (double)lo[0] * hi[1]});
-  a.may_end = !(1.0 - std::pow(std::max(1.0 - al, 0.0), (double)a.alpha_corr) <= (double)a.alpha_thr - 1e-4);
+  a.may_end = pairs >= n * n / 64;
+  const float* row = a.clamp0 ? a.d1 : a.o1;
+  a.along_rows = row[0] * row[0] > 0.98f * (row[0] * row[0] + row[1] * row[1] + row[2] * row[2]);
   double v[3], e[3], len = 0.0, area = 0.0;
   for (int i = 0; i < 3; ++i) {
     v[i] = a.d0[i] + 0.5 * a.W * a.d1[i] + 0.5 * a.H * a.d2[i];

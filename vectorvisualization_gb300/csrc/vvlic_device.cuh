@@ -67,8 +67,9 @@ struct RenderArgs {
   uint32_t* tape_n;
   unsigned long long* tape_overflow;  // rays with more samples than tape_stride
   int tape_stride, tape_nck;
-  // host rules of the work split (launch_one): whether a sample can end its ray, and the samples of an average ray
-  int may_end;
+  // for the host's rules of the work split (set_ray_length): whether rays may well end early, whether rows of pixels
+  // lie along rows of texels, and the samples of an average ray
+  int may_end, along_rows;
   float mean_samples;
   float taps[kMaxTaps];
 };

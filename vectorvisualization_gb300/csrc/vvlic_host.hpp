@@ -95,6 +95,7 @@ struct vvlic_ctx {
   float* d_scalar = nullptr;
   int sn[3] = {0, 0, 0};
   float tf[5 * VVLIC_TF_ENTRIES];  // RGBA entries then opacity entries
+  float tf_sorted[2 * VVLIC_TF_ENTRIES];  // alphas, then opacities, ascending (set_ray_length)
   float* d_tf = nullptr;
   uint8_t filter[1024];
   int filter_width = 0;
