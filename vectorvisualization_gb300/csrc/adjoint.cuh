@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(kThreads, ray_min_blocks<INTEG, GRAD>())
 template <int INTEG, bool GRAD> static bool lane_per_ray(const RenderArgs& a, int num_sms) {
   const long long tiles = cast_tiles(a), resident = resident_warps(num_sms);
   if (head_samples(a, num_sms) == 0xffffffffu) return true;
-  if (a.may_end && tiles >= (INTEG == VVLIC_RK4 ? 64 : 16) * resident) return true;
+  if (may_end(a) && tiles >= (INTEG == VVLIC_RK4 ? 64 : 16) * resident) return true;
   return GRAD && INTEG == VVLIC_RK4 && tiles >= (a.along_rows ? 64 : 192) * resident;
 }
 

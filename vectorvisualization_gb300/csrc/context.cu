@@ -316,6 +316,7 @@ static void sort_tf(vvlic_ctx* c) {
   }
   std::sort(s, s + VVLIC_TF_ENTRIES);
   std::sort(s + VVLIC_TF_ENTRIES, s + 2 * VVLIC_TF_ENTRIES);
+  c->share_thr = NAN;
 }
 
 static void default_tables(vvlic_ctx* c) {

@@ -164,14 +164,37 @@ static void set_noise_wrap(double start, RenderArgs& a) {
   for (int i = 0; i < 3; ++i) noise_wrap_constants(a.m[i], &a.nclamp[i], &a.nwrap_mul[i], &a.nwrap_off[i]);
 }
 
-// What the work split goes by (launch_one, lane_per_ray); results do not depend on it.
-//   may_end: rays may well end early, where a 64th of all pairs of a TF alpha and an opacity exceed the threshold
-//     (shade's alpha correction undone on the threshold).  A lower bar takes in random and default tables whose
-//     extremes alone exceed it, whose rays go on.
+// Samples of the ray through pixel position (u, v) if nothing ends it: ray_setup and outside_box in double; 0 if it
+// misses.
+static double ray_samples(const RenderArgs& a, double u, double v) {
+  double o[3], d[3], tn = -INFINITY, tf = INFINITY, len = 0.0;
+  for (int i = 0; i < 3; ++i) {
+    o[i] = a.o0[i] + u * a.o1[i] + v * a.o2[i];
+    d[i] = a.d0[i] + u * a.d1[i] + v * a.d2[i];
+    len += d[i] * d[i];
+    const double t0 = -o[i] / d[i], t1 = (a.ext[i] - o[i]) / d[i];  // d = 0: a slab's infinities, or NaN, which drop out
+    tn = std::fmax(tn, std::fmin(t0, t1));
+    tf = std::fmin(tf, std::fmax(t0, t1));
+  }
+  if (a.clamp0) tn = std::fmax(tn, 0.0);
+  if (!(tn < tf)) return 0.0;
+  double run = INFINITY;
+  for (int i = 0; i < 3; ++i) {
+    const double p = (o[i] + tn * d[i]) * a.scale_vol[i], step = d[i] / std::sqrt(len) * a.scale_vol[i] * a.step_size;
+    if (step != 0.0) run = std::fmin(run, ((step > 0.0 ? a.tex_max[i] : 0.0) - p) / step);
+  }
+  return run < 1e9 ? std::fmax(run, 1.0) : 1e9;
+}
+
+// What the work split goes by (launch_one, lane_per_ray, launch_tech_one, batches); results do not depend on it.
+//   end_share: the share of all pairs of a TF alpha and an opacity that exceed the threshold (shade's alpha
+//     correction undone on it).  Rays may well end early from a 64th on; a lower bar takes in random and default
+//     tables whose extremes alone exceed it, whose rays go on.  At 1 every sample ends its ray.
 //   along_rows: rows of pixels run (within eight degrees) along x.
-//   mean_samples: the box's volume over its projection along the view axis, in samples.
-static void set_ray_length(const vvlic_ctx* c, RenderArgs& a) {
-  const double thr = a.alpha_thr, bar = thr >= 1.0 ? 2.0 : (thr < 0.0 ? -1.0 : 1.0 - std::pow(1.0 - thr, 1.0 / a.alpha_corr));
+//   mean_samples: the box's volume over its projection along the view axis, in samples; where the lit shaders'
+//     scale makes rays march through another box than they enter (thin volumes), the mean of nine rays.
+static float end_share(const vvlic_ctx* c, double thr, double alpha_corr) {
+  const double bar = thr >= 1.0 ? 2.0 : (thr < 0.0 ? -1.0 : 1.0 - std::pow(1.0 - thr, 1.0 / alpha_corr));
   constexpr int n = VVLIC_TF_ENTRIES;
   const float *alpha = c->tf_sorted, *opacity = c->tf_sorted + n;  // ascending
   int pairs = 0;
@@ -179,7 +202,16 @@ static void set_ray_length(const vvlic_ctx* c, RenderArgs& a) {
     while (j > 0 && (double)alpha[i] * opacity[j - 1] > bar) --j;
     pairs += n - j;
   }
-  a.may_end = pairs >= n * n / 64;
+  return (float)pairs / (n * n);
+}
+
+static void set_ray_length(vvlic_ctx* c, RenderArgs& a) {
+  if (c->share_thr != a.alpha_thr || c->share_corr != a.alpha_corr) {  // NaN after set_tf
+    c->share = end_share(c, a.alpha_thr, a.alpha_corr);
+    c->share_thr = a.alpha_thr;
+    c->share_corr = a.alpha_corr;
+  }
+  a.end_share = c->share;
   const float* row = a.clamp0 ? a.d1 : a.o1;
   a.along_rows = row[0] * row[0] > 0.98f * (row[0] * row[0] + row[1] * row[1] + row[2] * row[2]);
   double v[3], e[3], len = 0.0, area = 0.0;
@@ -191,6 +223,17 @@ static void set_ray_length(const vvlic_ctx* c, RenderArgs& a) {
   for (int i = 0; i < 3; ++i) area += std::fabs(v[i]) * e[(i + 1) % 3] * e[(i + 2) % 3];
   const double mean = e[0] * e[1] * e[2] * std::sqrt(len) / area / a.step_size;
   a.mean_samples = mean > 0.0 && mean < 1e9 ? (float)mean : 1e9f;
+  bool same = true;
+  for (int i = 0; i < 3; ++i) same = same && std::fabs(e[i] - a.ext[i]) < 1e-3 * a.ext[i];
+  if (same) return;
+  double sum = 0.0;
+  int hits = 0;
+  for (int k = 0; k < 9; ++k) {
+    const double s = ray_samples(a, a.W * (k % 3 + 0.5) / 3.0, a.H * (k / 3 + 0.5) / 3.0);
+    sum += s;
+    hits += s > 0.0;
+  }
+  a.mean_samples = hits ? (float)(sum / hits) : 1e9f;
 }
 
 // Fill the kernel argument block for one volume and image size.

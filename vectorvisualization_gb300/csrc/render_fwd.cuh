@@ -142,6 +142,7 @@ inline long long cast_tiles(const RenderArgs& a) { return (long long)((a.W + 1) 
 inline long long resident_warps(int num_sms) { return 24ll * num_sms; }
 // Samples that a frame's rays take one at a time, a lane to a ray, before the groups: where rays end after a sample
 // or two, or are no longer than that, seven of a group's eight lanes are lost.
+//   Frames all of whose samples end their ray (end_share 1): all of them, 0xffffffff.
 //   Frames whose rays may well end early (may_end): the first 1 to 16 by the frame's size, since a lane to a ray is
 //     as fast as groups on a large frame only (192^3, 131 samples a ray, ms by lane / groups: 256^2
 //     3.9 / 1.6, 512^2 6.6 / 5.2, 1024^2 19.4 / 19.3).  All opaque, 1024^2, groups alone / so: unlit 1.23 / 0.23 ms, lit
@@ -151,10 +152,12 @@ inline long long resident_warps(int num_sms) { return 24ll * num_sms; }
 //     14 samples a ray 2.42 / 2.07, 3.08 / 2.61, 4.46 / 3.96.
 // A recording's checkpoints hold the state before every 32nd sample, which a group knows for its first one only:
 // its rays take eight or sixteen samples first, or none where the frame is so small that eight cost 10 %.
+inline bool may_end(const RenderArgs& a) { return a.end_share >= 1.0f / 64.0f; }
 inline uint32_t head_samples(const RenderArgs& a, int num_sms) {
+  if (a.end_share >= 1.0f) return 0xffffffffu;
   const uint32_t head = (uint32_t)std::min<long long>(16, cast_tiles(a) / (2 * resident_warps(num_sms)));
   if (head > 0 && a.mean_samples <= 1.5f * head) return 0xffffffffu;
-  return !a.may_end ? 0u : (a.tape_is ? (head < 3 ? 0u : (head + 7) / 8 * 8) : head);
+  return !may_end(a) ? 0u : (a.tape_is ? (head < 3 ? 0u : (head + 7) / 8 * 8) : head);
 }
 static_assert(kSegment % 8 == 0, "checkpoints at the first sample of a group");
 template <int INTEG, bool GRAD> static int cast_cta_threads(const RenderArgs& a, int num_sms) {

@@ -67,9 +67,10 @@ struct RenderArgs {
   uint32_t* tape_n;
   unsigned long long* tape_overflow;  // rays with more samples than tape_stride
   int tape_stride, tape_nck;
-  // for the host's rules of the work split (set_ray_length): whether rays may well end early, whether rows of pixels
-  // lie along rows of texels, and the samples of an average ray
-  int may_end, along_rows;
+  // for the host's rules of the work split (set_ray_length): the share of samples that would end their ray, whether
+  // rows of pixels lie along rows of texels, and the samples of an average ray
+  float end_share;
+  int along_rows;
   float mean_samples;
   float taps[kMaxTaps];
 };

@@ -96,6 +96,8 @@ struct vvlic_ctx {
   int sn[3] = {0, 0, 0};
   float tf[5 * VVLIC_TF_ENTRIES];  // RGBA entries then opacity entries
   float tf_sorted[2 * VVLIC_TF_ENTRIES];  // alphas, then opacities, ascending (set_ray_length)
+  // end_share of the tables for a threshold and an alpha correction (batches build hundreds of argument blocks)
+  float share = 0.f, share_thr = NAN, share_corr = NAN;
   float* d_tf = nullptr;
   uint8_t filter[1024];
   int filter_width = 0;
