@@ -157,10 +157,29 @@ vvlic_status prepare_batch(vvlic_ctx* c, const vvlic_job* jobs, int n, int tw, i
 // 12.7 at 64^2; 320 views at 32^2 14.9 / 21.9 ms, 800 at 16^2 27.6 / 13.6 (launches).  The line lies at a mean
 // of a sixteenth of the resident warps in 2x2-ray tiles, 30^2 pixels.  The context's streams have the priority
 // of the caller's.
-bool job_by_job(const vvlic_ctx* c, const vvlic_job* jobs, int n) {
+//
+// Rays of a few samples leave most lanes of a group idle and frames of them too short for a launch each.
+// Batches of them (`samples` a ray, on average) run in the persistent launch up to the size from which
+// single frames of such rays take a lane to a ray (head_samples), and there a lane to a ray (lane_per_ray).  All
+// opaque, one by one / persistent in groups / a lane to a ray (ms): 320 views at 32^2 1.14 / 0.32 / 0.11, 64 at 64^2
+// 0.63 / 0.23 / 0.08, 64 at 128^2 1.08 / 0.69 / 0.20, 24 at 256^2 0.28 / 0.95 / 0.26, 800 at 16^2 - / 0.26 / 0.11.
+// Opaque for half of the alphas, where half of the rays go on: 320 at 32^2 1.51 / 0.61 / 0.75, 64 at 128^2 1.15 / 1.27
+// / 0.87.
+bool job_by_job(const vvlic_ctx* c, const vvlic_job* jobs, int n, double samples) {
   double tiles = 0.0;
   for (int j = 0; j < n; ++j) tiles += (double)((jobs[j].w + 1) / 2) * (double)((jobs[j].h + 1) / 2);
-  return tiles >= 24.0 / 16.0 * c->num_sms * n;
+  const double resident = 24.0 * c->num_sms, mean = tiles / n;
+  return mean >= resident / 16.0 && !(samples <= 4.0 && mean < 2.0 * resident);
+}
+
+// Samples of an average ray of the prepared jobs, taken as two where half of all samples would end it.
+double expected_samples(const vvlic_ctx* c, int n) {
+  double sum = 0.0;
+  for (int j = 0; j < n; ++j) {
+    const RenderArgs& a = c->h_jobs[j];
+    sum += std::min(a.mean_samples, a.end_share >= 0.5f ? 2.0f : 64.0f);
+  }
+  return sum / n;
 }
 
 vvlic_status launch_jobs(vvlic_ctx* c, int n, int storage, int sampler, int integ, bool grad, cudaStream_t s) {
@@ -211,7 +230,10 @@ vvlic_status batch_render(vvlic_ctx* c, const vvlic_job* jobs, int n, cudaStream
   vvlic_status st = prepare_batch(c, jobs, n, tw, sampler_override, s, &storage, &sampler, &integ, &grad, &ntiles,
                                   start);
   if (st) return st;
-  if (job_by_job(c, jobs, n)) {
+  const double samples = expected_samples(c, n);
+  const bool lane_per_ray = samples <= 8.0;
+  c->batch_by_job = job_by_job(c, jobs, n, samples);
+  if (c->batch_by_job) {
     if ((st = launch_jobs(c, n, storage, sampler, integ, grad, s))) return st;
     c->stats_pending = true;
     c->tape_flag_pending = false;
@@ -241,7 +263,7 @@ vvlic_status batch_render(vvlic_ctx* c, const vvlic_job* jobs, int n, cudaStream
   }
   if (e != cudaSuccess) return cuda_fail(c, e, "batch upload");
   const uint64_t key[8] = {(uint64_t)n, (uint64_t)ntiles, (uint64_t)storage, (uint64_t)sampler, (uint64_t)integ,
-                           (uint64_t)grad, (uint64_t)tw, 0};
+                           (uint64_t)grad, (uint64_t)tw, (uint64_t)lane_per_ray};
   if (!c->batch_graph || std::memcmp(key, c->batch_key, sizeof key) != 0) {
     drop_graph(c);
     // capture: counters reset, order pass, queue reset, the persistent launch
@@ -252,7 +274,7 @@ vvlic_status batch_render(vvlic_ctx* c, const vvlic_job* jobs, int n, cudaStream
     if (ec == cudaSuccess) ec = launch_batch_order(bs, n, ntiles, s);
     if (ec == cudaSuccess) ec = cudaMemsetAsync(bs.next, 0, sizeof(unsigned), s);
     if (ec == cudaSuccess) {
-      BatchLaunch b{c->d_jobs, bs.order, ntiles, bs.next, c->d_tf, c->d_counters, tw, c->num_sms};
+      BatchLaunch b{c->d_jobs, bs.order, ntiles, bs.next, c->d_tf, c->d_counters, tw, c->num_sms, lane_per_ray};
       ec = launch_batch(storage, b, sampler, integ, grad, s);
     }
     e = cudaStreamEndCapture(s, &graph);
@@ -300,7 +322,7 @@ extern "C" vvlic_status vvlic_batch_autotune(vvlic_ctx* c, const vvlic_job* jobs
   const int tws[4] = {8, 4, 16, 32};
   float best = 1e30f;
   int bt = c->batch_tile_w, bs = jobs[0].params.sampler;
-  const bool shaped = !job_by_job(c, jobs, n);  // launched one by one, the jobs have no tile shape
+  bool shaped = true;  // launched one by one, the jobs have no tile shape
   for (int smp : samplers) {
     for (int tw : tws) {
       if (!shaped && tw != tws[0]) continue;
@@ -308,6 +330,7 @@ extern "C" vvlic_status vvlic_batch_autotune(vvlic_ctx* c, const vvlic_job* jobs
       for (int rep = 0; rep < 2; ++rep) {  // the first render builds layouts and the graph
         vvlic_status st = batch_render(c, jobs, n, s, tw, smp);
         if (st) return st;
+        shaped = !c->batch_by_job;
         cudaError_t e = cudaEventSynchronize(c->ev1);
         if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, c->ev0, c->ev1);
         if (e != cudaSuccess) return cuda_fail(c, e, "batch_autotune");

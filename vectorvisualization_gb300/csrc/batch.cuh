@@ -21,7 +21,7 @@ template <int INTEG, bool GRAD> constexpr int batch_min_blocks() {
   return (!GRAD && INTEG != VVLIC_RK4) ? VVLIC_BATCH_UNLIT_MIN_BLOCKS : min_blocks<INTEG>();
 }
 
-template <int ST, int FL, int NL, int INTEG, bool GRAD>
+template <int ST, int FL, int NL, int INTEG, bool GRAD, int S>
 __global__ void __launch_bounds__(kThreads, batch_min_blocks<INTEG, GRAD>())
     raycast_batch_kernel(const RenderArgs* __restrict__ jobs, const uint2* __restrict__ order, int nitems,
                          unsigned* __restrict__ next, const float* __restrict__ tf, unsigned long long* counters,
@@ -49,10 +49,10 @@ __global__ void __launch_bounds__(kThreads, batch_min_blocks<INTEG, GRAD>())
       cur = item.x;
     }
     const int tiles_x = (a.W + tw - 1) / tw;
-    // the tile's 32 pixels in four groups of 8 rays, four samples at a time
-    constexpr int S = 4, R = 32 / S;
+    // the tile's 32 pixels: four groups of 8 rays, four samples at a time, or a lane to a ray
+    constexpr int R = 32 / S;
     for (int sub = 0; sub < S; ++sub) {
-      const BatchPixel pixel = batch_pixel(tw, item.y, tiles_x, sub, lane % R);
+      const BatchPixel pixel = batch_pixel(tw, item.y, tiles_x, S == 1 ? lane / 8 : sub, S == 1 ? lane % 8 : lane % R);
       const int px = pixel.x, py = pixel.y;
       const bool ray = px < a.W && py < a.H;
       if (!__any_sync(0xffffffffu, ray)) continue;
@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kThreads, batch_min_blocks<INTEG, GRAD>())
 
 template <int ST, int FL, int NL, int INTEG, bool GRAD>
 static cudaError_t launch_batch_one(const BatchLaunch& b, cudaStream_t s) {
-  auto kern = raycast_batch_kernel<ST, FL, NL, INTEG, GRAD>;
+  auto kern = b.lane_per_ray ? raycast_batch_kernel<ST, FL, NL, INTEG, GRAD, 1> : raycast_batch_kernel<ST, FL, NL, INTEG, GRAD, 4>;
   int per_sm = 0;
   cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, 0);
   if (e != cudaSuccess) return e;

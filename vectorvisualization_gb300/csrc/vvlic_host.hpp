@@ -154,6 +154,7 @@ struct vvlic_ctx {
   int batch_tile_w = 8;                 // warp tile width (autotuned)
   int batch_sampler_override = -1;      // sampler chosen by the autotuner (-1: the jobs')
   bool last_was_batch = false;
+  bool batch_by_job = false;            // how the last batch ran (batch.cu, job_by_job)
   // streams of batches whose jobs are launched one by one (batch.cu), created on first use for each
   // priority of a caller's stream (a device has six)
   static constexpr int kBatchStreams = 7;

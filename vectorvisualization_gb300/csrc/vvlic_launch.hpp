@@ -55,6 +55,7 @@ struct BatchLaunch {
   unsigned long long* counters;  // [0] samples, [1] rays, [2] sample-steps
   int tw;                        // tile width in pixels (a warp covers tw x 32/tw)
   int num_sms;
+  bool lane_per_ray;             // else groups of four samples
 };
 cudaError_t launch_batch_f32(const BatchLaunch& b, int sampler, int integ, bool grad, cudaStream_t s);
 cudaError_t launch_batch_f16(const BatchLaunch& b, int sampler, int integ, bool grad, cudaStream_t s);
