@@ -607,12 +607,24 @@ __global__ void __launch_bounds__(kThreads, ray_min_blocks<INTEG, GRAD>())
 //     450^2 1.1 / 1.4, 6.8 / 6.9, 8.5 / 11.0;
 //   the largest lit RK4 frames, from 192 times as many, or 64 where rows of pixels lie along rows of texels: views of
 //     a 512^3 field so / turned, L = 60, 2048^2 1456 / 1274 and 1494 / 1470 ms (before the groups 1312 and 1491),
-//     1024^2 420 / 400 and 480 / 517 (387 and 512).
+//     1024^2 420 / 400 and 480 / 517 (387 and 512);
+//   large frames of the other kinds, the sooner the shorter the streamlines: all eight lanes of a ray blend its
+//     samples, so the compositing costs the groups more.  128^3, L = 30, default / random TF: lit Heun 500^2 5.0 / 5.1 and 8.0 / 7.8, 650^2 8.2 / 6.9
+//     and 13.2 / 11.8, 1100^2 23.0 / 15.8 and 37.1 / 29.9; unlit 650^2 1.34 / 0.76 and 3.74 / 4.93, 800^2 2.00 / 1.08 and 5.49 / 6.19;
+//     unlit RK4 1100^2 3.78 / 2.10 and 13.7 / 15.6.  192^3, L = 60: lit Heun 500^2 15.9 / 16.3 and 20.3 / 22.4, 650^2 26.3 / 25.6 and
+//     33.7 / 33.3; unlit 800^2 3.2 / 2.8 and 12.5 / 16.7, 1100^2 6.0 / 4.1 and 22.8 / 25.1; unlit RK4 1100^2 6.1 / 5.4 and 34.8 / 41.9.
+//     96^3, L = 10: lit Heun 500^2 1.56 / 0.94 and 3.43 / 2.81; RK4 800^2 unlit 1.56 / 0.89 and 3.45 / 3.53, lit 3.88 / 2.94 and
+//     9.82 / 9.77.
 template <int INTEG, bool GRAD> static bool lane_per_ray(const RenderArgs& a, int num_sms) {
   const long long tiles = cast_tiles(a), resident = resident_warps(num_sms);
   if (head_samples(a, num_sms) == 0xffffffffu) return true;
-  if (may_end(a) && tiles >= (INTEG == VVLIC_RK4 ? 64 : 16) * resident) return true;
-  return GRAD && INTEG == VVLIC_RK4 && tiles >= (a.along_rows ? 64 : 192) * resident;
+  if (may_end(a) && tiles >= (INTEG == VVLIC_RK4 && a.end_share < 0.5f ? 64 : 16) * resident) return true;
+  const int L = std::max(a.lb, a.lf);
+  int line = 0;
+  if (INTEG != VVLIC_RK4) line = GRAD ? (L <= 24 ? 16 : 24) : (L <= 36 ? 40 : 64);
+  else if (GRAD) line = L <= 24 ? 40 : (a.along_rows ? 64 : 192);
+  else line = L <= 24 ? 40 : (L <= 36 ? 64 : 128);
+  return tiles >= line * resident;
 }
 
 template <typename Kernel>
