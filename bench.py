@@ -55,8 +55,7 @@ def parse():
     ap.add_argument("--impl", choices=["ours", "reference"], default="ours")
     ap.add_argument("--sampler", default="hybrid", choices=["gather", "cell", "texture", "hybrid"])
     ap.add_argument("--schedule", default="auto", choices=["auto", "queue", "static"],
-                    help="passed on to the library, which runs the same raster grid for both (BRICK frames "
-                         "excepted); auto: static for the orbit frames, queue for the others")
+                    help="passed on to the library, which runs the same raster grid for both; auto: static for the orbit frames, queue for the others")
     ap.add_argument("--size", type=int, default=512, help="orbit field size per axis")
     ap.add_argument("--image", type=int, default=2048, help="orbit image size")
     ap.add_argument("--c2-size", type=int, default=256)
@@ -77,8 +76,7 @@ def parse():
 
 
 def schedule(args, workload: str) -> str:
-    """The schedule a section passes to the library.  Ray-casts run the same raster grid of sample
-    groups under either name; only the BRICK sampler tells them apart."""
+    """The schedule a section passes to the library, which accepts it without effect."""
     if args.schedule != "auto":
         return args.schedule
     return "static" if workload == "orbit" else "queue"
@@ -396,7 +394,7 @@ def bench_brick(ctx, torch, stream, flush, args):
         for sampler in ("brick", "gather", "cell", "texture", "hybrid"):
             p = capi.Params.from_buffer_copy(w.params)
             p.sampler = capi.SAMPLER[sampler]
-            p.schedule = capi.SCHEDULE["static" if sampler == "brick" else schedule(args, "brick_ab")]
+            p.schedule = capi.SCHEDULE[schedule(args, "brick_ab")]
             ctx.set_params(p)
             frame = lambda: ctx.render_device(vid, out.data_ptr(), W, H, None, stream.cuda_stream)  # noqa: E731
             timed(torch, stream, flush, frame)

@@ -69,8 +69,8 @@ enum { VVLIC_STORAGE_F32 = 0, VVLIC_STORAGE_F16 = 1, VVLIC_STORAGE_BF16 = 2, VVL
  *   BRICK   - field and noise texels staged per 16x8 ray tile into shared memory by TMA
  *             (cp.async.bulk.tensor), one brick pair per segment of 8 samples covering the
  *             samples' streamline reach; GATHER's arithmetic from shared memory, global memory
- *             for fetches outside the bricks.  RAYCAST renders only (no tape, no batch), static
- *             schedule; needs field rows (nx * texel bytes) and noise rows (mx * channels) that
+ *             for fetches outside the bricks.  RAYCAST renders only (no tape, no batch);
+ *             needs field rows (nx * texel bytes) and noise rows (mx * channels) that
  *             are multiples of 16 bytes (else VVLIC_ERR_UNSUPPORTED). */
 enum {
   VVLIC_SAMPLER_GATHER = 0,
@@ -181,9 +181,10 @@ typedef struct vvlic_params {
  *               vvlic_compute_lic_volume. */
 enum { VVLIC_TECHNIQUE_VOLUME = 0, VVLIC_TECHNIQUE_RAYCAST = 1, VVLIC_TECHNIQUE_SLICING = 2, VVLIC_TECHNIQUE_LICVOLUME = 3 };
 
-/* Work distribution of a render launch.  Forward ray-casts run one raster grid of small CTAs, a warp
- * on 2x2 (or 2x1) rays with 8 (16) consecutive samples of each side by side, under either value;
- * adjoints pull 2x2-ray tiles from a device counter (no spin-waits: one atomic per tile). */
+/* Accepted for older callers; without effect.  Every sampler's forward ray-casts run a raster grid (a
+ * warp on 2 to 8 rays with 16, 8 or 4 consecutive samples of each side by side, or on 32 rays by one sample each
+ * where rays are short or may end early), and adjoints pull tiles of rays from a device counter (no
+ * spin-waits: one atomic per tile). */
 enum { VVLIC_SCHEDULE_QUEUE = 0, VVLIC_SCHEDULE_STATIC = 1 };
 
 /* View.  PERSPECTIVE follows Camera::setCamera (camera.cpp:56-67) followed by
@@ -474,16 +475,18 @@ typedef struct vvlic_job {
   int32_t filter_clamp;
 } vvlic_job;
 
-/* Render n jobs side by side.  Jobs of 30 x 30 pixels and more (on average) are launched one by one over
- * `stream` and streams of the context, joined back into `stream`.  Smaller ones go through one persistent
- * launch: every (job, 8x4 tile) item enters one device work queue in job-major order (jobs in
- * submission order, each job's tiles in raster order), and the launch sequence is captured in a
+/* Render n jobs side by side.  Jobs of 30 x 30 pixels and more (on average; 170 x 170 where rays end at once or
+ * have up to four samples) are launched one by one over
+ * `stream` and streams of the context at its priority, joined back into `stream`; batches on several streams
+ * of one context share these and wait for one another.  Smaller ones go through one persistent launch: every
+ * (job, 8x4 tile) item enters one device work queue in job-major order (jobs in submission order, each job's tiles
+ * in raster order), and the launch sequence is captured in a
  * CUDA graph the first time a batch of a given shape is rendered and replayed afterwards (only the
  * job table is re-uploaded).  All jobs must share the field storage, sampler, integrator and
  * lighting (they are compiled variants); LIC length, step sizes, filter, view, image size, TF
  * index and the other runtime parameters may differ.  The noise, scalar volume and transfer function
  * are the context's.  `stream` must not be the legacy default stream (NULL selects the context's
- * stream).  Asynchronous; vvlic_get_stats reports the batch totals. */
+ * stream) nor one that is being captured.  Asynchronous; vvlic_get_stats reports the batch totals. */
 vvlic_status vvlic_batch_render(vvlic_ctx* ctx, const vvlic_job* jobs, int32_t n, void* stream);
 
 /* Time the batch under each warp tile shape of the persistent launch (8x4, 4x8, 16x2, 32x1 pixels; jobs
